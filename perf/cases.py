@@ -187,13 +187,14 @@ def prepare(case, seed):
         s["gate"] = (gate / gate.sum(1, keepdim=True)).contiguous()
         s["x"] = r.normal(t, h, dtype=dt)
         fp8 = dt == torch.float8_e4m3fn
-        s["w_up"] = r.normal(e, 2 * f, h, dtype=dt, std=1.0 if fp8 else 0.02)
+        s["w_gate"] = r.normal(e, f, h, dtype=dt, std=1.0 if fp8 else 0.02)
+        s["w_up"] = r.normal(e, f, h, dtype=dt, std=1.0 if fp8 else 0.02)
         s["w_down"] = r.normal(e, h, f, dtype=dt, std=1.0 if fp8 else 0.02)
-        s["s_up"] = r.scale(e, about=0.02) if fp8 else None
+        s["s_in"] = [r.scale(e, about=0.02), r.scale(e, about=0.02)] if fp8 else None
         s["s_down"] = r.scale(e, about=0.02) if fp8 else None
-        s["h"] = torch.empty(t * topk, 2 * f, device=DEVICE, dtype=out)
+        s["h"] = [torch.empty(t * topk, f, device=DEVICE, dtype=out) for _ in range(2)]
         env = flux.DistEnvTPWithEP(pg, 1, None, ep_size=1)
-        s["layer0"] = flux.GemmGroupedV3AGScatter(env, flux.MoeArguments(t, h, 2 * f, e, topk, dt, out))
+        s["layer0"] = flux.GemmGroupedV3AGScatter(env, flux.MoeArguments(t, h, f, e, topk, dt, out))
         s["layer1"] = flux.GemmGroupedV3GatherRS(e, t * topk, h, topk, 0, 1, 1, 1, tp_group=pg, dtype=out)
     elif kind == "ulysses":
         bs, seq, nh, hd = case["bs"], case["seq"], case["heads"], case["head_dim"]
@@ -237,16 +238,16 @@ def run(s):
         dw = gemm.wgrad(dyqt, xqt, input_scale=sdyt, weight_scale=sxt)
         return [y, dx, dw]
     if kind == "moe":
-        f = case["ffn"]
         splits, _, scatter, gather, tki = flux.moe_index_build(s["chosen"], case["experts"])
-        h = s["layer0"].forward(s["x"], s["w_up"], splits, scatter, output_scale=s["s_up"], outputs_buf=s["h"])
-        act = torch.nn.functional.silu(h[:, :f]).mul_(h[:, f:])
+        g, u = s["layer0"].forward_multiple_weights(s["x"], [s["w_gate"], s["w_up"]], splits, scatter,
+                                                    output_scale=s["s_in"], outputs_buf=s["h"])
+        act = torch.nn.functional.silu(g).mul_(u)
         if s["x"].dtype != act.dtype:
             act = act.to(s["x"].dtype)
         row_gate = s["gate"][gather, tki]
         y = s["layer1"].forward_gather_rs(act, s["w_down"], splits, scatter.reshape(-1), weight_scale=s["s_down"],
                                           output_vec_scale=row_gate)
-        return [splits, scatter, h, y]
+        return [splits, scatter, g, u, y]
     if kind == "ulysses":
         q, k, v = s["pre"].forward(s["x"], s["w_qkv"])
         return [q, k, v, s["post"].forward(s["o"], s["w_o"])]
