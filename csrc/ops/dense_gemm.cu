@@ -2,7 +2,7 @@
 // maps, tile-shape choice and the launch of dense_gemm_kernel.
 #include "../include/fluxb.h"
 #include "../runtime/host_common.h"
-#include "../sm100/gemm_dense.cuh"
+#include "dense_launch.cuh"
 
 #include <atomic>
 #include <cstdlib>
@@ -42,52 +42,6 @@ uint32_t* wave_counter_for(cudaStream_t stream) {
   return g_wave_pool[dev] + i * 32;
 }
 
-namespace {
-
-// coop: the launch carries the cooperative attribute, so the grid only starts when all of its CTAs
-// can be resident together (and the launch fails, instead of waiting forever inside the kernel, when
-// they never can). Every launch whose CTAs wait for one another or for peers asks for it.
-template <class Cfg>
-int launch_dense(const DenseGemmParams& p, int grid, cudaStream_t stream, bool coop = false) {
-  constexpr int kThreads = Cfg::THREADS;
-  static bool configured[64] = {false};
-  int dev = 0;
-  FLUXB_CUDA_OK(cudaGetDevice(&dev));
-  if (dev >= 64 || !configured[dev]) {
-    FLUXB_CUDA_OK(cudaFuncSetAttribute(dense_gemm_kernel<Cfg>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
-    if (dev < 64) configured[dev] = true;
-  }
-  {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid, 1, 1);
-    cfg.blockDim = dim3(kThreads, 1, 1);
-    cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    int na = 0;
-    if constexpr (Cfg::CG == 2) {
-      attr[na].id = cudaLaunchAttributeClusterDimension;
-      attr[na].val.clusterDim.x = 2;
-      attr[na].val.clusterDim.y = 1;
-      attr[na].val.clusterDim.z = 1;
-      ++na;
-    }
-    if (coop) {
-      attr[na].id = cudaLaunchAttributeCooperative;
-      attr[na].val.cooperative = 1;
-      ++na;
-    }
-    cfg.attrs = attr;
-    cfg.numAttrs = na;
-    FLUXB_CUDA_OK(cudaLaunchKernelEx(&cfg, dense_gemm_kernel<Cfg>, p));
-  }
-  FLUXB_CUDA_OK(cudaGetLastError());
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return kOk;
-}
-
-}  // namespace
 }  // namespace fluxb
 
 using namespace fluxb;

@@ -1,0 +1,5 @@
+// Block-scaled fp8, 128 x 256 tiles.
+#include "dense_launch_impl.cuh"
+
+FLUXB_DENSE_INSTANCE(256, 1, 3, 1, 32768, true);
+FLUXB_DENSE_INSTANCE(256, 1, 4, 1, 0, true);

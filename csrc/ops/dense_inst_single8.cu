@@ -1,0 +1,6 @@
+// Single CTAs, fp8 inputs.
+#include "dense_launch_impl.cuh"
+
+FLUXB_DENSE_INSTANCE(256, 1, 4);
+FLUXB_DENSE_INSTANCE(192, 1, 4);
+FLUXB_DENSE_INSTANCE(128, 1, 6);
