@@ -585,21 +585,23 @@ static int dense_impl(const fluxb_dense_args_t* a, const fluxb_a2a_args_t* x) {
   }
   if (a->blockscale) {
     if (cg == 2) {
-      if (p.mode == kModeAllGather) return launch_dense<DenseCfg<128, 1, 5, 2, 32768, true>>(p, grid, stream, coop);
-      return launch_dense<DenseCfg<128, 1, 6, 2, 0, true>>(p, grid, stream, coop);
+      if (p.mode == kModeAllGather) return launch_dense<DenseCfg<128, 1, 5, 2, 32768, kBsAny>>(p, grid, stream, coop);
+      return launch_dense<DenseCfg<128, 1, 6, 2, 0, kBsAny>>(p, grid, stream, coop);
     }
     if (bn == 256) {
-      if (p.mode == kModeAllGather) return launch_dense<DenseCfg<256, 1, 3, 1, 32768, true>>(p, grid, stream, coop);
-      return launch_dense<DenseCfg<256, 1, 4, 1, 0, true>>(p, grid, stream, coop);
+      if (p.mode == kModeAllGather) return launch_dense<DenseCfg<256, 1, 3, 1, 32768, kBsAny>>(p, grid, stream, coop);
+      if (p.mode == kModeReduceScatter) return launch_dense<DenseCfg<256, 1, 4, 1, 0, kBsAny>>(p, grid, stream, coop);
+      if (p.sb_groupwise) return launch_dense<DenseCfg<256, 1, 4, 1, 0, kBsColumn>>(p, grid, stream, coop);
+      return launch_dense<DenseCfg<256, 1, 4, 1, 0, kBsSquare>>(p, grid, stream, coop);
     }
-    if (p.mode == kModeAllGather) return launch_dense<DenseCfg<128, 1, 4, 1, 32768, true>>(p, grid, stream, coop);
-    return launch_dense<DenseCfg<128, 1, 5, 1, 0, true>>(p, grid, stream, coop);
+    if (p.mode == kModeAllGather) return launch_dense<DenseCfg<128, 1, 4, 1, 32768, kBsAny>>(p, grid, stream, coop);
+    return launch_dense<DenseCfg<128, 1, 5, 1, 0, kBsAny>>(p, grid, stream, coop);
   }
   if (p.mode == kModeAllGather || p.mode == kModeA2AGemm) {
     // variants that carry the staging rings of the all-gather / all-to-all push
     if (mt == 2) {
-      if (in16) return launch_dense<DenseCfg<256, 0, 4, 2, 16384, false, 2>>(p, grid, stream, coop);
-      return launch_dense<DenseCfg<256, 1, 4, 2, 16384, false, 2>>(p, grid, stream, coop);
+      if (in16) return launch_dense<DenseCfg<256, 0, 4, 2, 16384, kBsNone, 2>>(p, grid, stream, coop);
+      return launch_dense<DenseCfg<256, 1, 4, 2, 16384, kBsNone, 2>>(p, grid, stream, coop);
     }
     if (cg == 2 && bn == 256) {
       if (in16) return launch_dense<DenseCfg<256, 0, 6, 2, 16384>>(p, grid, stream, coop);
@@ -619,8 +621,8 @@ static int dense_impl(const fluxb_dense_args_t* a, const fluxb_a2a_args_t* x) {
     return launch_dense<DenseCfg<128, 2, 6>>(p, grid, stream, coop);
   }
   if (mt == 2) {
-    if (in16) return launch_dense<DenseCfg<256, 0, 4, 2, 0, false, 2>>(p, grid, stream, coop);
-    return launch_dense<DenseCfg<256, 1, 4, 2, 0, false, 2>>(p, grid, stream, coop);
+    if (in16) return launch_dense<DenseCfg<256, 0, 4, 2, 0, kBsNone, 2>>(p, grid, stream, coop);
+    return launch_dense<DenseCfg<256, 1, 4, 2, 0, kBsNone, 2>>(p, grid, stream, coop);
   }
   if (cg == 2) {
     if (in16) {

@@ -158,26 +158,39 @@ struct DenseGemmParams {
 // tcgen05.mma.cta_group::2 (MT_ of them per k-step, one per 256-row half), and each CTA ends up with
 // its 128 * MT_ x BN slice of D in its own TMEM.
 // COMM_ > 0 reserves COMM_ bytes of shared memory as staging rings for the all-gather push.
-// BS_ = true: block-scaled fp8 (1x128 A scales, 128x128 B scales): every 128-deep k-block is
+// BS_ != 0: block-scaled fp8 (1x128 A scales, 128x128 or 1x128 B scales): every 128-deep k-block is
 // accumulated into a fresh TMEM buffer (512 / BN_ of them: the issuer runs that many k-blocks ahead)
 // and promoted into fp32 registers, multiplied by its scales, by eight epilogue warps: two per
 // TMEM lane quadrant, each owning half of the tile's columns for the whole tile. BN_ = 256 (one CTA,
 // 128 x 256 tiles) is the faster shape: on 128 x 128 tiles even a kernel that promotes nothing stops at
 // a third of the fp8 rate. With CG_ = 2 and BN_ = 128 a CTA pair shares a 256 x 128 tile (each CTA loads
 // half of B; measured slower than single CTAs).
-template <int BN_, int KIND_, int STAGES_, int CG_ = 1, int COMM_ = 0, bool BS_ = false, int MT_ = 1>
+enum BlockScaleForm : int {
+  kBsNone = 0,
+  kBsAny = 1,      // weight scales per 128 x 128 block or per column, chosen at run time; every mode
+  kBsSquare = 2,   // per 128 x 128 block; plain GEMM only
+  kBsColumn = 3,   // per column and 128-deep k-block (the weight-gradient form); plain GEMM only
+};
+
+template <int BN_, int KIND_, int STAGES_, int CG_ = 1, int COMM_ = 0, int BS_ = kBsNone, int MT_ = 1>
 struct DenseCfg {
   static constexpr int COMM_BYTES = COMM_;
-  static constexpr bool BS = BS_;
+  static constexpr bool BS = BS_ != kBsNone;
+  static constexpr int BS_FORM = BS_;
+  // The multi-rank code is left out: the promotion loop is short of registers, and what else the kernel
+  // holds decides where the compiler puts its spills (28 - 32 bytes, none in the loop; 168 with it).
+  static constexpr bool PLAIN_ONLY = BS_ == kBsSquare || BS_ == kBsColumn;
+  static constexpr int REGS_LEAD = BN_ == 256 ? 40 : 88;       // after setmaxnreg
+  static constexpr int REGS_PROMOTE = BN_ == 256 ? 232 : 208;
   static constexpr int MT = MT_;
-  static constexpr int EPI_WARPS = BS_ ? 8 : 4;
+  static constexpr int EPI_WARPS = BS ? 8 : 4;
   static constexpr int THREADS = 128 + 32 * EPI_WARPS;
   // MT_ == 1: two accumulators used alternately (the epilogue of a tile overlaps the next main loop);
   // MT_ == 2: the two row halves of one tile; block-scaled: one buffer per k-block in flight (4 or 2)
-  static constexpr int ACC_BUFS = BS_ ? 512 / BN_ : 2;
-  static_assert(!BS_ || (KIND_ == 1 && (BN_ == 128 || (BN_ == 256 && CG_ == 1))),
+  static constexpr int ACC_BUFS = BS ? 512 / BN_ : 2;
+  static_assert(!BS || (KIND_ == 1 && (BN_ == 128 || (BN_ == 256 && CG_ == 1))),
                 "block-scaled variant: fp8; 128 columns (128 or 256 rows) or 128 x 256 tiles");
-  static_assert(MT_ == 1 || (MT_ == 2 && CG_ == 2 && BN_ == 256 && !BS_), "512-row tiles: CTA pairs, 256 columns");
+  static_assert(MT_ == 1 || (MT_ == 2 && CG_ == 2 && BN_ == 256 && !BS), "512-row tiles: CTA pairs, 256 columns");
   static constexpr int CG = CG_;
   static constexpr int BM_CTA = 128 * MT_;                 // rows of A / D per CTA
   static constexpr int BM = BM_CTA * CG_;                  // rows per tile
@@ -196,7 +209,7 @@ struct DenseCfg {
   // staging buffers per epilogue warp: the variants with a communication ring give one of the two
   // to a sixth pipeline stage (the epilogue of a tile hides behind the next tile's main loop anyway);
   // block-scaled 256-column tiles give it to the fourth 48 KB stage
-  static constexpr int EPI_BUFS = ((COMM_ > 0 && !BS_) || (BS_ && BN_ == 256)) ? 1 : 2;
+  static constexpr int EPI_BUFS = ((COMM_ > 0 && !BS) || (BS && BN_ == 256)) ? 1 : 2;
   static constexpr int EPI_BYTES = EPI_WARPS * EPI_BUFS * EPI_BUF_BYTES;
   static constexpr int BAR_BYTES = 256;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + COMM_BYTES + BAR_BYTES + 1024;
@@ -204,7 +217,7 @@ struct DenseCfg {
   static constexpr int TMEM_COLS = 512;
   static_assert(ACC_BUFS * BN <= TMEM_COLS, "accumulators must fit TMEM");
   // column pieces of a split tile are BN >> shift wide; the epilogue moves 64 columns at a time
-  static constexpr int MAX_SPLIT_SHIFT = (BN_ == 256 && !BS_) ? 2 : 0;
+  static constexpr int MAX_SPLIT_SHIFT = (BN_ == 256 && !BS) ? 2 : 0;
 };
 
 struct TileCoord {
@@ -343,7 +356,8 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
   const int n_tiles = (p.N + BN - 1) / BN;
   const int total_tiles = p.total_vtiles;   // work items: whole tiles, then the column pieces of split ones
   const int k_blocks = (p.K + BK - 1) / BK;
-  const bool multi = p.world > 1 && p.mode != kModePlain;
+  const int mode = Cfg::PLAIN_ONLY ? static_cast<int>(kModePlain) : p.mode;
+  const bool multi = p.world > 1 && mode != kModePlain;
 
   // -------------------------------------------------------------------- reduce-scatter tail
   // Run by 256 threads of the CTA (tid 0..255; `sync` is a barrier among exactly those): all threads after
@@ -461,7 +475,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
   // tiles the promotion warps hold 128 accumulators and take all they can get: 40 / 232 measured
   // 1560 TFLOP/s where 56 / 224 gave 1376 and 24 / 240 the same 1560 (the compiler's spill report:
   // 168, 176 and 226 bytes per thread, the last mostly in the leading warps).
-  if constexpr (Cfg::BS) ptx::setmaxnreg_dec<(BN == 256 ? 40 : 88)>();
+  if constexpr (Cfg::BS) ptx::setmaxnreg_dec<Cfg::REGS_LEAD>();
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
@@ -491,7 +505,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
         const int b_row = c.n0 + static_cast<int>(cta_rank) * (Cfg::B_ROWS_CTA >> c.shift);
         const int m_cta = c.m_in_seg + static_cast<int>(cta_rank) * Cfg::BM_CTA;
         int a_row = c.seg * p.seg_rows + m_cta;
-        if (p.mode == kModeAllGather && multi) {
+        if (mode == kModeAllGather && multi) {
           if (c.seg == p.rank) {
             a_row = m_cta;  // own shard straight from the caller's tensor
           } else {
@@ -511,10 +525,10 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
         }
         // post-attention mode: the K range is W slices, one per source rank, landing
         // independently; start with the own slice and gate each slice on its flag
-        const int kb_per_src = p.mode == kModeA2AGemm ? (p.a2a_local_heads * p.a2a_hd) / BK : k_blocks;
+        const int kb_per_src = mode == kModeA2AGemm ? (p.a2a_local_heads * p.a2a_hd) / BK : k_blocks;
         // (no division in the k loop: one thread issues every load of the CTA, and a few dozen
         // dependent integer instructions per k-block are enough to starve the tensor pipe)
-        const bool a2a_in = p.mode == kModeA2AGemm;
+        const bool a2a_in = mode == kModeA2AGemm;
         const bool own_in_place = a2a_in && p.a2a_copy_local == 0;
         const int hd_shift = p.a2a_hd == 128 ? 7 : 6;
         const int own_b = own_in_place ? m_cta / p.a2a_local_seq : 0;
@@ -765,7 +779,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
       ptx::st_release_sys(p.start_ctr[lane] + p.rank, p.epoch);
     }
     if constexpr (Cfg::COMM_BYTES > 0) {
-      if (p.mode == kModeAllGather && multi) {
+      if (mode == kModeAllGather && multi) {
         if (lane < p.world) flag_wait_ge(wc, p.start_ctr[p.rank] + lane, p.epoch, kSiteStartBarrier);
         __syncwarp();
         if (lane == 0 && warp == 2) stamp(kTraceHandshake);
@@ -910,7 +924,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
       }
     }
     if constexpr (Cfg::COMM_BYTES > 0) {
-      if (p.mode == kModeA2AGemm) {
+      if (mode == kModeA2AGemm) {
         // heads->seq all-to-all: every rank sends, for each destination d, the rows of its
         // attention output that belong to d's sequence range, re-laid out so that they form
         // columns [rank*local_heads*hd, +local_heads*hd) of d's GEMM input.
@@ -1086,7 +1100,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
     }
   }
   } else {
-      if constexpr (Cfg::BS) ptx::setmaxnreg_inc<(BN == 256 ? 232 : 208)>();
+      if constexpr (Cfg::BS) ptx::setmaxnreg_inc<Cfg::REGS_PROMOTE>();
     // ------------------------------------------------------------------ epilogue
     const int q = warp & 3;              // TMEM lane quadrant this warp may read
     const int ew = warp - 4;             // epilogue warp index
@@ -1101,7 +1115,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
     const bool scaled = p.scale_a != nullptr || p.scale_b != nullptr;
     int it = 0;
     uint32_t nstore = 0;
-    bool started = !(multi && (p.mode == kModeReduceScatter || p.mode == kModeGemmA2A));
+    bool started = !(multi && (mode == kModeReduceScatter || mode == kModeGemmA2A));
 
     // Reduce-scatter, tiles of the own segment: add the partial results that the W-1 peers stored
     // into this rank's staging slabs (64 columns of this thread's row per source, sources in the
@@ -1231,7 +1245,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
       if (lane == 0 && col0 < p.N && store_row0 < p.seg_rows &&
           dcheck(wc, store_row0 >= 0 && col0 >= 0 && (col0 & 7) == 0 && z >= 0 && z < kMaxRanks, kCheckStore,
                  static_cast<uint32_t>(col0), static_cast<uint32_t>(store_row0))) {
-        if (p.mode == kModeGemmA2A) {
+        if (mode == kModeGemmA2A) {
           // 64 columns of one head, 32 consecutive sequence positions of one batch entry:
           // goes to the rank that owns the head, at this rank's place in the full sequence
           const int head = col0 / p.a2a_hd, e0 = col0 % p.a2a_hd;
@@ -1263,6 +1277,142 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
         ptx::st_release_sys(p.rs_ctr[seg] + mt * kMaxRanks + p.rank, p.epoch);
       }
     };
+    if constexpr (Cfg::PLAIN_ONLY) {
+      // ---- block-scaled, plain GEMM on 128 x 256 tiles: every k-block's partial product is multiplied by its
+      // scales and added to fp32 registers. Warp (quadrant q, half) owns rows q*32.. and the 128 columns of one
+      // scale block of the weight for the whole tile. 128 accumulators and 32 staging registers leave about 40
+      // for everything else, so nothing that can be computed again is kept across the loop.
+      // Measured at 8192 x 3584 x 8192 / 8192 x 8192 x 3584 (one 128 x 256 tile per SM and k-block takes 477 ns
+      // without any promotion, the operand stream being the bound): square 303 / 283 us, 320 / 306 before with the
+      // general loop below (two polls of the full barrier and spills); per column 379 / 355 us, 1340 / 1128 before,
+      // when every warp read the column scales from global memory where it multiplied by them. Sixteen warps
+      // of 64 columns: 358 and 667 us. Register splits 24 / 240 and 56 / 224: within 2 % of 40 / 232.
+      constexpr bool kColumn = Cfg::BS_FORM == kBsColumn;
+      const int half = ew >> 2;
+      const int kbs = k_blocks;
+      const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + half * 128;
+      uint32_t n = 0;                                  // k-blocks promoted so far: TMEM buffer n & 1
+#ifdef FLUXB_DEBUG_CHECKS
+      uint64_t probe_wait = 0, probe_ld = 0;           // phase clocks of the self-checking build, as below
+      const long long probe_t0 = clock64();
+#endif
+      for (int t = tile_slot; t < total_tiles; t += tile_stride) {
+        if (*abort_word) break;
+        uint32_t so, bo;                               // offsets of this thread's row / this warp's column scales
+        {
+          const TileCoord c = decode_tile(p, t, m_tiles_seg, n_tiles, BM, BN);
+          const int row = c.m_in_seg + q * 32 + lane;
+          const int row_s = row < ((p.seg_rows + 127) & ~127) ? row : 0;
+          so = static_cast<uint32_t>(row_s >> 7) * static_cast<uint32_t>(kbs) * 128u + (row_s & 127);
+          int nblk = (c.n0 >> 7) + half;
+          if (nblk >= (p.N >> 7)) nblk = (p.N >> 7) - 1;   // (the clipped half of the last tile)
+          bo = static_cast<uint32_t>(nblk) * static_cast<uint32_t>(kbs) * (kColumn ? 128u : 1u) + (kColumn ? 4u * lane : 0u);
+        }
+        uint64_t acc[64];
+#pragma unroll
+        for (int j = 0; j < 64; ++j) acc[j] = 0ull;
+        // row scales and (square form) the weight's scale are fetched two k-blocks ahead; per-column scales one
+        // ahead, four columns per lane, and handed round through the warp's staging buffer (which is free until
+        // the tile is stored): from there every lane reads them as 16-byte broadcasts
+        float psa0, psa1, psb0 = 1.f, psb1 = 1.f;
+        float4 pcol;
+        psa0 = p.sa[so];
+        psa1 = p.sa[so + (kbs > 1 ? 128u : 0u)];
+        if constexpr (kColumn) {
+          pcol = *reinterpret_cast<const float4*>(p.sb + bo);
+          if (lane == 0) ptx::bulk_wait_read<0>();     // the previous tile's store has read the buffer
+          __syncwarp();
+        } else {
+          psb0 = p.sb[bo];
+          psb1 = p.sb[bo + (kbs > 1 ? 1u : 0u)];
+        }
+        for (int kb = 0; kb < kbs; ++kb, ++n) {
+          const float sc = psa0 * psb0;
+          psa0 = psa1;
+          psb0 = psb1;
+          {
+            const uint32_t ahead = kb + 2 < kbs ? kb + 2 : kb;
+            psa1 = p.sa[so + ahead * 128u];
+            if constexpr (!kColumn) psb1 = p.sb[bo + ahead];
+          }
+          const uint32_t slot = my_epi_u32 + (kb & 1) * 512u;
+          if constexpr (kColumn) {
+            // (slot kb & 1 was last read for k-block kb - 2: the warp barrier of kb - 1 lies in between)
+            ptx::st_shared_v4_f32(slot + lane * 16u, pcol);
+            pcol = *reinterpret_cast<const float4*>(p.sb + bo + static_cast<uint32_t>(kb + 1 < kbs ? kb + 1 : kb) * 128u);
+          }
+          const uint32_t buf = n & 1u;
+#ifdef FLUXB_DEBUG_CHECKS
+          const long long pc0 = clock64();
+#endif
+          mbar_wait(wc, tfull_bar(buf), (n >> 1) & 1u, kSiteTmemFull);
+          __syncwarp();
+          ptx::tc_fence_after();
+#ifdef FLUXB_DEBUG_CHECKS
+          const long long pc1 = clock64();
+          probe_wait += static_cast<uint64_t>(pc1 - pc0);
+#endif
+          const uint64_t sc2 = ptx::pack_f32x2(sc, sc);
+          uint32_t r[32];
+#pragma unroll
+          for (int c4 = 0; c4 < 4; ++c4) {
+            ptx::tmem_ld_32x32b_x32(lane_base + buf * 256u + 32 * c4, r);
+            ptx::tmem_ld_wait();
+            if (c4 == 3) {
+#ifdef FLUXB_DEBUG_CHECKS
+              probe_ld += static_cast<uint64_t>(clock64() - pc1);
+#endif
+              // the buffer's contents are in registers: the hand-over needs no release ordering
+              ptx::tc_fence_before();
+              __syncwarp();
+              if (lane == 0) ptx::mbar_arrive_relaxed(tempty_bar(buf));
+            }
+            if constexpr (kColumn) {
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                const ulonglong2 sv = ptx::ld_shared_v2_b64(slot + 128u * c4 + 16u * j);
+                uint64_t& a0 = acc[16 * c4 + 2 * j];
+                uint64_t& a1 = acc[16 * c4 + 2 * j + 1];
+                a0 = ptx::ffma2(ptx::pack_b32x2(r[4 * j], r[4 * j + 1]), ptx::fmul2(sc2, sv.x), a0);
+                a1 = ptx::ffma2(ptx::pack_b32x2(r[4 * j + 2], r[4 * j + 3]), ptx::fmul2(sc2, sv.y), a1);
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 16; ++j)
+                acc[16 * c4 + j] = ptx::ffma2(ptx::pack_b32x2(r[2 * j], r[2 * j + 1]), sc2, acc[16 * c4 + j]);
+            }
+          }
+        }
+        int t_again = t;
+        asm volatile("" : "+r"(t_again));              // (decoded again instead of kept in registers)
+        const TileCoord c = decode_tile(p, t_again, m_tiles_seg, n_tiles, BM, BN);
+        const int row = c.m_in_seg + q * 32 + lane;
+#pragma unroll
+        for (int ch = 0; ch < 2; ++ch) {
+          uint32_t r0[32], r1[32];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            r0[2 * j] = static_cast<uint32_t>(acc[ch * 32 + j]);
+            r0[2 * j + 1] = static_cast<uint32_t>(acc[ch * 32 + j] >> 32);
+            r1[2 * j] = static_cast<uint32_t>(acc[ch * 32 + 16 + j]);
+            r1[2 * j + 1] = static_cast<uint32_t>(acc[ch * 32 + 16 + j] >> 32);
+          }
+          emit_chunk(r0, r1, c.n0 + half * 128 + ch * 64, row, row, c.m_in_seg + q * 32, &p.tm_d[0], 0, false);
+        }
+      }
+      if (lane == 0) ptx::bulk_wait<0>();
+      __syncwarp();
+      if (ew == 0 && lane == 0) stamp(kTraceEnd);
+#ifdef FLUXB_DEBUG_CHECKS
+      if (p.trace != nullptr && ew == 0 && lane == 0) {
+        uint64_t* tr = p.trace + blockIdx.x * kTraceWords;
+        tr[8] = probe_wait;
+        tr[9] = probe_ld;
+        tr[11] = n;
+        tr[10] = static_cast<uint64_t>(clock64() - probe_t0);
+      }
+#endif
+    } else {
     int pend_seg = -1, pend_mt = 0;
     uint32_t pend_chunks = 0;
     uint32_t own_seen = 0;   // tile rows of the own segment whose W-1 slabs were seen to have landed
@@ -1277,13 +1427,13 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
       const int m_cta = c.m_in_seg + static_cast<int>(cta_rank) * Cfg::BM_CTA;
       const CUtensorMap* tmd = &p.tm_d[0];
       int z = c.seg;
-      if (p.mode == kModeGemmA2A && multi && !started) {
+      if (mode == kModeGemmA2A && multi && !started) {
         if (lane < p.world) flag_wait_ge(wc, p.start_ctr[p.rank] + lane, p.epoch, kSiteStartBarrier);
         __syncwarp();
         started = true;
       }
       bool own_rs = false;
-      if (p.mode == kModeReduceScatter && multi) {
+      if (mode == kModeReduceScatter && multi) {
         tmd = &p.tm_d[c.seg];
         z = p.rank;
         if (c.seg == p.rank && !p.rs_tail) {
@@ -1332,7 +1482,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
         // scales: they read those of the segment's first row
         const int row_s = row < ((p.seg_rows + 127) & ~127) ? row : 0;
         int64_t srow = static_cast<int64_t>(c.seg) * p.seg_rows + row_s;   // row in the scale tensor's frame
-        if (p.mode == kModeAllGather && multi) {
+        if (mode == kModeAllGather && multi) {
           if (c.seg == p.rank) {
             srow = row_s;
           } else {
@@ -1536,7 +1686,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
           emit_chunk(r0, r1, c.n0 + ch * 64, row, grow, m_cta + q * 32, tmd, z, own_rs);
         }
       }
-      if (p.mode == kModeReduceScatter && multi) {
+      if (mode == kModeReduceScatter && multi) {
         // Arrival counting runs one tile behind: waiting for this tile's stores to land would
         // stall the warp for an NVLink round trip, so wait only for the previous tile's (all but
         // the store groups committed for this tile) and count that one.
@@ -1557,14 +1707,14 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
       }
     }
     if (lane == 0) ptx::bulk_wait<0>();
-    if (p.mode == kModeReduceScatter && multi && lane == 0 && pend_seg >= 0) rs_arrive(pend_seg, pend_mt, pend_chunks);
+    if (mode == kModeReduceScatter && multi && lane == 0 && pend_seg >= 0) rs_arrive(pend_seg, pend_mt, pend_chunks);
     __syncwarp();
     if constexpr (Cfg::BS) {
       // (named barrier 1: the eight promotion warps)
-      if (p.mode == kModeReduceScatter && multi && p.rs_tail)
+      if (mode == kModeReduceScatter && multi && p.rs_tail)
         rs_tail(static_cast<int>(threadIdx.x) - 128, [] { asm volatile("bar.sync 1, 256;" ::: "memory"); });
     }
-    if (p.mode == kModeGemmA2A && multi) {
+    if (mode == kModeGemmA2A && multi) {
       // all stores of this warp have landed; the last warp of the whole grid tells every rank,
       // and everybody stays until all W sources have said so: when this kernel completes, the
       // local head-sharded output is complete
@@ -1589,6 +1739,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
       tr[10] = probe_total;   // cycles from this warp's start to the end of its last promotion
     }
 #endif
+    }
   }
 
   // -------------------------------------------------------------------- teardown of the GEMM
@@ -1610,7 +1761,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
 
   // -------------------------------------------------------------------- reduce-scatter tail
   if constexpr (!Cfg::BS)
-    if (p.mode == kModeReduceScatter && multi && p.rs_tail) rs_tail(static_cast<int>(threadIdx.x), [] { __syncthreads(); });
+    if (mode == kModeReduceScatter && multi && p.rs_tail) rs_tail(static_cast<int>(threadIdx.x), [] { __syncthreads(); });
 }
 
 }  // namespace fluxb

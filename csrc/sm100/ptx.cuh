@@ -499,6 +499,22 @@ __device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c) {
   return d;
 }
 
+__device__ __forceinline__ uint64_t fmul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+// shared memory, by address (volatile: kept in order with the barriers around them)
+__device__ __forceinline__ void st_shared_v4_f32(uint32_t saddr, float4 v) {
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+               : "memory");
+}
+__device__ __forceinline__ ulonglong2 ld_shared_v2_b64(uint32_t saddr) {
+  ulonglong2 v;
+  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(saddr));
+  return v;
+}
+
 // epilogue activations: 1 gelu (tanh form), 2 relu, 3 silu
 __device__ __forceinline__ float activate(float x, int kind) {
   if (kind == 1) {

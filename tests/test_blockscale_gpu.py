@@ -86,7 +86,10 @@ def test_blockscale_per_expert_forms_on_side_streams(dev):
     assert abs(total.item() - ref_total) <= 1e-3 * max(1.0, abs(ref_total))
 
 
-@pytest.mark.parametrize("M,N,K", [(256, 384, 512), (1024, 1024, 1024)])
+@pytest.mark.parametrize("M,N,K", [(256, 384, 512), (1024, 1024, 1024),
+                                   (128, 256, 128),        # one k-block: nothing to fetch ahead
+                                   (200, 2176, 384),       # ragged rows, odd k-blocks, half-empty last column tile
+                                   (19 * 128, 2304, 640)])  # more tiles than CTAs: buffers change parity per tile
 def test_blockscale_wgrad_form_per_column_weight_scales(dev, M, N, K):
     """Both operands carry 1x128 scales (weight_scale [N/128, K/128, 128]): the weight-gradient form,
     on the kernel, against the PyTorch statement."""
