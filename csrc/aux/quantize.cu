@@ -30,164 +30,12 @@ namespace {
 constexpr int kTile = 128;
 constexpr int kThreads = 256;
 
-template <typename T>
-__device__ __forceinline__ float to_f32(T v);
-template <>
-__device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
-template <>
-__device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }
-template <>
-__device__ __forceinline__ float to_f32<float>(float v) { return v; }
-
 __device__ __forceinline__ float compute_scale(float amax, float eps, float fp8_max) {
   const float a = fmaxf(amax, eps);
   if (a == 0.f) return 1.f;
   const float s = fp8_max / a;
   if (isinf(s)) return 3.3895313892515355e38f;  // largest finite bf16: the clamp of the reference
   return s;
-}
-
-__device__ __forceinline__ uint8_t to_fp8(float v, bool e5m2) {
-  return static_cast<uint8_t>(
-      __nv_cvt_float_to_fp8(v, __NV_SATFINITE, e5m2 ? __NV_E5M2 : __NV_E4M3));
-}
-
-// One CTA per 128x128 tile. The tile is staged in shared memory in the input type with a
-// padded pitch so that both row-wise and column-wise passes are bank-conflict free.
-template <typename T, bool SQUARE>
-__global__ void __launch_bounds__(kThreads) quant_block_kernel(
-    const T* __restrict__ x, int64_t ldx, uint8_t* __restrict__ q, uint8_t* __restrict__ qt,
-    float* __restrict__ sinv, float* __restrict__ sinv_t, int M, int K, float eps, int e5m2,
-    int64_t batch_stride_x, int64_t batch_stride_q, int64_t batch_stride_s) {
-  constexpr int kPitch = kTile + 16 / sizeof(T);  // elements
-  extern __shared__ __align__(16) uint8_t smem_raw[];
-  T* tile = reinterpret_cast<T*>(smem_raw);
-  __shared__ float red[kThreads / 32];
-  __shared__ float col_scale[kTile];
-
-  const int kb = blockIdx.x, mb = blockIdx.y, bz = blockIdx.z;
-  const int MB = gridDim.y, KB = gridDim.x;
-  x += bz * batch_stride_x;
-  q += bz * batch_stride_q;
-  if (qt) qt += bz * batch_stride_q;
-  sinv += bz * batch_stride_s;
-  if (sinv_t) sinv_t += bz * batch_stride_s;
-  const int row0 = mb * kTile, col0 = kb * kTile;
-  const int rows = min(kTile, M - row0), cols = min(kTile, K - col0);
-  const float fp8_max = e5m2 ? 57344.f : 448.f;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-
-  // ---- load (vectorised when the row pitch allows 16-byte accesses)
-  constexpr int VEC = 16 / sizeof(T);
-  const bool vec_ok = (ldx % VEC == 0) && (cols == kTile) &&
-                      ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
-  if (vec_ok) {
-    for (int i = tid; i < kTile * (kTile / VEC); i += kThreads) {
-      const int r = i / (kTile / VEC), c = (i % (kTile / VEC)) * VEC;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (r < rows) v = *reinterpret_cast<const uint4*>(x + (row0 + r) * ldx + col0 + c);
-      *reinterpret_cast<uint4*>(tile + r * kPitch + c) = v;
-    }
-  } else {
-    for (int i = tid; i < kTile * kTile; i += kThreads) {
-      const int r = i / kTile, c = i % kTile;
-      T v = T(0.f);
-      if (r < rows && c < cols) v = x[(row0 + r) * ldx + col0 + c];
-      tile[r * kPitch + c] = v;
-    }
-  }
-  __syncthreads();
-
-  if constexpr (SQUARE) {
-    // ---- one scale for the whole tile
-    float amax = 0.f;
-    for (int i = tid; i < kTile * kTile; i += kThreads)
-      amax = fmaxf(amax, fabsf(to_f32(tile[(i / kTile) * kPitch + (i % kTile)])));
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    if (lane == 0) red[warp] = amax;
-    __syncthreads();
-    amax = red[0];
-    for (int w = 1; w < kThreads / 32; ++w) amax = fmaxf(amax, red[w]);
-    const float scale = compute_scale(amax, eps, fp8_max);
-    if (tid == 0) {
-      sinv[mb * KB + kb] = 1.f / scale;
-      if (sinv_t) sinv_t[kb * MB + mb] = 1.f / scale;
-    }
-    // rows of q: each lane packs 4 consecutive columns
-    for (int r = warp; r < rows; r += kThreads / 32) {
-      const int c = lane * 4;
-      uint32_t pk = 0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        pk |= static_cast<uint32_t>(to_fp8(to_f32(tile[r * kPitch + c + j]) * scale, e5m2)) << (8 * j);
-      uint8_t* dst = q + static_cast<int64_t>(row0 + r) * K + col0 + c;
-      if (cols == kTile && (K & 3) == 0) {
-        *reinterpret_cast<uint32_t*>(dst) = pk;
-      } else {
-        for (int j = 0; j < 4; ++j)
-          if (c + j < cols) dst[j] = static_cast<uint8_t>(pk >> (8 * j));
-      }
-    }
-    if (qt) {
-      // rows of q_t are columns of the tile; lane l takes rows l, l+32, l+64, l+96 so that a
-      // warp reads 32 different rows (few bank conflicts) and writes 32 consecutive bytes
-      for (int c = warp; c < cols; c += kThreads / 32) {
-        uint8_t* dst = qt + static_cast<int64_t>(col0 + c) * M + row0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int r = lane + 32 * j;
-          if (r < rows) dst[r] = to_fp8(to_f32(tile[r * kPitch + c]) * scale, e5m2);
-        }
-      }
-    }
-  } else {
-    // ---- q: one scale per row of the tile (a warp owns 16 rows)
-    for (int r = warp; r < kTile; r += kThreads / 32) {
-      const int c = lane * 4;
-      float v[4];
-      float amax = 0.f;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        v[j] = to_f32(tile[r * kPitch + c + j]);
-        amax = fmaxf(amax, fabsf(v[j]));
-      }
-      for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-      const float scale = compute_scale(amax, eps, fp8_max);
-      if (lane == 0) sinv[(static_cast<int64_t>(mb) * KB + kb) * kTile + r] = 1.f / scale;
-      if (r < rows) {
-        uint32_t pk = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) pk |= static_cast<uint32_t>(to_fp8(v[j] * scale, e5m2)) << (8 * j);
-        uint8_t* dst = q + static_cast<int64_t>(row0 + r) * K + col0 + c;
-        if (cols == kTile && (K & 3) == 0) {
-          *reinterpret_cast<uint32_t*>(dst) = pk;
-        } else {
-          for (int j = 0; j < 4; ++j)
-            if (c + j < cols) dst[j] = static_cast<uint8_t>(pk >> (8 * j));
-        }
-      }
-    }
-    if (qt) {
-      // ---- q_t: one scale per column of the tile
-      if (tid < kTile) {
-        float amax = 0.f;
-        for (int r = 0; r < kTile; ++r) amax = fmaxf(amax, fabsf(to_f32(tile[r * kPitch + tid])));
-        const float scale = compute_scale(amax, eps, fp8_max);
-        col_scale[tid] = scale;
-        sinv_t[(static_cast<int64_t>(kb) * MB + mb) * kTile + tid] = 1.f / scale;
-      }
-      __syncthreads();
-      for (int c = warp; c < cols; c += kThreads / 32) {
-        const float scale = col_scale[c];
-        uint8_t* dst = qt + static_cast<int64_t>(col0 + c) * M + row0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int r = lane + 32 * j;
-          if (r < rows) dst[r] = to_fp8(to_f32(tile[r * kPitch + c]) * scale, e5m2);
-        }
-      }
-    }
-  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -375,6 +223,267 @@ __global__ void __launch_bounds__(kThreads) quant_tile_kernel(
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// Any other shape, pitch or alignment, and fp32 inputs: the same register tile with guards. What is outside
+// the matrix reads as zero, so the scales of the rows and columns that pad the last blocks are those of
+// zeros. Maxima ignore NaN. An 8-column chunk is read with 16-byte loads where the row pitch and the base
+// allow them and element by element elsewhere; q leaves as 8-byte stores where K allows them. Rows whose
+// start may be on any byte (q with K % 8 != 0, q^T with M % 16 != 0) are written from the shared tile one warp
+// per row, in aligned 32-bit words put together from two neighbouring words of the tile: 128 contiguous bytes
+// per instruction whatever the alignment, and single bytes at the two ends only.
+// Bound by instruction issue, not by memory: 5000 x 8192 bf16, 1x128 with the transpose, takes 44 us (3.7 TB/s);
+// 70 us with one thread per column for the column maxima and byte stores of q^T, 73 us with fp32 maxima and
+// every row of q^T through the word writer (2.7 instructions per cycle and SM either way).
+// ---------------------------------------------------------------------------------------------
+template <typename T>
+struct Chunk8 {      // 8 consecutive elements of a row, as they are in memory
+  static constexpr bool BF16 = std::is_same<T, __nv_bfloat16>::value;
+  static constexpr int NW = 4;                 // words; maxima are taken on pairs
+  uint32_t w[NW];
+  __device__ __forceinline__ uint32_t abs_word(int i) const { return w[i] & 0x7FFF7FFFu; }
+  static __device__ __forceinline__ uint32_t vmax(uint32_t a, uint32_t b) {   // NaN in one operand: the other
+    uint32_t r;
+    if constexpr (BF16) asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    else asm("max.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+  }
+  static __device__ __forceinline__ float column(uint32_t m, int c) { return (c & 1) ? h_hi<BF16>(m) : h_lo<BF16>(m); }
+  static __device__ __forceinline__ float row(uint32_t m) { return fmaxf(h_lo<BF16>(m), h_hi<BF16>(m)); }
+  __device__ __forceinline__ void zero() { w[0] = w[1] = w[2] = w[3] = 0u; }
+  __device__ __forceinline__ void load_vec(const T* p) {
+    const uint4 v = *reinterpret_cast<const uint4*>(p);
+    w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
+  }
+  __device__ __forceinline__ void load_some(const T* p, int n) {
+    zero();
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (j < n) w[j >> 1] |= static_cast<uint32_t>(reinterpret_cast<const uint16_t*>(p)[j]) << (16 * (j & 1));
+  }
+  __device__ __forceinline__ float get(int j) const {
+    return (j & 1) ? h_hi<BF16>(w[j >> 1]) : h_lo<BF16>(w[j >> 1]);
+  }
+};
+template <>
+struct Chunk8<float> {
+  static constexpr int NW = 8;
+  float w[NW];
+  __device__ __forceinline__ uint32_t abs_word(int i) const { return __float_as_uint(fabsf(w[i])); }
+  static __device__ __forceinline__ uint32_t vmax(uint32_t a, uint32_t b) {
+    return __float_as_uint(fmaxf(__uint_as_float(a), __uint_as_float(b)));
+  }
+  static __device__ __forceinline__ float column(uint32_t m, int) { return __uint_as_float(m); }
+  static __device__ __forceinline__ float row(uint32_t m) { return __uint_as_float(m); }
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] = 0.f;
+  }
+  __device__ __forceinline__ void load_vec(const float* p) {
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+    w[0] = a.x, w[1] = a.y, w[2] = a.z, w[3] = a.w;
+    w[4] = b.x, w[5] = b.y, w[6] = b.z, w[7] = b.w;
+  }
+  __device__ __forceinline__ void load_some(const float* p, int n) {
+    zero();
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (j < n) w[j] = p[j];
+  }
+  __device__ __forceinline__ float get(int j) const { return w[j]; }
+};
+
+// A row of a 128 x 128-byte shared tile (word i at i ^ swz) -> n bytes at dst, any alignment; one warp. Lane i
+// writes the aligned word that holds byte 4 * i - a of the row; the bytes before the first and after the last whole
+// word are single stores.
+__device__ __forceinline__ void store_tile_row(const uint32_t* tile_row, int swz, uint8_t* dst, int n, int lane) {
+  const int a = static_cast<int>(reinterpret_cast<uintptr_t>(dst) & 3);
+  const int b0 = 4 * lane - a;
+  const uint32_t hi = tile_row[lane ^ swz];
+  const uint32_t lo = __shfl_up_sync(0xffffffffu, hi, 1);      // (lane 0: its own word, only used below byte 0)
+  const uint32_t word = __funnelshift_l(lo, hi, 8 * a);
+  if (b0 >= 0 && b0 + 4 <= n) {
+    *reinterpret_cast<uint32_t*>(dst + b0) = word;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (b0 + j >= 0 && b0 + j < n) dst[b0 + j] = static_cast<uint8_t>(word >> (8 * j));
+  }
+  if (lane == 31)      // the last a bytes of a full row
+    for (int j = 4 - a; j < 4; ++j)
+      if (124 + j < n) dst[124 + j] = static_cast<uint8_t>(hi >> (8 * j));
+}
+
+template <typename T, bool SQUARE>
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) quant_ragged_kernel(
+    const T* __restrict__ x, int64_t ldx, uint8_t* __restrict__ q, uint8_t* __restrict__ qt,
+    float* __restrict__ sinv, float* __restrict__ sinv_t, int M, int K, float eps, int e5m2,
+    int64_t batch_stride_x, int64_t batch_stride_q, int64_t batch_stride_s) {
+  __shared__ __align__(16) uint32_t colred[kThreads / 32][16 * Chunk8<T>::NW];   // column maxima per warp
+  __shared__ float col_scale[kTile];
+  __shared__ float red[kThreads / 32];
+  __shared__ __align__(16) uint32_t tile[kTile * 32];     // q or q^T: 128 rows x 128 bytes
+  const int kb = blockIdx.x, mb = blockIdx.y, bz = blockIdx.z;
+  const int MB = gridDim.y, KB = gridDim.x;
+  x += bz * batch_stride_x;
+  q += bz * batch_stride_q;
+  if (qt) qt += bz * batch_stride_q;
+  sinv += bz * batch_stride_s;
+  if (sinv_t) sinv_t += bz * batch_stride_s;
+  const int row0 = mb * kTile, col0 = kb * kTile;
+  const int rows = min(kTile, M - row0), cols = min(kTile, K - col0);
+  const float fp8_max = e5m2 ? 57344.f : 448.f;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int chunk = lane & 15;
+  const bool e5 = e5m2 != 0;
+  const int ncol = min(8, cols - chunk * 8);              // columns of this thread's chunk inside the matrix
+  const bool vec_x = ncol == 8 && ldx % (16 / static_cast<int>(sizeof(T))) == 0 &&
+                     (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  const bool vec_q = (K & 7) == 0 && (reinterpret_cast<uintptr_t>(q) & 7) == 0;
+  const bool vec_qt = (M & 15) == 0 && (reinterpret_cast<uintptr_t>(qt) & 15) == 0 && rows == kTile;
+  const bool vec8_qt = (M & 7) == 0 && (reinterpret_cast<uintptr_t>(qt) & 7) == 0;
+
+  // ---- load: pass `it`, row group g = it * 16 + warp * 2 + lane / 16, rows 4g .. 4g + 3
+  Chunk8<T> v[2][4];
+#pragma unroll
+  for (int it = 0; it < 2; ++it)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int row = 4 * (it * 16 + warp * 2 + (lane >> 4)) + r;
+      const T* src = x + static_cast<int64_t>(row0 + row) * ldx + col0 + chunk * 8;
+      if (row < rows && vec_x) v[it][r].load_vec(src);
+      else if (row < rows) v[it][r].load_some(src, ncol);
+      else v[it][r].zero();
+    }
+  // ---- maxima
+  using C = Chunk8<T>;
+  constexpr int NW = C::NW;
+  float row_amax[2][4];
+  uint32_t cm[NW];
+#pragma unroll
+  for (int j = 0; j < NW; ++j) cm[j] = 0u;
+#pragma unroll
+  for (int it = 0; it < 2; ++it)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      uint32_t m = 0u;
+#pragma unroll
+      for (int j = 0; j < NW; ++j) {
+        const uint32_t w = v[it][r].abs_word(j);
+        m = C::vmax(m, w);
+        cm[j] = C::vmax(cm[j], w);
+      }
+      if constexpr (!SQUARE) {
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) m = C::vmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+      }
+      row_amax[it][r] = C::row(m);
+    }
+  float tile_scale = 1.f;
+  if constexpr (SQUARE) {
+    float m = 0.f;
+#pragma unroll
+    for (int it = 0; it < 2; ++it)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) m = fmaxf(m, row_amax[it][r]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0) red[warp] = m;
+    __syncthreads();
+    float amax = red[0];
+#pragma unroll
+    for (int w = 1; w < kThreads / 32; ++w) amax = fmaxf(amax, red[w]);
+    tile_scale = compute_scale(amax, eps, fp8_max);
+    if (tid == 0) {
+      sinv[mb * KB + kb] = 1.f / tile_scale;
+      if (sinv_t) sinv_t[kb * MB + mb] = 1.f / tile_scale;
+    }
+  } else if (qt != nullptr) {
+#pragma unroll
+    for (int j = 0; j < NW; ++j) cm[j] = C::vmax(cm[j], __shfl_xor_sync(0xffffffffu, cm[j], 16));
+    if (lane < 16) {
+#pragma unroll
+      for (int j = 0; j < NW; j += 4)
+        *reinterpret_cast<uint4*>(&colred[warp][chunk * NW + j]) = make_uint4(cm[j], cm[j + 1], cm[j + 2], cm[j + 3]);
+    }
+  }
+  // ---- q
+#pragma unroll
+  for (int it = 0; it < 2; ++it) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int row = 4 * (it * 16 + warp * 2 + (lane >> 4)) + r;
+      float scale = tile_scale;
+      if constexpr (!SQUARE) {
+        scale = compute_scale(row_amax[it][r], eps, fp8_max);
+        if (chunk == 0) sinv[(static_cast<int64_t>(mb) * KB + kb) * kTile + row] = 1.f / scale;
+      }
+      const C& c = v[it][r];
+      uint2 o;
+      o.x = cvt_fp8x2(c.get(0) * scale, c.get(1) * scale, e5) | (cvt_fp8x2(c.get(2) * scale, c.get(3) * scale, e5) << 16);
+      o.y = cvt_fp8x2(c.get(4) * scale, c.get(5) * scale, e5) | (cvt_fp8x2(c.get(6) * scale, c.get(7) * scale, e5) << 16);
+      if (!vec_q) *reinterpret_cast<uint2*>(&tile[row * 32 + chunk * 2]) = o;
+      else if (row < rows && ncol == 8)
+        *reinterpret_cast<uint2*>(q + static_cast<int64_t>(row0 + row) * K + col0 + chunk * 8) = o;
+    }
+  }
+  if (!vec_q) {
+    __syncthreads();
+    for (int r = warp; r < rows; r += kThreads / 32)
+      store_tile_row(&tile[r * 32], 0, q + static_cast<int64_t>(row0 + r) * K + col0, cols, lane);
+  }
+  if (qt == nullptr) return;
+  // ---- q^T (the barrier also ends the reading of a staged q)
+  __syncthreads();
+  if constexpr (!SQUARE) {
+    if (tid < kTile) {
+      uint32_t m = 0u;
+#pragma unroll
+      for (int w = 0; w < kThreads / 32; ++w) m = C::vmax(m, colred[w][NW == 8 ? tid : tid >> 1]);
+      const float s = compute_scale(C::column(m, tid), eps, fp8_max);
+      col_scale[tid] = s;
+      sinv_t[(static_cast<int64_t>(kb) * MB + mb) * kTile + tid] = 1.f / s;
+    }
+    __syncthreads();
+  }
+  // a thread's 4 rows of one column are one word of row c of the transposed tile; word g of row c
+  // sits at g ^ swizzle(c) so that the lanes of a warp hit different banks
+#pragma unroll
+  for (int it = 0; it < 2; ++it) {
+    const int g = it * 16 + warp * 2 + (lane >> 4);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int c = chunk * 8 + j;
+      const float scale = SQUARE ? tile_scale : col_scale[c];
+      tile[c * 32 + (g ^ ((chunk * 4) & 31))] =
+          cvt_fp8x2(v[it][0].get(j) * scale, v[it][1].get(j) * scale, e5) |
+          (cvt_fp8x2(v[it][2].get(j) * scale, v[it][3].get(j) * scale, e5) << 16);
+    }
+  }
+  __syncthreads();
+  if (vec_qt) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int idx = tid + k * kThreads;
+      const int c = idx >> 3, part = idx & 7;
+      if (c < cols)
+        *reinterpret_cast<uint4*>(qt + static_cast<int64_t>(col0 + c) * M + row0 + part * 16) =
+            *reinterpret_cast<const uint4*>(&tile[c * 32 + ((part * 4) ^ (((c >> 3) * 4) & 31))]);
+    }
+  } else if (vec8_qt) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int idx = tid + k * kThreads;
+      const int c = idx >> 4, part = idx & 15;
+      if (c < cols && part * 8 < rows)
+        *reinterpret_cast<uint2*>(qt + static_cast<int64_t>(col0 + c) * M + row0 + part * 8) =
+            *reinterpret_cast<const uint2*>(&tile[c * 32 + ((part * 2) ^ (((c >> 3) * 4) & 31))]);
+    }
+  } else {
+    for (int c = warp; c < cols; c += kThreads / 32)
+      store_tile_row(&tile[c * 32], ((c >> 3) * 4) & 31, qt + static_cast<int64_t>(col0 + c) * M + row0, rows, lane);
+  }
+}
+
 template <typename T, bool SQUARE>
 int launch_quant(const void* x, int64_t ldx, void* q, void* qt, float* sinv, float* sinv_t, int M,
                  int K, int batch, float eps, int e5m2, cudaStream_t stream) {
@@ -396,20 +505,10 @@ int launch_quant(const void* x, int64_t ldx, void* q, void* qt, float* sinv, flo
       return kOk;
     }
   }
-  constexpr int kPitch = kTile + 16 / sizeof(T);
-  constexpr int smem = kTile * kPitch * sizeof(T);
-  static bool configured[64] = {false};
-  int dev = 0;
-  FLUXB_CUDA_OK(cudaGetDevice(&dev));
-  if (smem > 48 * 1024 && (dev >= 64 || !configured[dev])) {
-    FLUXB_CUDA_OK(cudaFuncSetAttribute(quant_block_kernel<T, SQUARE>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    if (dev < 64) configured[dev] = true;
-  }
   const int MB = (M + kTile - 1) / kTile, KB = (K + kTile - 1) / kTile;
   dim3 grid(KB, MB, batch);
   const int64_t sstride = SQUARE ? static_cast<int64_t>(MB) * KB : static_cast<int64_t>(MB) * KB * kTile;
-  quant_block_kernel<T, SQUARE><<<grid, kThreads, smem, stream>>>(
+  quant_ragged_kernel<T, SQUARE><<<grid, kThreads, 0, stream>>>(
       reinterpret_cast<const T*>(x), ldx, reinterpret_cast<uint8_t*>(q),
       reinterpret_cast<uint8_t*>(qt), sinv, sinv_t, M, K, eps, e5m2,
       static_cast<int64_t>(M) * ldx, static_cast<int64_t>(M) * K, sstride);

@@ -61,6 +61,50 @@ def test_quantize_square_blockwise(dev, M, K):
     assert qtb.shape == (2, K, M) and stb.shape[0] == 2
 
 
+@pytest.mark.parametrize("in_dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("M,K,ld,shift", [
+    (1, 8, 8, 0), (127, 129, 129, 0), (129, 257, 264, 0), (200, 1000, 1000, 0), (136, 272, 272, 0), (131, 256, 256, 0),
+    (256, 250, 250, 0), (256, 384, 384, 1), (256, 384, 388, 4), (130, 384, 400, 8), (33, 7, 9, 3)])
+def test_quantize_edges(dev, M, K, ld, shift, in_dtype):
+    """Partial blocks, rows that start on any byte, padded and misaligned inputs: the statement in PyTorch computes
+    the same single-precision quotient, product and rounding, so bytes and scales are equal."""
+    from tempname_new_b200.ops.quantization import (Quantization, quantize_square_blockwise_torch,
+                                                    quantize_vector_blockwise_torch)
+    g = torch.Generator(device=dev).manual_seed(M * 1000 + K)
+    buf = (torch.randn(M * ld + shift + 16, device=dev, generator=g) * 3).to(in_dtype)
+    x = buf[shift:shift + M * ld].view(M, ld)[:, :K]
+    u8 = lambda t: t.contiguous().view(torch.uint8)  # noqa: E731
+    for out in (torch.float8_e4m3fn, torch.float8_e5m2):
+        op = Quantization(in_dtype, out)
+        q, s, qt, st = op.quantize_vector_blockwise(x, True, eps=1e-3)
+        for got, gs, src in ((q, s, x), (qt, st, x.t().contiguous())):
+            ref, ref_s = quantize_vector_blockwise_torch(src, out, 1e-3)
+            assert torch.equal(u8(got), u8(ref))
+            assert torch.equal(gs, ref_s)
+        q, s, qt, st = op.quantize_square_blockwise(x, True)
+        ref, ref_s = quantize_square_blockwise_torch(x, out)
+        assert torch.equal(u8(q), u8(ref)) and torch.equal(u8(qt), u8(ref.t()))
+        assert torch.equal(s, ref_s) and torch.equal(st, ref_s.t())
+    xb = torch.stack([x, -2 * x])
+    qb, sb, qtb, _ = op.batch_quantize_square_blockwise(xb, True)
+    for i in range(2):
+        ref, ref_s = quantize_square_blockwise_torch(xb[i], torch.float8_e5m2)
+        assert torch.equal(u8(qb[i]), u8(ref)) and torch.equal(u8(qtb[i]), u8(ref.t())) and torch.equal(sb[i], ref_s)
+
+
+def test_quantize_edges_ignore_nan(dev):
+    """A block's maximum leaves NaN out (the other values keep their scale) wherever a tile is partial."""
+    from tempname_new_b200.ops.quantization import Quantization
+    for dt in (torch.bfloat16, torch.float16, torch.float32):
+        x = torch.ones(130, 136, device=dev, dtype=dt)
+        x[1, 3] = float("nan")
+        x[129, 135] = -4.0
+        q, s, qt, st = Quantization(dt, torch.float8_e4m3fn).quantize_vector_blockwise(x, True)
+        assert s[0, 0, 1].item() == torch.tensor(1.0 / 448).item() and st[0, 0, 3].item() == s[0, 0, 1].item()
+        assert q[1, 3].float().isnan().item() and q[1, 2].float().item() == 448.0
+        assert s[1, 1, 1].item() == torch.tensor(4.0 / 448).item()
+
+
 @pytest.mark.parametrize("n", [1, 2047, 2048, 4097, 1048580, 1048573, 8388603])
 def test_inplace_cast(dev, n):
     from tempname_new_b200.ops.misc import InplaceCast, inplace_cast_fp32_to_bf16
