@@ -90,7 +90,7 @@ typedef struct {
   int32_t b_kn;              /* 1: b is [K, N] with N contiguous and ldb elements between k-rows (a weight held
                                 transposed, e.g. for the data gradient): read in place as an MN-major operand;
                                 16-bit inputs, not block-scaled */
-  int32_t reserved_tail;
+  int32_t auto_shape;        /* 1: tile_n / cta_group / tile_m / group_m are defaults, the library may pick another kernel */
 } fluxb_dense_args_t;
 
 int fluxb_dense_gemm(const fluxb_dense_args_t* args);

@@ -3,6 +3,7 @@
 #include "../include/fluxb.h"
 #include "../runtime/host_common.h"
 #include "dense_launch.cuh"
+#include "dense_skinny.h"
 
 #include <atomic>
 #include <cstdlib>
@@ -441,6 +442,17 @@ static int dense_impl(const fluxb_dense_args_t* a, const fluxb_a2a_args_t* x) {
       if ((rc = encode_tmap(&p.tm_d[0], out_dt, 3, out, dims, str, box,
                             Swz::B128)))
         return rc;
+      // Too few 128 x 128 tiles for the chip: a cluster of CTAs per tile, each with its share of K
+      if (p.mode == kModePlain && p.num_seg == 1 && p.trace == nullptr &&
+          (a->auto_shape || (a->tile_n == 0 && a->cta_group == 0 && a->tile_m == 0))) {
+        SkinnyShape s;
+        int sms = 0;
+        if ((rc = device_sm_count(&sms))) return rc;
+        if ((rc = fluxb_skinny_shape(a->M, a->N, (a->K + bk - 1) / bk, a->blockscale, sms, &s.bn, &s.tiles, &s.splits)))
+          return rc;
+        if (s.bn != 0 && (a->num_sms <= 0 || a->num_sms >= sms))
+          return dense_skinny(p, s, a, out, ldd, reinterpret_cast<cudaStream_t>(a->stream));
+      }
     }
   }
   if (multi) {

@@ -515,6 +515,15 @@ __device__ __forceinline__ ulonglong2 ld_shared_v2_b64(uint32_t saddr) {
   return v;
 }
 
+// 16 bytes of shared memory of any CTA of the cluster (shared::cluster address, see mapa_u32)
+__device__ __forceinline__ uint4 ld_cluster_v4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared::cluster.v4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "r"(addr));
+  return v;
+}
+
 // epilogue activations: 1 gelu (tanh form), 2 relu, 3 silu
 __device__ __forceinline__ float activate(float x, int kind) {
   if (kind == 1) {

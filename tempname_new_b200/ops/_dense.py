@@ -40,7 +40,7 @@ class DenseArgs(ctypes.Structure):
         ("blockscale", ctypes.c_int32), ("tile_m", ctypes.c_int32),
         ("stream", _VP),
         ("trace", _VP),
-        ("b_kn", ctypes.c_int32), ("reserved_tail", ctypes.c_int32),
+        ("b_kn", ctypes.c_int32), ("auto_shape", ctypes.c_int32),
     ]
 
 
@@ -203,8 +203,10 @@ def base_args(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor], ou
     if keep is not None:
         keep.extend([sa, sb])
     if tile_n == 0 and cta_group == 0 and m is not None:
-        from ..tuning.table import lookup
+        from ..tuning.table import lookup, pinned
         knobs = lookup(m, b.shape[0], a.shape[1], a.element_size())
+        # (a measured or pinned entry is taken as it is; a default may give way to the split-K kernel)
+        args.auto_shape = 0 if pinned(m, b.shape[0], a.shape[1]) or group_m or tile_m else 1
         tile_n, cta_group = knobs["tile_n"], knobs["cta_group"]
         if group_m == 0:
             group_m = knobs["group_m"]

@@ -63,6 +63,7 @@ def blockscale_args(a, w, sa, sb, bias, out_dtype, m, status=None, keep=None) ->
     args = _dense.base_args(a, w, bias, out_dtype, tile_n=tile_n, cta_group=cta_group, m=m, status=status, keep=keep)
     args.sa, args.sb = sa.data_ptr(), sb.data_ptr()
     args.blockscale = 2 if groupwise else 1
+    args.auto_shape = 1 if cta_group == 1 and tile_n == 0 else 0
     return args
 
 

@@ -117,3 +117,9 @@ def lookup(m: int, n: int, k: int, elt: int = 2) -> Dict[str, int]:
     if key in DENSE_TABLE:
         return dict(DENSE_TABLE[key])
     return heuristic(m, n, k, elt)
+
+
+def pinned(m: int, n: int, k: int) -> bool:
+    """True when ``lookup`` answers from a measured or pinned entry rather than from the heuristic."""
+    key = (m, n, k)
+    return key in _OVERRIDE or key in DENSE_TABLE or (_EXTRA is not None and key in _EXTRA)

@@ -114,3 +114,28 @@ def test_blockscale_ragged_rows(dev):
     ref = flux.blockscale_gemm_torch(xq, wq, sx, sw, torch.float32)
     assert out.shape == (M, N)
     assert (out.float() - ref).abs().max().item() <= 2e-2 * max(1.0, ref.abs().max().item())
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 128), (7, 512, 256), (48, 3584, 8192), (128, 8192, 512), (200, 8192, 1152),
+                                   (1000, 2048, 2048), (64, 16384, 640)])
+def test_split_k_block_scaled(dev, M, N, K):
+    """The split-K form against 64 bits and against the persistent kernel: partial row blocks, one to four splits."""
+    from tempname_new_b200.ops import _dense
+    from tempname_new_b200.ops.blockscale_gemm import blockscale_args
+    import tempname_new_b200 as flux
+    g = torch.Generator(device=dev).manual_seed(M + N + K)
+    a, b = (torch.randn(s, device=dev, generator=g).to(torch.float8_e4m3fn) for s in ((M, K), (N, K)))
+    sa = torch.rand((M + 127) // 128, K // 128, 128, device=dev, generator=g) + 0.5
+    sb = torch.rand(N // 128, K // 128, device=dev, generator=g) + 0.5
+    bias = torch.randn(N, device=dev, generator=g).bfloat16()
+    ad = a.double().view(M, K // 128, 128) * sa.double().permute(0, 2, 1).reshape(-1, K // 128)[:M, :, None]
+    bd = b.double().view(N, K // 128, 128) * sb.double().repeat_interleave(128, 0)[:, :, None]
+    ref = ad.reshape(M, K) @ bd.reshape(N, K).t() + bias.double()
+    new = flux.BlockScaleGemm().forward(a, b, bias=bias, input_scale=sa, weight_scale=sb)
+    old = torch.empty(M, N, device=dev, dtype=torch.bfloat16)
+    args = blockscale_args(a, b, sa, sb, bias, torch.bfloat16, M)
+    args.auto_shape, args.tile_n, args.M, args.d, args.ldd = 0, 128, M, old.data_ptr(), N
+    args.mode, args.rank, args.world, args.epoch = _dense.PLAIN, 0, 1, 1
+    _dense.run(args)
+    e_new, e_old = ((t.double() - ref).norm().item() for t in (new, old))
+    assert not new.isnan().any() and e_new <= 1.02 * e_old and e_new <= 2e-3 * ref.norm().item()

@@ -288,3 +288,87 @@ def test_int8_per_row_and_per_column_scales(dev):
     assert (out2.float() - ref2).abs().max().item() <= 1e-2 * max(1.0, ref2.abs().max().item())
     with pytest.raises(ValueError):
         op.forward(a8, b8, input_scale=sa[:7], weight_scale=sb)
+
+
+def _shape_rule(M, N, k_blocks, blockscale=0, sms=148):
+    import ctypes
+    from tempname_new_b200 import _native
+    v = [ctypes.c_int32() for _ in range(3)]
+    _native.check(_native.lib().fluxb_skinny_shape(M, N, k_blocks, blockscale, sms, *map(ctypes.byref, v)), "rule")
+    return tuple(x.value for x in v)
+
+
+# (edges of the 128-row and 64- / 128-column tiles, K remainders, one to four CTAs per tile, both sides of the rule)
+@pytest.mark.parametrize("M,N,K", [
+    (1, 8, 16), (7, 264, 256), (16, 4096, 2048), (64, 1032, 4112), (65, 136, 1040), (127, 512, 8192),
+    (128, 4096, 4096), (129, 1000, 2064), (300, 6144, 4096), (16, 19000, 1024), (600, 3704, 2048),
+    (2000, 1096, 256)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float8_e4m3fn, torch.float8_e5m2, torch.int8])
+def test_split_k(dev, M, N, K, dtype):
+    """The split-K kernel against the product in 64 bits and against the persistent kernel (knobs given): the same
+    fp32 sums in another order, so the outputs differ by an ulp of the 16-bit result here and there, and for int8,
+    whose sums are exact, not at all."""
+    import tempname_new_b200 as flux
+    from tempname_new_b200.ops import _dense
+    g = torch.Generator(device=dev).manual_seed(M + N + K)
+    odt = torch.float16 if dtype == torch.float16 else torch.bfloat16
+    if dtype == torch.int8:
+        a, b = (torch.randint(-127, 128, s, device=dev, generator=g).to(dtype) for s in ((M, K), (N, K)))
+        sa, sb = (torch.rand(s, device=dev, generator=g) * 1e-3 + 1e-4 for s in ((M, 1), (1, N)))
+    else:
+        a, b = (torch.randn(s, device=dev, generator=g).to(dtype) for s in ((M, K), (N, K)))
+        sa = sb = None if dtype.itemsize == 2 else torch.full((1,), 0.5, device=dev)
+    eb = 128 // dtype.itemsize
+    assert _shape_rule(M, N, -(-K // eb))[0] != 0
+    bias = torch.randn(1, N, device=dev, generator=g).to(odt)
+    big = torch.full((M, N + 8), float("nan"), device=dev, dtype=odt)      # (an output with a row pitch)
+    ref = a.double() @ b.double().t()
+    if sa is not None:
+        ref = ref * sa.double() * sb.double()
+    ref = ref + bias.double()
+    out = flux.GemmOnly(dtype, output_dtype=odt, use_fp8_gemm=dtype.itemsize == 1).forward(
+        a, b, bias=bias, output_buf=big[:, :N], input_scale=sa, weight_scale=sb)
+    old = torch.empty(M, N, device=dev, dtype=odt)
+    _dense.plain_gemm(a, b, old, bias, sa, sb, tile_n=128, cta_group=1)
+    assert big[:, N:].isnan().all() and not out.isnan().any()
+    # half a unit in the last place: at most 2^-8 of the value with bf16's 8 significant bits, 2^-11 with fp16's 11;
+    # the fp32 sums of K products err by far less
+    ulp = 2.0 ** (-8 if odt == torch.bfloat16 else -11)
+    assert ((out.double() - ref).abs() <= 1.01 * ulp * ref.abs() + 2e-6 * K ** 0.5 * ref.abs().max()).all()
+    if dtype == torch.int8:
+        assert torch.equal(out, old)
+    e_new, e_old = ((t.double() - ref).norm().item() for t in (out, old))
+    assert e_new <= 1.02 * e_old
+    if dtype.itemsize == 2:      # [K, N] weight read in place, activations
+        for act in ("gelu", "relu", "silu"):
+            new = torch.empty(M, N, device=dev, dtype=odt)
+            _dense.plain_gemm(a, b.t().contiguous().t(), new, bias[0], act=act)
+            _dense.plain_gemm(a, b, old, bias[0], act=act, tile_n=128, cta_group=1)
+            assert (new.double() - old.double()).abs().max() <= 2 * ulp * max(1.0, old.abs().max().item())
+    again = torch.empty(M, N, device=dev, dtype=odt)
+    _dense.plain_gemm(a, b, again, bias, sa, sb)
+    assert torch.equal(again, out)                 # the sum has a fixed order
+
+
+def test_split_k_rule_and_knobs(dev):
+    """Pinned knobs, a margin of SMs and a timeline stay with the persistent kernel; a status word stays clear."""
+    from tempname_new_b200.ops import _dense
+    from tempname_new_b200.tuning import table
+    assert _shape_rule(16, 4096, 256) == (128, 32, 4)
+    assert _shape_rule(128, 4096, 64) == (64, 64, 4)
+    assert _shape_rule(2048, 1024, 64) == (128, 128, 2)
+    assert _shape_rule(4096, 4096, 64)[0] == 0 and _shape_rule(16, 4096, 64, 2)[0] == 0
+    a, b = _ab(16, 512, 1024, dev)
+    out, ref = torch.empty(16, 512, device=dev, dtype=torch.bfloat16), a.float() @ b.float().t()
+    status = torch.zeros(4, dtype=torch.int32, device=dev)
+    for kw in (dict(), dict(num_sms=20), dict(group_m=2)):
+        out.fill_(float("nan"))
+        _dense.plain_gemm(a, b, out, status=status, **kw)
+        assert (out.float() - ref).abs().max().item() <= _tol(ref) and status.tolist()[0] == 0
+    with table.override((16, 512, 1024), {"cta_group": 1, "tile_n": 128, "group_m": 8}):
+        assert table.pinned(16, 512, 1024)
+        _dense.plain_gemm(a, b, out)
+    assert not table.pinned(16, 512, 1024) and (out.float() - ref).abs().max().item() <= _tol(ref)
+    with _dense.KernelTimeline(dev) as tl:
+        _dense.plain_gemm(a, b, out)
+        assert "entry_us" in tl.summary()
