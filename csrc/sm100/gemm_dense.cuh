@@ -1201,13 +1201,29 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
       if (bias != nullptr && col0 < p.N) {
         const uint16_t* brow = bias + (p.bias_row_stride ? grow * p.bias_row_stride : 0);
         const bool row_ok = row < p.seg_rows;
+        if (row_ok && col0 + 64 <= p.N && (reinterpret_cast<uintptr_t>(brow + col0) & 15) == 0) {
+          // eight columns per load (the same address for every lane when one row is broadcast)
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          if (row_ok && col0 + j < p.N)
-            r0[j] = __float_as_uint(__uint_as_float(r0[j]) + ptx::half_bits_to_float(brow[col0 + j], f16));
-          if (row_ok && col0 + 32 + j < p.N)
-            r1[j] = __float_as_uint(__uint_as_float(r1[j]) +
-                                    ptx::half_bits_to_float(brow[col0 + 32 + j], f16));
+          for (int j = 0; j < 8; ++j) {
+            const uint4 b = *reinterpret_cast<const uint4*>(brow + col0 + 8 * j);
+            const uint32_t w[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              uint32_t& lo = j < 4 ? r0[(8 * j + 2 * e) & 31] : r1[(8 * j + 2 * e) & 31];
+              uint32_t& hi = j < 4 ? r0[(8 * j + 2 * e + 1) & 31] : r1[(8 * j + 2 * e + 1) & 31];
+              lo = __float_as_uint(__uint_as_float(lo) + ptx::half_bits_to_float(static_cast<uint16_t>(w[e] & 0xFFFFu), f16));
+              hi = __float_as_uint(__uint_as_float(hi) + ptx::half_bits_to_float(static_cast<uint16_t>(w[e] >> 16), f16));
+            }
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            if (row_ok && col0 + j < p.N)
+              r0[j] = __float_as_uint(__uint_as_float(r0[j]) + ptx::half_bits_to_float(brow[col0 + j], f16));
+            if (row_ok && col0 + 32 + j < p.N)
+              r1[j] = __float_as_uint(__uint_as_float(r1[j]) +
+                                      ptx::half_bits_to_float(brow[col0 + 32 + j], f16));
+          }
         }
       }
       if (p.act != 0) {

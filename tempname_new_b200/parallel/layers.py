@@ -90,11 +90,11 @@ class _ColumnParallelFn(torch.autograd.Function):
 
 class _RowParallelFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, weight, cache: _OpCache):
+    def forward(ctx, x, weight, cache: _OpCache, bias=None):
         op = cache.rs(x.shape[0], weight.shape[0], x.dtype)
-        out = op.forward(x, weight)
+        out = op.forward(x, weight, bias=bias)
         ctx.save_for_backward(x, weight)
-        ctx.cache = cache
+        ctx.cache, ctx.has_bias = cache, bias is not None
         return out
 
     @staticmethod
@@ -109,7 +109,7 @@ class _RowParallelFn(torch.autograd.Function):
         gathered = torch.empty((M, g.shape[1]), dtype=g.dtype, device=g.device)
         grad_x = op.forward(g, weight, transpose_weight=True, gathered_input=gathered)
         grad_w = gathered.t().matmul(x)
-        return grad_x, grad_w, None
+        return grad_x, grad_w, None, (g.sum(0) if ctx.has_bias and ctx.needs_input_grad[3] else None)
 
 
 class ColumnParallelLinear(nn.Module):
@@ -150,8 +150,14 @@ class RowParallelLinear(nn.Module):
         self._cache = _OpCache.shared(self.group)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        b = self.bias
+        if (b is not None and x.is_cuda and dist.get_world_size(self.group) == 1 and b.dtype == x.dtype
+                and b.device == x.device and b.is_contiguous()):
+            # one rank: the GEMM's epilogue adds the bias to the fp32 sum (a broadcast add over 8192 x 12288 bf16
+            # is 235 us next to a GEMM of 970)
+            return _RowParallelFn.apply(x, self.weight, self._cache, b)
         y = _RowParallelFn.apply(x, self.weight, self._cache)
-        return y + self.bias if self.bias is not None else y
+        return y + b if b is not None else y
 
 
 def patch_megatron_linears(model, tp_group=None, row: bool = True, column: bool = True) -> int:

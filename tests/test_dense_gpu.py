@@ -372,3 +372,46 @@ def test_split_k_rule_and_knobs(dev):
     with _dense.KernelTimeline(dev) as tl:
         _dense.plain_gemm(a, b, out)
         assert "entry_us" in tl.summary()
+
+
+@pytest.mark.parametrize("N,shift,rows", [(512, 0, 1), (520, 0, 1), (512, 1, 1), (512, 8, 1), (776, 0, 700), (776, 4, 700)])
+def test_bias_alignment(dev, N, shift, rows):
+    """The epilogue reads a bias 16 bytes at a time where it may and element by element elsewhere: same sums."""
+    from tempname_new_b200.ops import _dense
+    a, b = _ab(700, N, 256, dev)
+    buf = torch.randn(rows * N + shift, device=dev).bfloat16()
+    bias = buf[shift:].view(rows, N)
+    out = torch.full((700, N), float("nan"), device=dev, dtype=torch.bfloat16)
+    for tile_n, cg in ((128, 1), (256, 1), (256, 2)):
+        _dense.plain_gemm(a, b, out, bias, tile_n=tile_n, cta_group=cg)
+        ref = a.float() @ b.float().t() + bias.float()
+        assert (out.float() - ref).abs().max().item() <= _tol(ref)
+
+
+def test_row_parallel_bias_one_rank(dev):
+    """One rank: the bias joins the fp32 sum inside the GEMM, with the gradients of the separate add."""
+    import os
+    import torch.distributed as dist
+    from tempname_new_b200.parallel.layers import RowParallelLinear
+    if not dist.is_initialized():
+        os.environ.setdefault("MASTER_ADDR", "127.0.0.1")
+        os.environ.setdefault("MASTER_PORT", "29551")
+        dist.init_process_group("nccl", rank=0, world_size=1, device_id=dev)
+    lin = RowParallelLinear(256, 520, device=dev)
+    with torch.no_grad():
+        lin.bias.normal_()
+    x = torch.randn(300, 256, device=dev).bfloat16().requires_grad_(True)
+    gy = torch.randn(300, 520, device=dev).bfloat16()
+    y = lin(x)
+    ref = x.detach().float() @ lin.weight.detach().float().t() + lin.bias.detach().float()
+    assert (y.float() - ref).abs().max().item() <= _tol(ref)
+    gx, gw, gb = torch.autograd.grad(y, [x, lin.weight, lin.bias], gy)
+    assert torch.equal(gb, gy.sum(0))
+    for got, want in ((gx, gy.float() @ lin.weight.detach().float()), (gw, gy.float().t() @ x.detach().float())):
+        assert (got.float() - want).abs().max().item() <= _tol(want)
+    lin.bias.requires_grad_(False)
+    assert torch.equal(lin(x), y)
+    with torch.no_grad():
+        wide = RowParallelLinear(256, 520, device=dev)
+        wide.bias = torch.nn.Parameter(torch.zeros(520, device=dev))     # an fp32 bias still promotes the sum
+        assert wide(x).dtype == torch.float32
