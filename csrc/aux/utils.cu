@@ -230,15 +230,17 @@ __global__ void __launch_bounds__(kIdxThreads) moe_hist_kernel(const int32_t* ex
                                                                int E, int32_t* block_hist) {
   extern __shared__ int32_t hist[];
   for (int e = threadIdx.x; e < E; e += kIdxThreads) hist[e] = 0;
-  __syncthreads();
   const int64_t base = static_cast<int64_t>(blockIdx.x) * kIdxPerBlock;
-  for (int i = threadIdx.x; i < kIdxPerBlock; i += kIdxThreads) {
-    const int64_t idx = base + i;
-    if (idx < n) {
-      const int e = experts[idx];
-      if (e >= 0 && e < E) atomicAdd(&hist[e], 1);
-    }
+  int mine[kIdxPerBlock / kIdxThreads];          // all loads in flight before the first count
+#pragma unroll
+  for (int i = 0; i < kIdxPerBlock / kIdxThreads; ++i) {
+    const int64_t idx = base + i * kIdxThreads + threadIdx.x;
+    mine[i] = idx < n ? experts[idx] : -1;
   }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kIdxPerBlock / kIdxThreads; ++i)
+    if (mine[i] >= 0 && mine[i] < E) atomicAdd(&hist[mine[i]], 1);
   __syncthreads();
   for (int e = threadIdx.x; e < E; e += kIdxThreads) block_hist[blockIdx.x * E + e] = hist[e];
 }
@@ -246,70 +248,108 @@ __global__ void __launch_bounds__(kIdxThreads) moe_hist_kernel(const int32_t* ex
 // block_hist[b][e] -> exclusive start of (expert e, block b); splits; offsets
 __global__ void __launch_bounds__(kMaxExperts) moe_scan_kernel(int32_t* block_hist, int nblocks, int E,
                                                                int32_t* splits, int32_t* offsets) {
-  __shared__ int32_t totals[kMaxExperts];
-  const int e = threadIdx.x;
+  __shared__ int32_t warp_sum[kMaxExperts / 32];
+  const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
+  constexpr int kBatch = 16;                      // loads in flight
   int32_t total = 0;
   if (e < E) {
-    for (int b = 0; b < nblocks; ++b) {
-      const int32_t c = block_hist[b * E + e];
-      block_hist[b * E + e] = total;  // exclusive count of expert e in earlier blocks
-      total += c;
+    for (int b0 = 0; b0 < nblocks; b0 += kBatch) {
+      int32_t c[kBatch];
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) c[i] = b0 + i < nblocks ? block_hist[static_cast<int64_t>(b0 + i) * E + e] : 0;
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) total += c[i];
     }
-    totals[e] = total;
     if (splits) splits[e] = total;
   }
-  __syncthreads();
-  if (e == 0) {
-    int32_t run = 0;
-    for (int i = 0; i < E; ++i) {
-      const int32_t c = totals[i];
-      totals[i] = run;
-      offsets[i] = run;
-      run += c;
-    }
-    offsets[E] = run;
+  // exclusive prefix sum over the experts: within the warp, then over the warps
+  int32_t incl = total;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
   }
+  if (lane == 31) warp_sum[warp] = incl;
   __syncthreads();
+  int32_t before = 0;
+  for (int w = 0; w < warp; ++w) before += warp_sum[w];
+  int32_t start = before + incl - total;
   if (e < E) {
-    const int32_t start = totals[e];
-    for (int b = 0; b < nblocks; ++b) block_hist[b * E + e] += start;
+    offsets[e] = start;
+    if (e == E - 1) offsets[E] = start + total;
+    // per block: first row of the expert's entries of that block
+    for (int b0 = 0; b0 < nblocks; b0 += kBatch) {
+      int32_t c[kBatch];
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) c[i] = b0 + i < nblocks ? block_hist[static_cast<int64_t>(b0 + i) * E + e] : 0;
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) {
+        if (b0 + i < nblocks) block_hist[static_cast<int64_t>(b0 + i) * E + e] = start;
+        start += c[i];
+      }
+    }
   }
 }
 
 __global__ void __launch_bounds__(kIdxThreads) moe_place_kernel(
     const int32_t* experts, int64_t n, int E, int topk, const int32_t* block_start,
     int32_t* scatter_index, int32_t* gather_index, int32_t* topk_index) {
-  // running[e]: next free row of expert e for this block; warps are served in order and lanes in
-  // order inside a warp, so equal experts keep their input order
-  extern __shared__ int32_t running[];
-  for (int e = threadIdx.x; e < E; e += kIdxThreads) running[e] = block_start[blockIdx.x * E + e];
-  __syncthreads();
+  // Each warp owns kPerWarp consecutive entries and counts them first; a scan over the warps then gives every
+  // warp the first free row of each expert, and the warps place their entries side by side, 32 at a time, lanes
+  // in order: equal experts keep their input order. (Serving the eight warps in turn for every 256 entries, with
+  // a block barrier each, took 76 us for 65536 entries and 15 for 512.)
+  constexpr int kWarps = kIdxThreads / 32, kPerWarp = kIdxPerBlock / kWarps, kSteps = kPerWarp / 32;
+  extern __shared__ int32_t running[];            // [kWarps][E]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t base = static_cast<int64_t>(blockIdx.x) * kIdxPerBlock;
-  for (int step = 0; step < kIdxPerBlock / kIdxThreads; ++step) {
-    const int64_t idx = base + step * kIdxThreads + threadIdx.x;
-    int e = -1;
-    if (idx < n) {
-      e = experts[idx];
-      if (e < 0 || e >= E) e = -1;
-    }
-    const unsigned peers = __match_any_sync(0xffffffffu, e);
-    const int rank_in_warp = __popc(peers & ((1u << lane) - 1u));
-    const int leader = __ffs(peers) - 1;
-    for (int w = 0; w < kIdxThreads / 32; ++w) {
-      if (w == warp && e >= 0) {
-        int start = 0;
-        if (lane == leader) {
-          start = running[e];
-          running[e] = start + __popc(peers);
-        }
-        start = __shfl_sync(peers, start, leader);
-        const int32_t row = start + rank_in_warp;
-        scatter_index[idx] = row;
-        if (gather_index) gather_index[row] = static_cast<int32_t>(idx / topk);
-        if (topk_index) topk_index[row] = static_cast<int32_t>(idx % topk);
+  const int64_t base = static_cast<int64_t>(blockIdx.x) * kIdxPerBlock + warp * kPerWarp;
+  int32_t* mine = running + warp * E;
+  int32_t start0[(kMaxExperts + kIdxThreads - 1) / kIdxThreads];
+#pragma unroll
+  for (int j = 0; j < (kMaxExperts + kIdxThreads - 1) / kIdxThreads; ++j) {
+    const int e = threadIdx.x + j * kIdxThreads;
+    start0[j] = e < E ? block_start[static_cast<int64_t>(blockIdx.x) * E + e] : 0;
+  }
+  int ex[kSteps];
+#pragma unroll
+  for (int i = 0; i < kSteps; ++i) {
+    const int64_t idx = base + i * 32 + lane;
+    const int e = idx < n ? experts[idx] : -1;
+    ex[i] = e >= 0 && e < E ? e : -1;
+  }
+  for (int e = lane; e < E; e += 32) mine[e] = 0;
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < kSteps; ++i)
+    if (ex[i] >= 0) atomicAdd(&mine[ex[i]], 1);
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < (kMaxExperts + kIdxThreads - 1) / kIdxThreads; ++j) {
+    const int e = threadIdx.x + j * kIdxThreads;
+    if (e < E) {
+      int32_t run = start0[j];
+      for (int w = 0; w < kWarps; ++w) {
+        const int32_t c = running[w * E + e];
+        running[w * E + e] = run;
+        run += c;
       }
-      __syncthreads();
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kSteps; ++i) {
+    const int64_t idx = base + i * 32 + lane;
+    const int e = ex[i];
+    const unsigned peers = __match_any_sync(0xffffffffu, e);
+    const int before = __popc(peers & ((1u << lane) - 1u));
+    int32_t first = 0;
+    if (e >= 0) first = mine[e];
+    __syncwarp();
+    if (e >= 0 && before == 0) mine[e] = first + __popc(peers);
+    __syncwarp();
+    if (e >= 0) {
+      const int32_t row = first + before;
+      scatter_index[idx] = row;
+      if (gather_index) gather_index[row] = static_cast<int32_t>(idx / topk);
+      if (topk_index) topk_index[row] = static_cast<int32_t>(idx % topk);
     }
   }
 }
@@ -419,7 +459,7 @@ extern "C" int fluxb_moe_index_build(const int32_t* experts, int64_t n, int E, i
   const int nblocks = static_cast<int>((n + kIdxPerBlock - 1) / kIdxPerBlock);
   moe_hist_kernel<<<nblocks, kIdxThreads, E * sizeof(int32_t), s>>>(experts, n, E, scratch);
   moe_scan_kernel<<<1, kMaxExperts, 0, s>>>(scratch, nblocks, E, splits, offsets);
-  moe_place_kernel<<<nblocks, kIdxThreads, E * sizeof(int32_t), s>>>(
+  moe_place_kernel<<<nblocks, kIdxThreads, kIdxThreads / 32 * E * sizeof(int32_t), s>>>(
       experts, n, E, topk, scratch, scatter_index, gather_index, topk_index);
   FLUXB_CUDA_OK(cudaGetLastError());
   g_launches.fetch_add(3, std::memory_order_relaxed);
@@ -467,7 +507,7 @@ extern "C" int fluxb_moe_index_build_static(const int32_t* experts, int64_t n, i
   const int nblocks = static_cast<int>(nblocks64);
   moe_hist_kernel<<<nblocks, kIdxThreads, E * sizeof(int32_t), s>>>(experts, n, E, scratch);
   moe_scan_kernel<<<1, kMaxExperts, 0, s>>>(scratch, nblocks, E, splits, offsets);
-  moe_place_kernel<<<nblocks, kIdxThreads, E * sizeof(int32_t), s>>>(
+  moe_place_kernel<<<nblocks, kIdxThreads, kIdxThreads / 32 * E * sizeof(int32_t), s>>>(
       experts, n, E, topk, scratch, scatter_index, gather_index, topk_index);
   FLUXB_CUDA_OK(cudaGetLastError());
   g_launches.fetch_add(3, std::memory_order_relaxed);

@@ -10,6 +10,7 @@
 #include "../runtime/host_common.h"
 #include "../sm100/gemm_grouped.cuh"
 
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <string>
@@ -21,20 +22,47 @@ namespace {
 
 constexpr int kMaxE = 512;
 
-// ---- scatter_index -> gather_index, per-(expert, source rank) counts -------------------------
-__global__ void moe_gather_index_kernel(const int32_t* scatter_index, const int32_t* splits, int64_t n,
-                                        int E, int topk, int tokens_per_rank, int W,
-                                        int32_t* gather_index, int32_t* cnt /* [E][W], zeroed */) {
-  __shared__ int32_t offs[kMaxE + 1];
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int e = 0; e < E; ++e) {
-      offs[e] = run;
-      run += splits[e];
-    }
-    offs[E] = run;
+constexpr int kSchedThreads = 512;
+static_assert(kMaxE <= kSchedThreads, "one thread per expert");
+
+// Exclusive prefix sum over the block's threads (all kSchedThreads of them); `total` gets the sum.
+__device__ __forceinline__ int32_t block_exclusive_sum(int32_t v, int32_t* total) {
+  __shared__ int32_t warp_sum[kSchedThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int32_t incl = v;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
   }
+  __syncthreads();                   // (an earlier call's sums have been read)
+  if (lane == 31) warp_sum[warp] = incl;
   __syncthreads();
+  int32_t before = 0, all = 0;
+#pragma unroll
+  for (int w = 0; w < kSchedThreads / 32; ++w) {
+    if (w < warp) before += warp_sum[w];
+    all += warp_sum[w];
+  }
+  *total = all;
+  return before + incl - v;
+}
+
+// offs[e] = first sorted row of expert e, offs[E] = number of rows
+__device__ __forceinline__ void scan_splits(const int32_t* splits, int E, int32_t* offs) {
+  const int e = threadIdx.x;
+  int32_t total;
+  const int32_t first = block_exclusive_sum(e < E ? splits[e] : 0, &total);
+  if (e < E) offs[e] = first;
+  if (e == 0) offs[E] = total;
+  __syncthreads();
+}
+
+// ---- scatter_index -> gather_index, per-(expert, source rank) counts (several ranks) -----------
+__global__ void __launch_bounds__(kSchedThreads) moe_gather_index_kernel(
+    const int32_t* scatter_index, const int32_t* splits, int64_t n, int E, int topk, int tokens_per_rank, int W,
+    int32_t* gather_index, int32_t* cnt /* [E][W], zeroed */) {
+  __shared__ int32_t offs[kMaxE + 1];
+  scan_splits(splits, E, offs);
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
     const int r = scatter_index[i];
@@ -50,58 +78,57 @@ __global__ void moe_gather_index_kernel(const int32_t* scatter_index, const int3
 }
 
 // ---- schedule: sub-problems (expert, source) in the order this rank should run them ---------
-// With routing_idx the launch has more than one block and all of them also fill row_entry: the
-// index token * topk + k of every sorted row that lives on this rank.
-__global__ void moe_schedule_kernel(const int32_t* splits, const int32_t* cnt /* [E][W] or null */,
-                                    int E, int e0, int E_local, int rank, int W, int n_tiles, int BM,
-                                    SubProblem* sp, int32_t* tile_begin, int32_t* hdr,
-                                    const int32_t* routing_idx, int64_t n_entries, int32_t* row_entry) {
+// Block 0 builds the schedule. With entry_rows (sorted row of every entry token * topk + k) all blocks also fill
+// row_entry (layer 1: the entry of every sorted row that lives on this rank) or gather_index (layer 0 without
+// source ranks: the token of every sorted row). A thread per expert and block-wide prefix sums: 2 us where one
+// thread that walked the experts took 6.
+__global__ void __launch_bounds__(kSchedThreads) moe_schedule_kernel(
+    const int32_t* splits, const int32_t* cnt /* [E][W] or null */, int E, int e0, int E_local, int rank, int W,
+    int n_tiles, int BM, SubProblem* sp, int32_t* tile_begin, int32_t* hdr, const int32_t* entry_rows,
+    int64_t n_entries, int32_t* row_entry, int32_t* gather_index, int topk) {
   __shared__ int32_t offs[kMaxE + 1];
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int e = 0; e < E; ++e) {
-      offs[e] = run;
-      run += splits[e];
-    }
-    offs[E] = run;
-  }
-  __syncthreads();
-  if (routing_idx != nullptr) {
-    const int base = offs[e0], rows = offs[e0 + E_local] - offs[e0];
+  scan_splits(splits, E, offs);
+  const int base = offs[e0], rows = offs[e0 + E_local] - offs[e0];
+  if (entry_rows != nullptr) {
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n_entries; i += stride) {
-      const int r = routing_idx[i] - base;
-      if (r >= 0 && r < rows) row_entry[r] = static_cast<int32_t>(i);
+      const int r = entry_rows[i];
+      if (gather_index != nullptr) gather_index[r] = static_cast<int32_t>(i / topk);
+      else if (r - base >= 0 && r - base < rows) row_entry[r - base] = static_cast<int32_t>(i);
     }
   }
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    hdr[0] = offs[e0];
-    hdr[1] = offs[e0 + E_local] - offs[e0];
-    int tiles = 0, s = 0;
-    if (cnt != nullptr) {
-      for (int step = 0; step < W; ++step) {
-        int src = rank + step;
-        if (src >= W) src -= W;
-        for (int el = 0; el < E_local; ++el, ++s) {
-          const int e = e0 + el;
-          int begin = offs[e];
-          for (int r = 0; r < src; ++r) begin += cnt[e * W + r];
-          const int rows = cnt[e * W + src];
-          sp[s] = SubProblem{begin, begin + rows, el, src};
-          tile_begin[s] = tiles;
-          tiles += ((rows + BM - 1) / BM) * n_tiles;
-        }
-      }
-    } else {
-      for (int el = 0; el < E_local; ++el, ++s) {
-        const int e = e0 + el;
-        sp[s] = SubProblem{offs[e], offs[e + 1], el, -1};
-        tile_begin[s] = tiles;
-        tiles += ((offs[e + 1] - offs[e] + BM - 1) / BM) * n_tiles;
-      }
-    }
-    tile_begin[s] = tiles;
+  if (blockIdx.x != 0) return;
+  if (threadIdx.x == 0) {
+    hdr[0] = base;
+    hdr[1] = rows;
   }
+  // every thread takes `per` consecutive sub-problems
+  const int S = cnt != nullptr ? E_local * W : E_local;
+  const int per = (S + kSchedThreads - 1) / kSchedThreads;
+  const int s0 = threadIdx.x * per, s1 = min(S, s0 + per);
+  auto make = [&](int s) -> SubProblem {
+    const int step = s / E_local, el = s - step * E_local, e = e0 + el;
+    if (cnt == nullptr) return SubProblem{offs[e], offs[e + 1], el, -1};
+    int src = rank + step;
+    if (src >= W) src -= W;
+    int begin = offs[e];
+    for (int r = 0; r < src; ++r) begin += cnt[e * W + r];
+    return SubProblem{begin, begin + cnt[e * W + src], el, src};
+  };
+  int32_t tiles = 0;
+  for (int s = s0; s < s1; ++s) {
+    const SubProblem q = make(s);
+    sp[s] = q;
+    tiles += ((q.row_end - q.row_begin + BM - 1) / BM) * n_tiles;
+  }
+  int32_t total;
+  int32_t t = block_exclusive_sum(tiles, &total);
+  for (int s = s0; s < s1; ++s) {
+    const SubProblem q = make(s);
+    tile_begin[s] = t;
+    t += ((q.row_end - q.row_begin + BM - 1) / BM) * n_tiles;
+  }
+  if (threadIdx.x == 0) tile_begin[S] = total;
 }
 
 // ---- top-k combine + reduce-scatter -----------------------------------------------------------
@@ -290,24 +317,33 @@ extern "C" int fluxb_moe_grouped_gemm(const fluxb_moe_gemm_args_t* a) {
   int32_t* hdr = tile_begin + static_cast<int64_t>(a->E) * a->world + 1;
   int32_t* cnt = hdr + 4;
 
+  const int entry_blocks = static_cast<int>(std::min<int64_t>(148, (a->n_entries + kSchedThreads - 1) / kSchedThreads));
   if (a->gathered) {
     FLUXB_REQUIRE(a->scatter_index && a->gather_index && a->n_entries > 0 && a->topk > 0, "routing indices");
-    FLUXB_CUDA_OK(cudaMemsetAsync(cnt, 0, static_cast<size_t>(a->E) * a->world * 4, stream));
-    moe_gather_index_kernel<<<296, 256, 0, stream>>>(a->scatter_index, a->splits, a->n_entries, a->E, a->topk,
-                                                     a->tokens_per_rank, a->world, a->gather_index, cnt);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
+    if (by_src) {
+      FLUXB_CUDA_OK(cudaMemsetAsync(cnt, 0, static_cast<size_t>(a->E) * a->world * 4, stream));
+      moe_gather_index_kernel<<<entry_blocks, kSchedThreads, 0, stream>>>(a->scatter_index, a->splits, a->n_entries, a->E,
+                                                                          a->topk, a->tokens_per_rank, a->world,
+                                                                          a->gather_index, cnt);
+      g_launches.fetch_add(1, std::memory_order_relaxed);
+    }
   }
   if (a->scatter) {
     FLUXB_REQUIRE(!a->gathered, "the fused combine takes contiguous rows");
     FLUXB_REQUIRE(a->routing_idx && a->row_entry && a->n_entries > 0 && a->topk >= 1 && a->tokens_per_rank > 0 &&
                       a->sc_out && a->local_cnt,
                   "fused combine: routing index / scratch / output missing");
-    moe_schedule_kernel<<<148, 256, 0, stream>>>(a->splits, nullptr, a->E, a->e0, a->E_local, a->rank, a->world,
-                                                 n_tiles, 128, sp, tile_begin, hdr, a->routing_idx, a->n_entries,
-                                                 a->row_entry);
+    moe_schedule_kernel<<<entry_blocks, kSchedThreads, 0, stream>>>(
+        a->splits, nullptr, a->E, a->e0, a->E_local, a->rank, a->world, n_tiles, 128, sp, tile_begin, hdr,
+        a->routing_idx, a->n_entries, a->row_entry, nullptr, a->topk);
+  } else if (a->gathered && !by_src) {
+    moe_schedule_kernel<<<entry_blocks, kSchedThreads, 0, stream>>>(
+        a->splits, nullptr, a->E, a->e0, a->E_local, a->rank, a->world, n_tiles, 128, sp, tile_begin, hdr,
+        a->scatter_index, a->n_entries, nullptr, a->gather_index, a->topk);
   } else {
-    moe_schedule_kernel<<<1, 32, 0, stream>>>(a->splits, by_src ? cnt : nullptr, a->E, a->e0, a->E_local, a->rank,
-                                              a->world, n_tiles, 128, sp, tile_begin, hdr, nullptr, 0, nullptr);
+    moe_schedule_kernel<<<1, kSchedThreads, 0, stream>>>(a->splits, by_src ? cnt : nullptr, a->E, a->e0, a->E_local,
+                                                         a->rank, a->world, n_tiles, 128, sp, tile_begin, hdr, nullptr,
+                                                         0, nullptr, nullptr, 1);
   }
   g_launches.fetch_add(1, std::memory_order_relaxed);
   FLUXB_CUDA_OK(cudaGetLastError());

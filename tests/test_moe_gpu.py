@@ -112,3 +112,51 @@ def test_moe_layer1_fused_fp8(dev):
         ref = y[scatter.reshape(-1).long()].view(tokens, topk, H).sum(1)
         assert (out.float() - ref).abs().max().item() <= 3e-2 * max(1.0, ref.abs().max().item())
     op.check_status()
+
+
+@pytest.mark.parametrize("tokens,E,topk,kind", [(3, 8, 2, "random"), (64, 64, 8, "random"), (64, 64, 1, "one"),
+                                                (300, 128, 2, "few"), (4801, 32, 4, "random"), (4801, 8, 4, "one")])
+def test_moe_layer0_gather_chunks(dev, tokens, E, topk, kind):
+    """Rows are gathered in chunks that may touch several experts (one to four rows each), and an expert is published
+    when its last row is written: empty experts, one-row experts, all rows on one expert, twice on the same op."""
+    import tempname_new_b200 as flux
+    H, ffn = 136, 128
+    g = torch.Generator(device=dev).manual_seed(tokens + E)
+    if kind == "random":
+        chosen = torch.stack([torch.randperm(E, device=dev, generator=g)[:topk] for _ in range(tokens)])
+    elif kind == "one":
+        chosen = torch.arange(topk, device=dev).add(E - topk).repeat(tokens, 1)
+    else:
+        chosen = torch.randint(0, 5, (tokens, topk), device=dev, generator=g) * (E // 5)
+    chosen = chosen.to(torch.int32)
+    splits, _, scatter, gather, _ = flux.moe_index_build(chosen, E)
+    order = torch.argsort(chosen.reshape(-1), stable=True)
+    assert torch.equal(gather, (order // topk).int()) and torch.equal(splits, torch.bincount(chosen.reshape(-1).long(), minlength=E).int())
+    x = torch.randn(tokens, H, device=dev, generator=g).bfloat16()
+    w = [(torch.randn(E, ffn, H, device=dev, generator=g) * 0.2).bfloat16() for _ in range(2)]
+    env = flux.DistEnvTPWithEP(dist.group.WORLD, 1, None, ep_size=1)
+    op = flux.GemmGroupedV3AGScatter(env, flux.MoeArguments(tokens, H, ffn, E, topk, torch.bfloat16, torch.bfloat16))
+    rows = x[order // topk].float()
+    expert = chosen.reshape(-1)[order].long()
+    ref = [torch.empty(tokens * topk, ffn, device=dev) for _ in range(2)]
+    for e in range(E):
+        sel = expert == e
+        for i in range(2):
+            ref[i][sel] = rows[sel] @ w[i][e].float().t()
+    for _ in range(2):
+        for got, want in zip(op.forward_multiple_weights(x, w, splits, scatter), ref):
+            assert (got.float() - want).abs().max().item() <= 1e-2 * max(1.0, want.abs().max().item())
+    op.check_status()
+
+
+@pytest.mark.parametrize("n,E", [(1, 1), (31, 512), (4096, 3), (4097, 64), (20000, 512), (70001, 7)])
+def test_moe_index_build_stable(dev, n, E):
+    """The counting sort is stable across lanes, warps and blocks."""
+    import tempname_new_b200 as flux
+    chosen = torch.randint(0, E, (n,), device=dev, dtype=torch.int32)
+    splits, offsets, scatter, gather, tki = flux.moe_index_build(chosen, E)
+    order = torch.argsort(chosen, stable=True)
+    assert torch.equal(splits.long(), torch.bincount(chosen.long(), minlength=E))
+    assert torch.equal(offsets.long(), torch.cat([offsets.new_zeros(1).long(), splits.long().cumsum(0)]))
+    assert torch.equal(scatter[order].long(), torch.arange(n, device=dev)) and torch.equal(gather.long(), order)
+    assert (tki == 0).all()
