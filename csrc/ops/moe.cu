@@ -461,6 +461,7 @@ extern "C" int fluxb_moe_grouped_gemm(const fluxb_moe_gemm_args_t* a) {
       return e ? atoi(e) : 0;   // measured slower at four ranks: 1.97 against 1.88 ms for layer 0
     }();
     p.comm_split = split_env;
+
   }
   // (the cp.async variant keeps its own producer warps per tile and is left alone)
   if (wave_env != 0 && !(a->gathered && gather_mode == 1)) p.wave_ctr = wave_counter_for(stream);

@@ -1,8 +1,8 @@
 // Dense GEMM core for sm_100a: D[M,N] = A[M,K] * B[N,K]^T (+bias), fp32 accumulation in TMEM.
 //
 // One persistent CTA per SM, 8 warps with fixed roles:
-//   warp 0      TMA producer    (one lane): A/B k-blocks -> shared-memory ring
-//   warp 1      MMA issuer      (one lane): tcgen05.mma from the ring into one of two TMEM
+//   warp 0      TMA producer    (one elected lane): A/B k-blocks -> shared-memory ring
+//   warp 1      MMA issuer      (one elected lane): tcgen05.mma from the ring into one of two TMEM
 //                                accumulators; tcgen05.commit frees ring slots / publishes tiles
 //   warps 2,3   communication   cross-rank "everyone entered this call" handshake; in all-gather
 //                                mode they push this rank's A shard into every peer's landing
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
   const uint32_t ring_bar_base = bar_base + 8u * (2 * STAGES + 2 * NACC) + 16u;
   static_assert(8 * (2 * STAGES + 2 * NACC) + 16 + 64 + 16 <= Cfg::BAR_BYTES, "barrier block too small");
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = ptx::warp_index();
   const int lane = threadIdx.x & 31;
   constexpr int CG = Cfg::CG;
   // position inside the CTA pair (CG == 2): rank 0 leads (issues the MMAs, owns the barriers
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
   ptx::tc_fence_before();
   if constexpr (CG == 2) ptx::cluster_sync(); else __syncthreads();
   ptx::tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   WaitCtx wc{p.status, abort_word, p.timeout_ns};
   auto stamp = [&](int slot) {
@@ -478,7 +478,10 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
   if constexpr (Cfg::BS) ptx::setmaxnreg_dec<Cfg::REGS_LEAD>();
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    // (the whole warp walks the tiles and waits, one elected lane issues: see elect_one. With one lane doing
+    // both, a k-block took 0.55 us whatever the tile: 128 x 256 tiles 1227 -> 1410 TFLOP/s, 256 x 256 pairs 1263 ->
+    // 1473 at 65536 x 1536 x 4096 bf16, 1024 x 3072 x 5120 fp16 46 -> 36 us.)
+    {
       int stage = 0;
       uint32_t phase = 0;
       const uint32_t full_owner0 = CG == 2 ? ptx::mapa_u32(full_bar(0), 0) : full_bar(0);
@@ -487,9 +490,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
       const uint64_t pol_a = ptx::l2_policy_evict_last(), pol_b = ptx::l2_policy_evict_first();
       uint64_t ag_seen = 0;               // all-gather: shard units seen to have arrived
       uint32_t a2a_seen[kMaxRanks] = {};  // post-attention: row units seen, per source
-      stamp(kTraceEntry);
+      if (lane == 0) stamp(kTraceEntry);
       for (int t = tile_slot; t < total_tiles; t += tile_stride, ++wave) {
-        if (*abort_word) break;   // a wait gave up: issue nothing more
+        if (__any_sync(0xffffffffu, *abort_word)) break;   // a wait gave up: issue nothing more
         const TileCoord c = decode_tile(p, t, m_tiles_seg, n_tiles, BM, BN);
         if (!dcheck(wc, c.seg >= 0 && c.seg < p.num_seg && c.m_in_seg >= 0 && c.m_in_seg < p.seg_rows &&
                             c.n0 >= 0 && c.n0 < n_tiles * BN,   // (a piece of a split edge tile may lie past N)
@@ -497,7 +500,8 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
           break;
         if (p.wave_ctr != nullptr && leader && wave > 0) {
           const uint32_t need = min(static_cast<uint32_t>(wave) * tile_stride, static_cast<uint32_t>(total_tiles));
-          flag_wait_ge(wc, p.wave_ctr, need, kSiteStartBarrier);
+          if (lane == 0) flag_wait_ge(wc, p.wave_ctr, need, kSiteStartBarrier);
+          __syncwarp();
         }
         const CUtensorMap* tma = &p.tm_a;
         const CUtensorMap* tmb = c.shift == 0 ? &p.tm_b : (c.shift == 1 ? &p.tm_b_half : &p.tm_b_quarter);
@@ -516,7 +520,8 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
             const int fi = c.seg * ag_units + c.m_in_seg / p.flag_unit_rows;
             if (fi >= 64 || ((ag_seen >> fi) & 1ull) == 0ull) {
               const uint64_t w0 = p.trace != nullptr ? ptx::globaltimer_ns() : 0;
-              flag_wait_ge(wc, p.ag_flags[p.rank] + fi, p.epoch, kSiteShardFlag);
+              if (lane == 0) flag_wait_ge(wc, p.ag_flags[p.rank] + fi, p.epoch, kSiteShardFlag);
+              __syncwarp();
               ptx::fence_proxy_async_all();
               if (fi < 64) ag_seen |= 1ull << fi;
               if (p.trace != nullptr) flag_ns += ptx::globaltimer_ns() - w0;
@@ -546,20 +551,21 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
             in_place = own_in_place && src == p.rank;
             if (kin == 0 && !in_place && (a2a_unit >= 32 || ((a2a_seen[src] >> a2a_unit) & 1u) == 0u)) {
               const uint64_t w0 = p.trace != nullptr ? ptx::globaltimer_ns() : 0;
-              flag_wait_ge(wc, a2a_flag_row + src * a2a_units, p.epoch, kSiteA2AFlag);
+              if (lane == 0) flag_wait_ge(wc, a2a_flag_row + src * a2a_units, p.epoch, kSiteA2AFlag);
+              __syncwarp();
               ptx::fence_proxy_async_all();
               if (a2a_unit < 32) a2a_seen[src] |= 1u << a2a_unit;
               if (p.trace != nullptr) {
                 flag_ns += ptx::globaltimer_ns() - w0;
                 int j = p.rank - src;
                 if (j < 0) j += p.world;
-                if (wave == 0) stamp(kTraceSlice0 + j);
+                if (wave == 0 && lane == 0) stamp(kTraceSlice0 + j);
               }
             }
           }
           // (a wait that gave up, here or in another role: stop issuing at once, so that what is in flight
           // at the teardown is bounded by the depth of the pipeline)
-          if (!mbar_wait(wc, empty_bar(stage), phase ^ 1u, kSiteSmemEmpty)) break;
+          if (!mbar_wait_warp(wc, empty_bar(stage), phase ^ 1u, kSiteSmemEmpty)) break;
           const uint32_t sa = smem_base + stage * Cfg::STAGE_BYTES;
           // post-attention input: (column in head, head of the slice, source); the own slice comes
           // straight from the attention output
@@ -571,6 +577,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
             kin = 0;
             src = src == 0 ? p.world - 1 : src - 1;
           }
+          if (ptx::elect_one()) {
           if constexpr (CG == 1) {
             ptx::mbar_arrive_expect_tx(full_bar(stage), stage_tx);
             if (in_place) ptx::tma_load_4d(sa, &p.tm_a_own, full_bar(stage), own_col, own_s, own_head, own_b);
@@ -599,24 +606,27 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
             } else if (p.l2_hints) ptx::tma_load_2d_cg2_hint(sa + Cfg::A_BYTES, tmb, fb, kb * BK, b_row, pol_b);
             else ptx::tma_load_2d_cg2(sa + Cfg::A_BYTES, tmb, fb, kb * BK, b_row);
           }
+          }
+          __syncwarp();
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
           }
         }
-        if (p.wave_ctr != nullptr && leader) {
+        if (p.wave_ctr != nullptr && leader && lane == 0) {
           // this tile's loads are all issued; whoever issues the last tile of the launch puts the
           // counter back to zero (every wait of the launch is for a smaller value)
           if (atomicAdd(p.wave_ctr, 1u) == static_cast<uint32_t>(total_tiles) - 1u) atomicExch(p.wave_ctr, 0u);
         }
-        if (wave == 0) stamp(kTraceFirstLoads);
+        if (wave == 0 && lane == 0) stamp(kTraceFirstLoads);
+        __syncwarp();
       }
-      stamp(kTraceLastLoads);
-      if (p.trace != nullptr) p.trace[blockIdx.x * kTraceWords + kTraceFlagWait] = flag_ns;
+      if (lane == 0) stamp(kTraceLastLoads);
+      if (p.trace != nullptr && lane == 0) p.trace[blockIdx.x * kTraceWords + kTraceFlagWait] = flag_ns;
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && leader) {
+    // ------------------------------------------------------------------ MMA issuer (likewise)
+    if (leader) {
       // one instruction covers 128 rows per CTA of the group
       // B as [K, N] (16-bit inputs): MN-major operand tiles - 64-column groups BK * 128 bytes apart, 8-k-row
       // groups 1024 bytes apart, one UMMA_K step = 16 k-rows of 128 bytes
@@ -635,7 +645,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
       uint64_t probe_tempty = 0, probe_full = 0;
 #endif
       for (int t = tile_slot; t < total_tiles; t += tile_stride, ++it) {
-        if (*abort_word) break;
+        if (__any_sync(0xffffffffu, *abort_word)) break;
         // a column piece of a split tile is a narrower instruction on the same operands
         const int shift = t >= p.split_from ? p.split_shift : 0;
         const uint32_t idesc = shift == 0 ? idesc_full
@@ -649,11 +659,11 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
 #ifdef FLUXB_DEBUG_CHECKS
             const long long pc0 = clock64();
 #endif
-            if (!mbar_wait(wc, tempty_bar(buf), ((n / NACC) & 1u) ^ 1u, kSiteTmemEmpty)) break;
+            if (!mbar_wait_warp(wc, tempty_bar(buf), ((n / NACC) & 1u) ^ 1u, kSiteTmemEmpty)) break;
 #ifdef FLUXB_DEBUG_CHECKS
             const long long pc1 = clock64();
 #endif
-            if (!mbar_wait(wc, full_bar(stage), phase, kSiteSmemFull)) break;
+            if (!mbar_wait_warp(wc, full_bar(stage), phase, kSiteSmemFull)) break;
 #ifdef FLUXB_DEBUG_CHECKS
             // self-checking build: cycles the issuer waited for a free TMEM buffer / for operands
             probe_tempty += static_cast<uint64_t>(pc1 - pc0);
@@ -663,17 +673,20 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
             const uint32_t sa = smem_base + stage * Cfg::STAGE_BYTES;
             const uint64_t adesc = ptx::umma_desc_k_sw128(sa);
             const uint64_t bdesc = ptx::umma_desc_k_sw128(sa + Cfg::A_BYTES);
+            if (ptx::elect_one()) {
 #pragma unroll
-            for (int k = 0; k < BK / Cfg::UMMA_K; ++k)
-              ptx::umma_ss<CG, Cfg::KIND>(tmem_base + buf * BN, adesc + 2u * k, bdesc + 2u * k, idesc,
-                                          k != 0 ? 1u : 0u);
-            if constexpr (CG == 1) {
-              ptx::umma_commit(empty_bar(stage));
-              ptx::umma_commit(tfull_bar(buf));
-            } else {
-              ptx::umma_commit_cg2(empty_bar(stage), 3);
-              ptx::umma_commit_cg2(tfull_bar(buf), 3);
+              for (int k = 0; k < BK / Cfg::UMMA_K; ++k)
+                ptx::umma_ss<CG, Cfg::KIND>(tmem_base + buf * BN, adesc + 2u * k, bdesc + 2u * k, idesc,
+                                            k != 0 ? 1u : 0u);
+              if constexpr (CG == 1) {
+                ptx::umma_commit(empty_bar(stage));
+                ptx::umma_commit(tfull_bar(buf));
+              } else {
+                ptx::umma_commit_cg2(empty_bar(stage), 3);
+                ptx::umma_commit_cg2(tfull_bar(buf), 3);
+              }
             }
+            __syncwarp();
             if (++stage == STAGES) {
               stage = 0;
               phase ^= 1u;
@@ -688,83 +701,92 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
           // k-blocks into accumulator 1 (which releases their stages).
           const uint32_t par_e = (static_cast<uint32_t>(it) & 1u) ^ 1u;
           const int head = k_blocks < STAGES ? k_blocks : STAGES;
-          auto issue_half = [&](int st, int half, bool first) {
+          auto issue_half = [&](int st, int half, bool first, bool release) {
             const uint32_t sa = smem_base + st * Cfg::STAGE_BYTES;
             const uint64_t adesc = ptx::umma_desc_k_sw128(sa + half * Cfg::A_HALF_BYTES);
             const uint64_t bdesc = make_bdesc(sa + Cfg::A_BYTES);
+            if (ptx::elect_one()) {
 #pragma unroll
-            for (int k = 0; k < BK / Cfg::UMMA_K; ++k)
-              ptx::umma_ss<CG, Cfg::KIND>(tmem_base + half * BN, adesc + 2u * k, bdesc + bstep * k, idesc,
-                                          (!first || k != 0) ? 1u : 0u);
+              for (int k = 0; k < BK / Cfg::UMMA_K; ++k)
+                ptx::umma_ss<CG, Cfg::KIND>(tmem_base + half * BN, adesc + 2u * k, bdesc + bstep * k, idesc,
+                                            (!first || k != 0) ? 1u : 0u);
+              if (release) ptx::umma_commit_cg2(empty_bar(st), 3);
+            }
+            __syncwarp();
           };
-          if (!mbar_wait(wc, tempty_bar(0), par_e, kSiteTmemEmpty)) break;
+          if (!mbar_wait_warp(wc, tempty_bar(0), par_e, kSiteTmemEmpty)) break;
           ptx::tc_fence_after();
           {
             int st = stage;
             uint32_t ph = phase;
             for (int kb = 0; kb < head; ++kb) {
-              if (!mbar_wait(wc, full_bar(st), ph, kSiteSmemFull)) break;
+              if (!mbar_wait_warp(wc, full_bar(st), ph, kSiteSmemFull)) break;
               ptx::tc_fence_after();
-              issue_half(st, 0, kb == 0);
+              issue_half(st, 0, kb == 0, false);
               if (++st == STAGES) {
                 st = 0;
                 ph ^= 1u;
               }
             }
           }
-          if (*abort_word || !mbar_wait(wc, tempty_bar(1), par_e, kSiteTmemEmpty)) break;
+          if (__any_sync(0xffffffffu, *abort_word) || !mbar_wait_warp(wc, tempty_bar(1), par_e, kSiteTmemEmpty)) break;
           ptx::tc_fence_after();
           for (int kb = 0; kb < head; ++kb) {
-            issue_half(stage, 1, kb == 0);
-            ptx::umma_commit_cg2(empty_bar(stage), 3);
+            issue_half(stage, 1, kb == 0, true);
             if (++stage == STAGES) {
               stage = 0;
               phase ^= 1u;
             }
           }
           for (int kb = head; kb < k_blocks; ++kb) {
-            if (!mbar_wait(wc, full_bar(stage), phase, kSiteSmemFull)) break;
+            if (!mbar_wait_warp(wc, full_bar(stage), phase, kSiteSmemFull)) break;
             ptx::tc_fence_after();
-            issue_half(stage, 0, false);
-            issue_half(stage, 1, false);
-            ptx::umma_commit_cg2(empty_bar(stage), 3);
+            issue_half(stage, 0, false, false);
+            issue_half(stage, 1, false, true);
             if (++stage == STAGES) {
               stage = 0;
               phase ^= 1u;
             }
           }
-          ptx::umma_commit_cg2(tfull_bar(0), 3);
+          if (ptx::elect_one()) ptx::umma_commit_cg2(tfull_bar(0), 3);
+          __syncwarp();
           continue;
         }
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(wc, tempty_bar(acc), acc_phase ^ 1u, kSiteTmemEmpty)) break;
+        if (!mbar_wait_warp(wc, tempty_bar(acc), acc_phase ^ 1u, kSiteTmemEmpty)) break;
         ptx::tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!mbar_wait(wc, full_bar(stage), phase, kSiteSmemFull)) break;
+          if (!mbar_wait_warp(wc, full_bar(stage), phase, kSiteSmemFull)) break;
           ptx::tc_fence_after();
           const uint32_t sa = smem_base + stage * Cfg::STAGE_BYTES;
           const uint64_t adesc = ptx::umma_desc_k_sw128(sa);
           const uint64_t bdesc = make_bdesc(sa + Cfg::A_BYTES);
+          if (ptx::elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / Cfg::UMMA_K; ++k) {
-            // 32 bytes per UMMA_K step inside the 128-byte swizzled row: +2 in 16-byte units
-            ptx::umma_ss<CG, Cfg::KIND>(d_tmem, adesc + 2u * k, bdesc + bstep * k, idesc,
-                                        (kb | k) != 0 ? 1u : 0u);
+            for (int k = 0; k < BK / Cfg::UMMA_K; ++k) {
+              // 32 bytes per UMMA_K step inside the 128-byte swizzled row: +2 in 16-byte units
+              ptx::umma_ss<CG, Cfg::KIND>(d_tmem, adesc + 2u * k, bdesc + bstep * k, idesc,
+                                          (kb | k) != 0 ? 1u : 0u);
+            }
+            if constexpr (CG == 1) ptx::umma_commit(empty_bar(stage));
+            else ptx::umma_commit_cg2(empty_bar(stage), 3);
           }
-          if constexpr (CG == 1) ptx::umma_commit(empty_bar(stage));
-          else ptx::umma_commit_cg2(empty_bar(stage), 3);
+          __syncwarp();
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
           }
         }
-        if constexpr (CG == 1) ptx::umma_commit(tfull_bar(acc));
-        else ptx::umma_commit_cg2(tfull_bar(acc), 3);
+        if (ptx::elect_one()) {
+          if constexpr (CG == 1) ptx::umma_commit(tfull_bar(acc));
+          else ptx::umma_commit_cg2(tfull_bar(acc), 3);
+        }
+        __syncwarp();
       }
 #ifdef FLUXB_DEBUG_CHECKS
-      if (Cfg::BS && p.trace != nullptr) {
+      if (Cfg::BS && p.trace != nullptr && lane == 0) {
         p.trace[blockIdx.x * kTraceWords + 12] = probe_tempty;
         p.trace[blockIdx.x * kTraceWords + 13] = probe_full;
       }
@@ -1298,11 +1320,10 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
       // scales and added to fp32 registers. Warp (quadrant q, half) owns rows q*32.. and the 128 columns of one
       // scale block of the weight for the whole tile. 128 accumulators and 32 staging registers leave about 40
       // for everything else, so nothing that can be computed again is kept across the loop.
-      // Measured at 8192 x 3584 x 8192 / 8192 x 8192 x 3584 (one 128 x 256 tile per SM and k-block takes 477 ns
-      // without any promotion, the operand stream being the bound): square 303 / 283 us, 320 / 306 before with the
-      // general loop below (two polls of the full barrier and spills); per column 379 / 355 us, 1340 / 1128 before,
-      // when every warp read the column scales from global memory where it multiplied by them. Sixteen warps
-      // of 64 columns: 358 and 667 us. Register splits 24 / 240 and 56 / 224: within 2 % of 40 / 232.
+      // Measured at 8192 x 3584 x 8192: square 252 us (303 while one lane walked the issue loops, 320 with the
+      // general loop below: two polls of the full barrier and spills); per column 360 us (379; 1340 before,
+      // when every warp read the column scales from global memory where it multiplied by them). Sixteen warps
+      // of 64 columns, with the one-lane loops: 358 and 667 us. Register splits 24 / 240 and 56 / 224: within 2 % of 40 / 232.
       constexpr bool kColumn = Cfg::BS_FORM == kBsColumn;
       const int half = ew >> 2;
       const int kbs = k_blocks;

@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
   const uint32_t ring_bar_base = bar_base + 8u * (2 * STAGES + 4) + 16u;
   static_assert(8 * (2 * STAGES + 4) + 16 + 64 <= Cfg::BAR_BYTES, "barrier block too small");
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       // B arrives by TMA (one arrival + bytes); gathered A adds one arrival per producer thread
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   WaitCtx wc{p.status, abort_word, p.timeout_ns};
 
   const int n_tiles = (p.N + BN - 1) / BN;
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
     uint32_t phase = 0;
     int32_t* idx_buf = reinterpret_cast<int32_t*>(bar_ptr + 256);
     for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++nt) {
-      if (*abort_word) break;   // a wait gave up: issue nothing more
+      if (__any_sync(0xffffffffu, *abort_word)) break;   // a wait gave up: issue nothing more
       const GroupedTile g = grouped_decode(p, t, cursor, n_tiles, BM, BN);
       int32_t* idx = idx_buf + (nt & 1) * 128;
       if constexpr (Cfg::GATHER4) {
@@ -193,8 +193,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
           // tokens of this source must have landed (sub-problems are ordered by source, own first)
           if (lane == 0) {
             flag_wait_ge(wc, p.ag_flags[p.rank] + g.src, p.epoch, kSiteMoeFlag);
-            ptx::fence_proxy_async_all();
           }
+          __syncwarp();
+          ptx::fence_proxy_async_all();
           ready_src = g.src;
         }
         // the 128 token ids of this tile (rows past the end of the sub-problem read token 0; their
@@ -212,21 +213,24 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
         if (g.sp != ready_src) {
           if (lane == 0) {
             flag_wait_ge(wc, p.local_cnt + kGatherFlagBase + g.sp, p.epoch, kSiteMoeFlag);
-            ptx::fence_proxy_async_all();
           }
+          __syncwarp();
+          ptx::fence_proxy_async_all();
           ready_src = g.sp;
         }
       }
-      if (lane == 0) {
-        // wave-synchronous starts: tile nt of this CTA waits until every CTA has issued the loads
-        // of its tile nt - 1, which keeps the CTAs on neighbouring tiles and k ranges (L2 reuse)
-        if (p.wave_ctr != nullptr && nt > 0) {
-          const uint32_t need = min(static_cast<uint32_t>(nt) * gridDim.x, static_cast<uint32_t>(total_tiles));
-          flag_wait_ge(wc, p.wave_ctr, need, kSiteStartBarrier);
-        }
-        for (int kb = 0; kb < k_blocks; ++kb) {
-          mbar_wait(wc, empty_bar(stage), phase ^ 1u, kSiteSmemEmpty);
-          const uint32_t sa = smem_base + stage * Cfg::STAGE_BYTES;
+      // wave-synchronous starts: tile nt of this CTA waits until every CTA has issued the loads
+      // of its tile nt - 1, which keeps the CTAs on neighbouring tiles and k ranges (L2 reuse)
+      if (p.wave_ctr != nullptr && nt > 0) {
+        const uint32_t need = min(static_cast<uint32_t>(nt) * gridDim.x, static_cast<uint32_t>(total_tiles));
+        if (lane == 0) flag_wait_ge(wc, p.wave_ctr, need, kSiteStartBarrier);
+      }
+      __syncwarp();
+      // the whole warp walks the k-blocks, one elected lane issues
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        mbar_wait_warp(wc, empty_bar(stage), phase ^ 1u, kSiteSmemEmpty);
+        const uint32_t sa = smem_base + stage * Cfg::STAGE_BYTES;
+        if (ptx::elect_one()) {
           if constexpr (Cfg::GATHER) {
             ptx::mbar_arrive_expect_tx(full_bar(stage), Cfg::B_BYTES);
           } else if constexpr (Cfg::GATHER4) {
@@ -240,47 +244,52 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
             ptx::tma_load_2d(sa, &p.tm_a, full_bar(stage), kb * BK, g.row0 - row_base);
           }
           ptx::tma_load_3d(sa + Cfg::A_BYTES, &p.tm_b, full_bar(stage), kb * BK, g.n0, g.expert);
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
         }
-        if (p.wave_ctr != nullptr &&
-            atomicAdd(p.wave_ctr, 1u) == static_cast<uint32_t>(total_tiles) - 1u)
-          atomicExch(p.wave_ctr, 0u);   // last tile of the launch: every wait was for a smaller value
+        __syncwarp();
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1u;
+        }
       }
+      if (p.wave_ctr != nullptr && lane == 0 &&
+          atomicAdd(p.wave_ctr, 1u) == static_cast<uint32_t>(total_tiles) - 1u)
+        atomicExch(p.wave_ctr, 0u);   // last tile of the launch: every wait was for a smaller value
       __syncwarp();
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    // ------------------------------------------------------------------ MMA issuer (likewise)
+    {
       const uint32_t idesc = ptx::umma_idesc(p.ab_fmt, p.ab_fmt, BM, BN);
       int stage = 0, it = 0;
       uint32_t phase = 0;
       for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++it) {
-        if (*abort_word) break;   // a wait gave up: issue nothing more
+        if (__any_sync(0xffffffffu, *abort_word)) break;   // a wait gave up: issue nothing more
         const int acc = it & 1;
-        mbar_wait(wc, tempty_bar(acc), (((it >> 1) & 1) ^ 1u), kSiteTmemEmpty);
+        mbar_wait_warp(wc, tempty_bar(acc), (((it >> 1) & 1) ^ 1u), kSiteTmemEmpty);
         ptx::tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < k_blocks; ++kb) {
-          mbar_wait(wc, full_bar(stage), phase, kSiteSmemFull);
+          mbar_wait_warp(wc, full_bar(stage), phase, kSiteSmemFull);
           // gathered A rows were written through the generic proxy (cp.async)
           if constexpr (Cfg::GATHER) ptx::fence_proxy_async_smem();
           ptx::tc_fence_after();
           const uint32_t sa = smem_base + stage * Cfg::STAGE_BYTES;
           const uint64_t adesc = ptx::umma_desc_k_sw128(sa);
           const uint64_t bdesc = ptx::umma_desc_k_sw128(sa + Cfg::A_BYTES);
+          if (ptx::elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / Cfg::UMMA_K; ++k)
-            ptx::umma_ss<1, Cfg::KIND>(d_tmem, adesc + 2u * k, bdesc + 2u * k, idesc, (kb | k) != 0 ? 1u : 0u);
-          ptx::umma_commit(empty_bar(stage));
+            for (int k = 0; k < BK / Cfg::UMMA_K; ++k)
+              ptx::umma_ss<1, Cfg::KIND>(d_tmem, adesc + 2u * k, bdesc + 2u * k, idesc, (kb | k) != 0 ? 1u : 0u);
+            ptx::umma_commit(empty_bar(stage));
+          }
+          __syncwarp();
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
           }
         }
-        ptx::umma_commit(tfull_bar(acc));
+        if (ptx::elect_one()) ptx::umma_commit(tfull_bar(acc));
+        __syncwarp();
       }
     }
   } else if (warp == 2 || warp == 3) {

@@ -10,8 +10,8 @@
 // them whatever lies behind in the ring (inside this CTA's shared memory), and those rows of D are never read.
 //
 //   warps 0..3  epilogue (TMEM lane quadrant = warp); block-scaled: they also promote every k-block
-//   warp 4      TMA producer (one lane)
-//   warp 5      MMA issuer (one lane)
+//   warp 4      TMA producer
+//   warp 5      MMA issuer
 #pragma once
 
 #include "gemm_dense.cuh"
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 2) skinny_gemm_kernel(const __gr
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_ptr + kWords);
   volatile uint32_t* abort_word = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
   const int S = p.splits;
   const int rank = S > 1 ? static_cast<int>(ptx::cluster_ctarank()) : 0;
   const int tile = blockIdx.x / S;
@@ -113,18 +113,19 @@ __global__ void __launch_bounds__(Cfg::THREADS, 2) skinny_gemm_kernel(const __gr
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   WaitCtx wc{p.status, abort_word, p.timeout_ns};
 
   uint32_t facc[Cfg::BS ? BN : 1];   // block-scaled: this thread's row of the tile, fp32
   if (warp == 4) {
-    if (lane == 0) {
-      const bool b_kn = Cfg::KIND == 0 && p.b_kn != 0;
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        if (!mbar_wait(wc, empty_bar(stage), phase ^ 1u, kSiteSmemEmpty)) break;
-        const uint32_t sb = b_base + stage * Cfg::B_BYTES;
+    // (the whole warp walks the k-blocks, one elected lane issues)
+    const bool b_kn = Cfg::KIND == 0 && p.b_kn != 0;
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      if (!mbar_wait_warp(wc, empty_bar(stage), phase ^ 1u, kSiteSmemEmpty)) break;
+      const uint32_t sb = b_base + stage * Cfg::B_BYTES;
+      if (ptx::elect_one()) {
         ptx::mbar_arrive_expect_tx(full_bar(stage), static_cast<uint32_t>(a_bytes + Cfg::B_BYTES));
         if (b_kn) {
 #pragma unroll
@@ -134,43 +135,46 @@ __global__ void __launch_bounds__(Cfg::THREADS, 2) skinny_gemm_kernel(const __gr
           ptx::tma_load_2d(sb, &p.tm_b, full_bar(stage), kb * BK, n0);
         }
         ptx::tma_load_2d(smem_base + stage * a_bytes, &p.tm_a, full_bar(stage), kb * BK, m0);
-        if (++stage == p.stages) {
-          stage = 0;
-          phase ^= 1u;
-        }
+      }
+      __syncwarp();
+      if (++stage == p.stages) {
+        stage = 0;
+        phase ^= 1u;
       }
     }
-    __syncwarp();
   } else if (warp == 5) {
-    if (lane == 0) {
-      const bool b_kn = Cfg::KIND == 0 && p.b_kn != 0;
-      const uint32_t bstep = b_kn ? static_cast<uint32_t>(Cfg::UMMA_K * 128) >> 4 : 2u;
-      const uint32_t idesc = ptx::umma_idesc(p.ab_fmt, p.ab_fmt, 128, BN, 0, b_kn ? 1u : 0u, Cfg::KIND == 2 ? 2u : 1u);
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        const uint32_t n = static_cast<uint32_t>(kb - kb0);
-        const uint32_t buf = n % Cfg::ACC_BUFS;
-        if (Cfg::BS && !mbar_wait(wc, tempty_bar(buf), ((n / Cfg::ACC_BUFS) & 1u) ^ 1u, kSiteTmemEmpty)) break;
-        if (!mbar_wait(wc, full_bar(stage), phase, kSiteSmemFull)) break;
-        ptx::tc_fence_after();
-        const uint64_t adesc = ptx::umma_desc_k_sw128(smem_base + stage * a_bytes);
-        const uint32_t sb = b_base + stage * Cfg::B_BYTES;
-        const uint64_t bdesc = b_kn ? ptx::umma_desc_mn_sw128(sb, BK * 128, 1024) : ptx::umma_desc_k_sw128(sb);
+    const bool b_kn = Cfg::KIND == 0 && p.b_kn != 0;
+    const uint32_t bstep = b_kn ? static_cast<uint32_t>(Cfg::UMMA_K * 128) >> 4 : 2u;
+    const uint32_t idesc = ptx::umma_idesc(p.ab_fmt, p.ab_fmt, 128, BN, 0, b_kn ? 1u : 0u, Cfg::KIND == 2 ? 2u : 1u);
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      const uint32_t n = static_cast<uint32_t>(kb - kb0);
+      const uint32_t buf = n % Cfg::ACC_BUFS;
+      if (Cfg::BS && !mbar_wait_warp(wc, tempty_bar(buf), ((n / Cfg::ACC_BUFS) & 1u) ^ 1u, kSiteTmemEmpty)) break;
+      if (!mbar_wait_warp(wc, full_bar(stage), phase, kSiteSmemFull)) break;
+      ptx::tc_fence_after();
+      const uint64_t adesc = ptx::umma_desc_k_sw128(smem_base + stage * a_bytes);
+      const uint32_t sb = b_base + stage * Cfg::B_BYTES;
+      const uint64_t bdesc = b_kn ? ptx::umma_desc_mn_sw128(sb, BK * 128, 1024) : ptx::umma_desc_k_sw128(sb);
+      if (ptx::elect_one()) {
 #pragma unroll
         for (int k = 0; k < BK / Cfg::UMMA_K; ++k)
           ptx::umma_ss<1, Cfg::KIND>(tmem_base + buf * BN, adesc + 2u * k, bdesc + bstep * k, idesc,
                                      (k != 0 || (!Cfg::BS && n != 0)) ? 1u : 0u);
         ptx::umma_commit(empty_bar(stage));
         if constexpr (Cfg::BS) ptx::umma_commit(tfull_bar(buf));
-        if (++stage == p.stages) {
-          stage = 0;
-          phase ^= 1u;
-        }
       }
-      if constexpr (!Cfg::BS) ptx::umma_commit(tfull_bar(0));
+      __syncwarp();
+      if (++stage == p.stages) {
+        stage = 0;
+        phase ^= 1u;
+      }
     }
-    __syncwarp();
+    if constexpr (!Cfg::BS) {
+      if (ptx::elect_one()) ptx::umma_commit(tfull_bar(0));
+      __syncwarp();
+    }
   } else {
     const bool live = warp * 32 < rows;            // some row of this quadrant exists
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
