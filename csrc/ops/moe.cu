@@ -267,7 +267,23 @@ int launch_grouped(const GroupedParams& p, int grid, cudaStream_t stream) {
                                        Cfg::SMEM_BYTES));
     if (dev < 64) configured[dev] = true;
   }
-  grouped_gemm_kernel<Cfg><<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(p);
+  if constexpr (Cfg::CG == 1) {
+    grouped_gemm_kernel<Cfg><<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(p);
+  } else {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid & ~1, 1, 1);
+    cfg.blockDim = dim3(Cfg::THREADS, 1, 1);
+    cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    FLUXB_CUDA_OK(cudaLaunchKernelEx(&cfg, grouped_gemm_kernel<Cfg>, p));
+  }
   FLUXB_CUDA_OK(cudaGetLastError());
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return kOk;
@@ -305,8 +321,27 @@ extern "C" int fluxb_moe_grouped_gemm(const fluxb_moe_gemm_args_t* a) {
   const CUtensorMapDataType in_dt = in8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   FLUXB_REQUIRE((a->K * elt) % 16 == 0, "K row bytes must be a multiple of 16");
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(a->stream);
+  // gathered rows: by default the communication warps copy them into a sorted buffer (when the
+  // caller provides one); FLUXB_MOE_GATHER=cpasync | gather4 selects the in-loader variants
+  static const int gather_mode = [] {
+    const char* e = getenv("FLUXB_MOE_GATHER");
+    if (e && std::string(e) == "cpasync") return 1;
+    if (e && std::string(e) == "gather4") return 2;
+    return 3;
+  }();
   const int bn = (a->N % 256 == 0 || a->N > 1024) ? 256 : 128;
+  int sms = 0, rc;
+  if ((rc = device_sm_count(&sms))) return rc;
   const int n_tiles = (a->N + bn - 1) / bn;
+  // CTA pairs on 256 x 256 tiles from 768 rows per expert on. They read a third less per k-block, but pad every expert
+  // to a multiple of 256 rows. Single -> pair, us, E x N x K with random routing: 1024 rows per expert 668 -> 632
+  // (64 x 1536 x 4096), 234 -> 196 (16 x 4096 x 1536), 626 -> 569 (64 x 2816 x 2048); 512 rows 368 -> 367, 127 -> 123,
+  // 352 -> 329 and 79 -> 86 (8 x 3072 x 2048); 256 rows 233 -> 238; 64 rows 145 -> 175. One rank only: the flags of
+  // the exchange with other ranks are the business of single CTAs.
+  const int64_t rows_here = a->n_entries > 0 ? a->n_entries * a->E_local / a->E : a->a_rows;
+  const bool pair = bn == 256 && a->world == 1 && sms >= 2 && rows_here >= 768 * static_cast<int64_t>(a->E_local) &&
+                    (!a->gathered || (gather_mode == 3 && a->a_sorted != nullptr && a->E_local <= 512));
+  const int bm = pair ? 256 : 128;
   const bool by_src = a->gathered && a->world > 1 && a->do_allgather;
   const int64_t S = by_src ? static_cast<int64_t>(a->E_local) * a->world : a->E_local;
 
@@ -334,15 +369,15 @@ extern "C" int fluxb_moe_grouped_gemm(const fluxb_moe_gemm_args_t* a) {
                       a->sc_out && a->local_cnt,
                   "fused combine: routing index / scratch / output missing");
     moe_schedule_kernel<<<entry_blocks, kSchedThreads, 0, stream>>>(
-        a->splits, nullptr, a->E, a->e0, a->E_local, a->rank, a->world, n_tiles, 128, sp, tile_begin, hdr,
+        a->splits, nullptr, a->E, a->e0, a->E_local, a->rank, a->world, n_tiles, bm, sp, tile_begin, hdr,
         a->routing_idx, a->n_entries, a->row_entry, nullptr, a->topk);
   } else if (a->gathered && !by_src) {
     moe_schedule_kernel<<<entry_blocks, kSchedThreads, 0, stream>>>(
-        a->splits, nullptr, a->E, a->e0, a->E_local, a->rank, a->world, n_tiles, 128, sp, tile_begin, hdr,
+        a->splits, nullptr, a->E, a->e0, a->E_local, a->rank, a->world, n_tiles, bm, sp, tile_begin, hdr,
         a->scatter_index, a->n_entries, nullptr, a->gather_index, a->topk);
   } else {
     moe_schedule_kernel<<<1, kSchedThreads, 0, stream>>>(a->splits, by_src ? cnt : nullptr, a->E, a->e0, a->E_local,
-                                                         a->rank, a->world, n_tiles, 128, sp, tile_begin, hdr, nullptr,
+                                                         a->rank, a->world, n_tiles, bm, sp, tile_begin, hdr, nullptr,
                                                          0, nullptr, nullptr, 1);
   }
   g_launches.fetch_add(1, std::memory_order_relaxed);
@@ -372,22 +407,13 @@ extern "C" int fluxb_moe_grouped_gemm(const fluxb_moe_gemm_args_t* a) {
   p.epoch = a->epoch;
   p.timeout_ns = a->timeout_ns ? a->timeout_ns : 5000000000ull;
   p.status = reinterpret_cast<Status*>(a->status);
-  int rc;
   {
     uint64_t dims[3] = {static_cast<uint64_t>(a->K), static_cast<uint64_t>(a->N), static_cast<uint64_t>(a->E_local)};
     uint64_t str[2] = {static_cast<uint64_t>(a->K) * elt, static_cast<uint64_t>(a->K) * elt * a->N};
-    uint32_t box[3] = {bk, static_cast<uint32_t>(bn), 1};
+    uint32_t box[3] = {bk, static_cast<uint32_t>(pair ? 128 : bn), 1};
     if ((rc = encode_tmap(&p.tm_b, in_dt, 3, a->weights, dims, str, box, Swz::B128)))
       return rc;
   }
-  // gathered rows: by default the communication warps copy them into a sorted buffer (when the
-  // caller provides one); FLUXB_MOE_GATHER=cpasync | gather4 selects the in-loader variants
-  static const int gather_mode = [] {
-    const char* e = getenv("FLUXB_MOE_GATHER");
-    if (e && std::string(e) == "cpasync") return 1;
-    if (e && std::string(e) == "gather4") return 2;
-    return 3;
-  }();
   static const int wave_env = [] {
     const char* e = getenv("FLUXB_MOE_WAVE_SYNC");
     return e ? atoi(e) : 0;
@@ -448,8 +474,6 @@ extern "C" int fluxb_moe_grouped_gemm(const fluxb_moe_gemm_args_t* a) {
     if ((rc = encode_tmap(&p.tm_a, in_dt, 2, a->a, dims, str, box, Swz::B128)))
       return rc;
   }
-  int sms = 0;
-  if ((rc = device_sm_count(&sms))) return rc;
   {
     static const int inflight_env = [] {
       const char* e = getenv("FLUXB_MOE_INFLIGHT");
@@ -461,7 +485,6 @@ extern "C" int fluxb_moe_grouped_gemm(const fluxb_moe_gemm_args_t* a) {
       return e ? atoi(e) : 0;   // measured slower at four ranks: 1.97 against 1.88 ms for layer 0
     }();
     p.comm_split = split_env;
-
   }
   // (the cp.async variant keeps its own producer warps per tile and is left alone)
   if (wave_env != 0 && !(a->gathered && gather_mode == 1)) p.wave_ctr = wave_counter_for(stream);
@@ -469,17 +492,21 @@ extern "C" int fluxb_moe_grouped_gemm(const fluxb_moe_gemm_args_t* a) {
     // 8-bit operands (tcgen05 kind::f8f6f4): contiguous A, the sorted-buffer gather and the fused combine
     FLUXB_REQUIRE(!a->gathered || pregather, "fp8 grouped GEMM gathers rows through the sorted buffer only");
     if (pregather) {
+      if (pair) return launch_grouped<GroupedCfg<256, 1, 6, 3, false, 2>>(p, sms, stream);
       if (bn == 256) return launch_grouped<GroupedCfg<256, 1, 4, 3>>(p, sms, stream);
       return launch_grouped<GroupedCfg<128, 1, 5, 3>>(p, sms, stream);
     }
     if (a->scatter) {
+      if (pair) return launch_grouped<GroupedCfg<256, 1, 6, 0, true, 2>>(p, sms, stream);
       if (bn == 256) return launch_grouped<GroupedCfg<256, 1, 4, 0, true>>(p, sms, stream);
       return launch_grouped<GroupedCfg<128, 1, 6, 0, true>>(p, sms, stream);
     }
+    if (pair) return launch_grouped<GroupedCfg<256, 1, 6, 0, false, 2>>(p, sms, stream);
     if (bn == 256) return launch_grouped<GroupedCfg<256, 1, 4, 0>>(p, sms, stream);
     return launch_grouped<GroupedCfg<128, 1, 6, 0>>(p, sms, stream);
   }
   if (pregather) {
+    if (pair) return launch_grouped<GroupedCfg<256, 0, 6, 3, false, 2>>(p, sms, stream);
     if (bn == 256) return launch_grouped<GroupedCfg<256, 0, 4, 3>>(p, sms, stream);
     return launch_grouped<GroupedCfg<128, 0, 5, 3>>(p, sms, stream);
   }
@@ -493,9 +520,11 @@ extern "C" int fluxb_moe_grouped_gemm(const fluxb_moe_gemm_args_t* a) {
   }
   if (a->scatter) {
     // every CTA takes part in the arrival counting and in the tail: full grid
+    if (pair) return launch_grouped<GroupedCfg<256, 0, 6, 0, true, 2>>(p, sms, stream);
     if (bn == 256) return launch_grouped<GroupedCfg<256, 0, 4, 0, true>>(p, sms, stream);
     return launch_grouped<GroupedCfg<128, 0, 6, 0, true>>(p, sms, stream);
   }
+  if (pair) return launch_grouped<GroupedCfg<256, 0, 6, 0, false, 2>>(p, sms, stream);
   if (bn == 256) return launch_grouped<GroupedCfg<256, 0, 4, 0>>(p, sms, stream);
   return launch_grouped<GroupedCfg<128, 0, 6, 0>>(p, sms, stream);
 }

@@ -74,11 +74,15 @@ struct GroupedParams {
 // 2 = gathered A rows by TMA tile::gather4 (four indexed rows per instruction) from the producer lane;
 // 3 = the communication warps copy the gathered rows, whole rows at a time, into an expert-sorted
 //     buffer as soon as their source shard has landed, and the GEMM reads that buffer by TMA.
-template <int BN_, int KIND_, int STAGES_, int GATHER_, bool SCATTER_ = false>
+// CG_ = 2: a pair of CTAs (one cluster) shares a 256 x 256 tile as in the dense kernel: each CTA loads its 128 rows of A
+//     and half of the expert's 256 weight rows, the leader issues the MMAs of both, each epilogue has its own 128 rows.
+template <int BN_, int KIND_, int STAGES_, int GATHER_, bool SCATTER_ = false, int CG_ = 1>
 struct GroupedCfg {
+  static constexpr int CG = CG_;
+  static_assert(CG_ == 1 || (BN_ == 256 && (GATHER_ == 0 || GATHER_ == 3)), "pairs: 256 columns, A by tiled TMA loads");
   static constexpr bool SCATTER = SCATTER_;        // layer 1: rows go to the token owner's [token][k] slot
   static_assert(!SCATTER_ || GATHER_ == 0, "the scatter epilogue reads contiguous A");
-  static constexpr int BM = 128, BN = BN_, KIND = KIND_, STAGES = STAGES_;
+  static constexpr int BM = 128 * CG_, BN = BN_, KIND = KIND_, STAGES = STAGES_;   // (BM: rows of a tile)
   static constexpr bool GATHER = GATHER_ == 1;     // cp.async producers
   static constexpr bool GATHER4 = GATHER_ == 2;    // TMA gather4
   static constexpr bool PREGATHER = GATHER_ == 3;  // rows copied into a sorted buffer by the comm warps
@@ -86,7 +90,7 @@ struct GroupedCfg {
   static constexpr int ELT = KIND_ == 0 ? 2 : 1;
   static constexpr int BK = 128 / ELT;
   static constexpr int UMMA_K = 32 / ELT;
-  static constexpr int A_BYTES = BM * 128, B_BYTES = BN * 128, STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int A_BYTES = 128 * 128, B_BYTES = BN / CG_ * 128, STAGE_BYTES = A_BYTES + B_BYTES;   // per CTA
   // scatter epilogue: every epilogue warp stages 32 rows x 64 columns (128 bytes per row, 144-byte
   // pitch so that the lanes' 16-byte writes fall into different banks) before the rows leave as
   // one bulk copy each
@@ -148,6 +152,10 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
   static_assert(8 * (2 * STAGES + 4) + 16 + 64 <= Cfg::BAR_BYTES, "barrier block too small");
 
   const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
+  constexpr int CG = Cfg::CG;
+  const uint32_t cta_rank = CG == 2 ? ptx::cluster_ctarank() : 0u;   // rank 0 of a pair leads
+  const bool leader = cta_rank == 0;
+  const int tile_first = blockIdx.x / CG, tile_stride = gridDim.x / CG;
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       // B arrives by TMA (one arrival + bytes); gathered A adds one arrival per producer thread
@@ -156,7 +164,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
     }
     for (int a = 0; a < 2; ++a) {
       ptx::mbar_init(tfull_bar(a), 1);
-      ptx::mbar_init(tempty_bar(a), 4);
+      ptx::mbar_init(tempty_bar(a), 4 * CG);
     }
     for (int i = 0; i < 8; ++i) ptx::mbar_init(ring_bar_base + 8u * i, 1);
     *abort_word = 0;
@@ -164,11 +172,11 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
     ptx::prefetch_tmap(&p.tm_b);
   }
   if (warp == 1) {
-    ptx::tmem_alloc<1>(ptx::smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
-    ptx::tmem_relinquish<1>();
+    ptx::tmem_alloc<CG>(ptx::smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
+    ptx::tmem_relinquish<CG>();
   }
   ptx::tc_fence_before();
-  __syncthreads();
+  if constexpr (CG == 2) ptx::cluster_sync(); else __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   WaitCtx wc{p.status, abort_word, p.timeout_ns};
@@ -184,7 +192,8 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
     int stage = 0, cursor = 0, ready_src = -1, nt = 0;
     uint32_t phase = 0;
     int32_t* idx_buf = reinterpret_cast<int32_t*>(bar_ptr + 256);
-    for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++nt) {
+    const uint32_t full_owner0 = CG == 2 ? ptx::mapa_u32(full_bar(0), 0) : full_bar(0);   // the leader counts both CTAs' bytes
+    for (int t = tile_first; t < total_tiles; t += tile_stride, ++nt) {
       if (__any_sync(0xffffffffu, *abort_word)) break;   // a wait gave up: issue nothing more
       const GroupedTile g = grouped_decode(p, t, cursor, n_tiles, BM, BN);
       int32_t* idx = idx_buf + (nt & 1) * 128;
@@ -221,8 +230,8 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
       }
       // wave-synchronous starts: tile nt of this CTA waits until every CTA has issued the loads
       // of its tile nt - 1, which keeps the CTAs on neighbouring tiles and k ranges (L2 reuse)
-      if (p.wave_ctr != nullptr && nt > 0) {
-        const uint32_t need = min(static_cast<uint32_t>(nt) * gridDim.x, static_cast<uint32_t>(total_tiles));
+      if (p.wave_ctr != nullptr && nt > 0 && leader) {
+        const uint32_t need = min(static_cast<uint32_t>(nt) * tile_stride, static_cast<uint32_t>(total_tiles));
         if (lane == 0) flag_wait_ge(wc, p.wave_ctr, need, kSiteStartBarrier);
       }
       __syncwarp();
@@ -239,11 +248,18 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
             for (int i = 0; i < 32; ++i)
               ptx::tma_gather4_2d(sa + i * 512, &p.tm_a, full_bar(stage), kb * BK, idx[4 * i], idx[4 * i + 1],
                                   idx[4 * i + 2], idx[4 * i + 3]);
+          } else if constexpr (CG == 2) {
+            // (the second CTA's rows may lie past the end of the sub-problem: they read what follows, and the
+            // results are never stored)
+            const uint32_t fb = full_owner0 + 8u * stage;
+            if (leader) ptx::mbar_arrive_expect_tx(full_bar(stage), 2 * Cfg::STAGE_BYTES);
+            ptx::tma_load_2d_cg2(sa, &p.tm_a, fb, kb * BK, g.row0 - row_base + static_cast<int>(cta_rank) * 128);
+            ptx::tma_load_3d_cg2(sa + Cfg::A_BYTES, &p.tm_b, fb, kb * BK, g.n0 + static_cast<int>(cta_rank) * (BN / 2), g.expert);
           } else {
             ptx::mbar_arrive_expect_tx(full_bar(stage), Cfg::STAGE_BYTES);
             ptx::tma_load_2d(sa, &p.tm_a, full_bar(stage), kb * BK, g.row0 - row_base);
           }
-          ptx::tma_load_3d(sa + Cfg::A_BYTES, &p.tm_b, full_bar(stage), kb * BK, g.n0, g.expert);
+          if constexpr (CG == 1) ptx::tma_load_3d(sa + Cfg::A_BYTES, &p.tm_b, full_bar(stage), kb * BK, g.n0, g.expert);
         }
         __syncwarp();
         if (++stage == STAGES) {
@@ -251,18 +267,18 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
           phase ^= 1u;
         }
       }
-      if (p.wave_ctr != nullptr && lane == 0 &&
+      if (p.wave_ctr != nullptr && lane == 0 && leader &&
           atomicAdd(p.wave_ctr, 1u) == static_cast<uint32_t>(total_tiles) - 1u)
         atomicExch(p.wave_ctr, 0u);   // last tile of the launch: every wait was for a smaller value
       __syncwarp();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (likewise)
-    {
+    if (leader) {
       const uint32_t idesc = ptx::umma_idesc(p.ab_fmt, p.ab_fmt, BM, BN);
       int stage = 0, it = 0;
       uint32_t phase = 0;
-      for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++it) {
+      for (int t = tile_first; t < total_tiles; t += tile_stride, ++it) {
         if (__any_sync(0xffffffffu, *abort_word)) break;   // a wait gave up: issue nothing more
         const int acc = it & 1;
         mbar_wait_warp(wc, tempty_bar(acc), (((it >> 1) & 1) ^ 1u), kSiteTmemEmpty);
@@ -279,8 +295,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
           if (ptx::elect_one()) {
 #pragma unroll
             for (int k = 0; k < BK / Cfg::UMMA_K; ++k)
-              ptx::umma_ss<1, Cfg::KIND>(d_tmem, adesc + 2u * k, bdesc + 2u * k, idesc, (kb | k) != 0 ? 1u : 0u);
-            ptx::umma_commit(empty_bar(stage));
+              ptx::umma_ss<CG, Cfg::KIND>(d_tmem, adesc + 2u * k, bdesc + 2u * k, idesc, (kb | k) != 0 ? 1u : 0u);
+            if constexpr (CG == 1) ptx::umma_commit(empty_bar(stage));
+            else ptx::umma_commit_cg2(empty_bar(stage), 3);
           }
           __syncwarp();
           if (++stage == STAGES) {
@@ -288,7 +305,10 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
             phase ^= 1u;
           }
         }
-        if (ptx::elect_one()) ptx::umma_commit(tfull_bar(acc));
+        if (ptx::elect_one()) {
+          if constexpr (CG == 1) ptx::umma_commit(tfull_bar(acc));
+          else ptx::umma_commit_cg2(tfull_bar(acc), 3);
+        }
         __syncwarp();
       }
     }
@@ -411,11 +431,12 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
             if (!p.by_src) {
               // No source ranks: the rows of all experts are one run of the sorted order, dealt out in chunks of a
               // few rows. Each chunk adds its rows to its expert's counter once they are written, and the last one
-              // publishes the expert. Four slots of 4 KB, three loads in flight; a warp pays one drain and one
+              // publishes the expert. At most eight rows: 65536 rows of 8 KB under a GEMM of 660 us then cost 110 us,
+              // with two 220, with four 115, with sixteen 115. Four slots of 4 KB, three loads in flight; a warp pays one drain and one
               // atomic per chunk, whatever the number of experts (a drain, a fence and an atomic per warp
               // and expert, with one load in flight, cost 260 us for 64 experts of 8 rows).
               const int total = p.hdr[1];
-              const int cr = min(max(total / static_cast<int>(ncw * 16u), 1), 4);
+              const int cr = min(max(total / static_cast<int>(ncw * 16u), 1), 8);
               for (int r0 = static_cast<int>(cw) * cr; r0 < total; r0 += static_cast<int>(ncw) * cr) {
                 const int first = row_base + r0, last = row_base + min(r0 + cr, total);
                 int lo = 0, hi = p.E_local;                 // expert of the first row
@@ -455,7 +476,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
                   if (n <= 0) continue;
                   q += n;
                   uint32_t* cnt = p.local_cnt + kGatherCountBase + lo;
-                  if (ptx::atom_add_acq_rel_sys(cnt, static_cast<uint32_t>(n)) + n ==
+                  if (ptx::atom_add_acq_rel_gpu(cnt, static_cast<uint32_t>(n)) + n ==
                       static_cast<uint32_t>(sp.row_end - sp.row_begin)) {
                     *cnt = 0;
                     ptx::st_release_sys(p.local_cnt + kGatherFlagBase + lo, p.epoch);
@@ -523,7 +544,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
       if (lane < p.world) flag_wait_ge(wc, p.start_ctr[p.rank] + lane, p.epoch, kSiteStartBarrier);
       __syncwarp();
     }
-    for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++it) {
+    for (int t = tile_first; t < total_tiles; t += tile_stride, ++it) {
       if (*abort_word) break;   // a wait gave up: issue nothing more
       const GroupedTile g = grouped_decode(p, t, cursor, n_tiles, BM, BN);
       const int acc = it & 1;
@@ -532,7 +553,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
       __syncwarp();
       mbar_wait(wc, tfull_bar(acc), par, kSiteTmemFull);
       ptx::tc_fence_after();
-      const int r_in_tile = q * 32 + lane;
+      const int r_in_tile = static_cast<int>(cta_rank) * 128 + q * 32 + lane;
       const bool row_ok = r_in_tile < g.rows;
       const int64_t orow = static_cast<int64_t>(g.row0) - row_base + r_in_tile;
       float scale = sscale;
@@ -558,7 +579,10 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
         if (ch == BN / 64 - 1) {
           ptx::tc_fence_before();
           __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(tempty_bar(acc));
+          if (lane == 0) {
+            if (leader) ptx::mbar_arrive(tempty_bar(acc));
+            else ptx::mbar_arrive_remote(tempty_bar(acc), 0);
+          }
         }
         const int col0 = g.n0 + ch * 64;
         if constexpr (Cfg::SCATTER) {
@@ -676,10 +700,10 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
     while (ptx::globaltimer_ns() - t0 < 200000ull) __nanosleep(2000);
   }
   ptx::tc_fence_before();
-  __syncthreads();
+  if constexpr (CG == 2) ptx::cluster_sync(); else __syncthreads();
   if (warp == 1) {
     ptx::tc_fence_after();
-    ptx::tmem_dealloc<1>(tmem_base, 512);
+    ptx::tmem_dealloc<CG>(tmem_base, 512);
   }
 
   if constexpr (Cfg::SCATTER) {

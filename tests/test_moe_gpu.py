@@ -160,3 +160,43 @@ def test_moe_index_build_stable(dev, n, E):
     assert torch.equal(offsets.long(), torch.cat([offsets.new_zeros(1).long(), splits.long().cumsum(0)]))
     assert torch.equal(scatter[order].long(), torch.arange(n, device=dev)) and torch.equal(gather.long(), order)
     assert (tki == 0).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float8_e4m3fn])
+@pytest.mark.parametrize("splits,N,K", [([1000, 0, 900, 1300], 256, 64), ([769, 768, 1, 1600], 520 + 504, 200),
+                                        ([3000, 127, 129, 256], 2056, 144)])
+def test_grouped_pairs(dev, dtype, splits, N, K):
+    """Tiles shared by two CTAs (768 rows per expert on average and more): one-row and empty experts, tiles whose second
+    half has no rows, column and K remainders; contiguous rows, gathered rows and the fused combine."""
+    import tempname_new_b200 as flux
+    K = K if dtype.itemsize == 2 else K * 2
+    E, rows = len(splits), sum(splits)
+    assert rows >= 768 * E
+    g = torch.Generator(device=dev).manual_seed(rows + N)
+    w = (torch.randn(E, N, K, device=dev, generator=g) * 0.2).to(dtype)
+    x = torch.randn(rows, K, device=dev, generator=g).to(dtype)
+    expert = torch.repeat_interleave(torch.arange(E, device=dev), torch.tensor(splits, device=dev))
+    ref = torch.cat([x[expert == e].float() @ w[e].float().t() for e in range(E)])
+    tol = 1e-2 * ref.abs().max().item()
+    out = flux.GemmGroupedV3(w, E).forward(x, torch.tensor(splits))
+    assert (out.float() - ref).abs().max().item() <= tol
+    # the same rows gathered from shuffled tokens (top-1), and back through the combine
+    perm = torch.randperm(rows, device=dev, generator=g)          # token of every sorted row
+    tokens = torch.empty_like(x.view(torch.uint8)).view(dtype)
+    tokens.view(torch.uint8)[perm] = x.view(torch.uint8)
+    scatter = torch.empty(rows, dtype=torch.int32, device=dev)
+    scatter[perm] = torch.arange(rows, dtype=torch.int32, device=dev)
+    sp = torch.tensor(splits, dtype=torch.int32, device=dev)
+    env = flux.DistEnvTPWithEP(dist.group.WORLD, 1, None, ep_size=1)
+    o16 = out.dtype
+    op = flux.GemmGroupedV3AGScatter(env, flux.MoeArguments(rows, K, N, E, 1, dtype, o16))
+    for _ in range(2):
+        got = op.forward(tokens, w, sp, scatter.view(rows, 1))
+        assert (got.float() - ref).abs().max().item() <= tol
+    op.check_status()
+    gate = torch.rand(rows, device=dev, generator=g)
+    rs = flux.GemmGroupedV3GatherRS(E, rows, N, 1, 0, 1, 1, 1, tp_group=dist.group.WORLD, dtype=o16)
+    for _ in range(2):
+        y = rs.forward_gather_rs(x, w, sp, scatter, output_vec_scale=gate)
+        assert (y[perm].float() - ref * gate[:, None]).abs().max().item() <= tol
+    rs.check_status()
