@@ -432,8 +432,8 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
               // No source ranks: the rows of all experts are one run of the sorted order, dealt out in chunks of a
               // few rows. Each chunk adds its rows to its expert's counter once they are written, and the last one
               // publishes the expert. At most eight rows: 65536 rows of 8 KB under a GEMM of 660 us then cost 110 us,
-              // with two 220, with four 115, with sixteen 115. Four slots of 4 KB, three loads in flight; a warp pays one drain and one
-              // atomic per chunk, whatever the number of experts (a drain, a fence and an atomic per warp
+              // with two 220, with four 115, with sixteen 115. Four slots of 4 KB, three loads in flight; a warp pays
+              // one drain and one atomic per chunk, whatever the number of experts (a drain, a fence and an atomic per warp
               // and expert, with one load in flight, cost 260 us for 64 experts of 8 rows).
               const int total = p.hdr[1];
               const int cr = min(max(total / static_cast<int>(ncw * 16u), 1), 8);

@@ -28,10 +28,7 @@ DENSE_TABLE: Dict[Key, Dict[str, int]] = {
     (8192, 12288, 12288): {"cta_group": 2, "tile_n": 256, "tile_m": 512, "group_m": 8},   # 1323 | 1313
     (8192, 6144, 12288): {"cta_group": 2, "tile_n": 256, "tile_m": 512, "group_m": 8},    # 1267 | 1316
     (8192, 12288, 6144): {"cta_group": 2, "tile_n": 256, "tile_m": 512, "group_m": 8},    # 1291 | 1316
-    (4096, 4096, 4096): {"cta_group": 2, "tile_n": 256, "tile_m": 512, "group_m": 8},     # 1176 | 1268
-    (4096, 12288, 4096): {"cta_group": 2, "tile_n": 256, "tile_m": 512, "group_m": 8},    # 1229 | 1295
     (16384, 3584, 8192): {"cta_group": 2, "tile_n": 256, "tile_m": 512, "group_m": 2},    # 1255 | 1272
-    (16384, 8192, 3584): {"cta_group": 2, "tile_n": 256, "tile_m": 512, "group_m": 8},    # 1279 | 1371
 }
 
 _NUM_SMS = 148
@@ -43,16 +40,22 @@ def _wave_eff(tiles: int, slots: int) -> float:
 
 
 def heuristic(m: int, n: int, k: int, elt: int = 2) -> Dict[str, int]:
-    """CTA pairs on 256 x 256 tiles unless the problem is too small to fill 74 pairs; raster groups
-    of 2048 rows (with wave-synchronous tile starts the grid walks K together, so the group does
-    not have to fit L2 over the whole K extent)."""
-    if m >= 256 and n >= 256 and (m // 256) * -(-n // 256) >= _NUM_SMS // 4:
-        cg, bn = 2, 256      # (tile_m stays 0: the launcher picks 512-row tiles when the rows allow them)
+    """CTA pairs on 256 x 256 tiles wherever they need no more waves than single CTAs on 128 x 256 (1000 x 3000 x 5000
+    fp16: 41 against 53 us; 1500 x 4000 x 4096 bf16: 52 either way); tile_m stays 0, the launcher picks 512-row tiles
+    where K is long. Raster groups of 2048 rows (with wave-synchronous tile starts the grid walks K together, so the
+    group does not have to fit L2 over the whole K extent), of 4096 rows for the 256-row tiles of a short K (4096 x
+    16384 x 4096 bf16 434 -> 416 us, 8192 x 8192 x 8192 fp8 427 -> 416, never slower by more than the noise)."""
+    up = lambda a, b: -(-a // b)  # noqa: E731
+    t1, t2 = up(m, 128) * up(n, 256), up(m, 256) * up(n, 256)
+    pairs = m >= 256 and n >= 256
+    if pairs and ((m // 256) * up(n, 256) >= _NUM_SMS // 4 or
+                  (t2 >= _NUM_SMS // 8 and up(t2, _NUM_SMS // 2) <= up(t1, _NUM_SMS))):
+        cg, bn = 2, 256
     elif n % 256 == 0 or n > 2048:
         cg, bn = 1, 256
     else:
         cg, bn = 1, 128
-    group = 8 if cg == 2 else 16
+    group = 16 if cg == 1 or k * elt < 80 * 128 else 8
     return {"cta_group": cg, "tile_n": bn, "group_m": group}
 
 

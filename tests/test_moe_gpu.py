@@ -131,7 +131,8 @@ def test_moe_layer0_gather_chunks(dev, tokens, E, topk, kind):
     chosen = chosen.to(torch.int32)
     splits, _, scatter, gather, _ = flux.moe_index_build(chosen, E)
     order = torch.argsort(chosen.reshape(-1), stable=True)
-    assert torch.equal(gather, (order // topk).int()) and torch.equal(splits, torch.bincount(chosen.reshape(-1).long(), minlength=E).int())
+    assert torch.equal(gather, (order // topk).int())
+    assert torch.equal(splits, torch.bincount(chosen.reshape(-1).long(), minlength=E).int())
     x = torch.randn(tokens, H, device=dev, generator=g).bfloat16()
     w = [(torch.randn(E, ffn, H, device=dev, generator=g) * 0.2).bfloat16() for _ in range(2)]
     env = flux.DistEnvTPWithEP(dist.group.WORLD, 1, None, ep_size=1)
