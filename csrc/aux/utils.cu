@@ -223,23 +223,25 @@ __global__ void copy_bytes_kernel(uint8_t* dst, const uint8_t* src, int64_t nbyt
 // Three passes: per-block histograms, one-block scan, stable placement.
 // ----------------------------------------------------------------------------------------
 constexpr int kIdxThreads = 256;
-constexpr int kIdxPerBlock = 4096;
+constexpr int kIdxPerBlock = 1024;         // entries per block
+constexpr int kIdxPerBlockStatic = 4096;   // in the form with the built-in scratch, whose capacity counts such blocks
 constexpr int kMaxExperts = 512;
 
+template <int PB>
 __global__ void __launch_bounds__(kIdxThreads) moe_hist_kernel(const int32_t* experts, int64_t n,
                                                                int E, int32_t* block_hist) {
   extern __shared__ int32_t hist[];
   for (int e = threadIdx.x; e < E; e += kIdxThreads) hist[e] = 0;
-  const int64_t base = static_cast<int64_t>(blockIdx.x) * kIdxPerBlock;
-  int mine[kIdxPerBlock / kIdxThreads];          // all loads in flight before the first count
+  const int64_t base = static_cast<int64_t>(blockIdx.x) * PB;
+  int mine[PB / kIdxThreads];          // all loads in flight before the first count
 #pragma unroll
-  for (int i = 0; i < kIdxPerBlock / kIdxThreads; ++i) {
+  for (int i = 0; i < PB / kIdxThreads; ++i) {
     const int64_t idx = base + i * kIdxThreads + threadIdx.x;
     mine[i] = idx < n ? experts[idx] : -1;
   }
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < kIdxPerBlock / kIdxThreads; ++i)
+  for (int i = 0; i < PB / kIdxThreads; ++i)
     if (mine[i] >= 0 && mine[i] < E) atomicAdd(&hist[mine[i]], 1);
   __syncthreads();
   for (int e = threadIdx.x; e < E; e += kIdxThreads) block_hist[blockIdx.x * E + e] = hist[e];
@@ -290,17 +292,21 @@ __global__ void __launch_bounds__(kMaxExperts) moe_scan_kernel(int32_t* block_hi
   }
 }
 
+template <int PB>
 __global__ void __launch_bounds__(kIdxThreads) moe_place_kernel(
     const int32_t* experts, int64_t n, int E, int topk, const int32_t* block_start,
     int32_t* scatter_index, int32_t* gather_index, int32_t* topk_index) {
-  // Each warp owns kPerWarp consecutive entries and counts them first; a scan over the warps then gives every
-  // warp the first free row of each expert, and the warps place their entries side by side, 32 at a time, lanes
-  // in order: equal experts keep their input order. (Serving the eight warps in turn for every 256 entries, with
-  // a block barrier each, took 76 us for 65536 entries and 15 for 512.)
-  constexpr int kWarps = kIdxThreads / 32, kPerWarp = kIdxPerBlock / kWarps, kSteps = kPerWarp / 32;
+  // Each warp owns an equal share of the block's entries, a run of them, and counts them first; a scan over the warps
+  // then gives every warp the first free row of each expert, and the warps place their entries side by side, 32 at a
+  // time, lanes in order: equal experts keep their input order. (Serving the eight warps in turn for every 256
+  // entries, with a block barrier each, took 76 us for 65536 entries and 15 for 512; runs of 512 per warp 11 and 10.)
+  constexpr int kWarps = kIdxThreads / 32, kSteps = PB / kWarps / 32;
   extern __shared__ int32_t running[];            // [kWarps][E]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t base = static_cast<int64_t>(blockIdx.x) * kIdxPerBlock + warp * kPerWarp;
+  const int64_t first_entry = static_cast<int64_t>(blockIdx.x) * PB;
+  const int count = static_cast<int>(n - first_entry < PB ? n - first_entry : PB);
+  const int steps = (count + kIdxThreads - 1) / kIdxThreads;         // of 32 entries per warp
+  const int64_t base = first_entry + warp * steps * 32;
   int32_t* mine = running + warp * E;
   int32_t start0[(kMaxExperts + kIdxThreads - 1) / kIdxThreads];
 #pragma unroll
@@ -312,7 +318,7 @@ __global__ void __launch_bounds__(kIdxThreads) moe_place_kernel(
 #pragma unroll
   for (int i = 0; i < kSteps; ++i) {
     const int64_t idx = base + i * 32 + lane;
-    const int e = idx < n ? experts[idx] : -1;
+    const int e = i < steps && idx < n ? experts[idx] : -1;
     ex[i] = e >= 0 && e < E ? e : -1;
   }
   for (int e = lane; e < E; e += 32) mine[e] = 0;
@@ -336,6 +342,7 @@ __global__ void __launch_bounds__(kIdxThreads) moe_place_kernel(
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < kSteps; ++i) {
+    if (i >= steps) break;
     const int64_t idx = base + i * 32 + lane;
     const int e = ex[i];
     const unsigned peers = __match_any_sync(0xffffffffu, e);
@@ -457,9 +464,9 @@ extern "C" int fluxb_moe_index_build(const int32_t* experts, int64_t n, int E, i
   FLUXB_REQUIRE(E >= 1 && E <= kMaxExperts && topk >= 1 && n > 0, "moe index sizes");
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const int nblocks = static_cast<int>((n + kIdxPerBlock - 1) / kIdxPerBlock);
-  moe_hist_kernel<<<nblocks, kIdxThreads, E * sizeof(int32_t), s>>>(experts, n, E, scratch);
+  moe_hist_kernel<kIdxPerBlock><<<nblocks, kIdxThreads, E * sizeof(int32_t), s>>>(experts, n, E, scratch);
   moe_scan_kernel<<<1, kMaxExperts, 0, s>>>(scratch, nblocks, E, splits, offsets);
-  moe_place_kernel<<<nblocks, kIdxThreads, kIdxThreads / 32 * E * sizeof(int32_t), s>>>(
+  moe_place_kernel<kIdxPerBlock><<<nblocks, kIdxThreads, kIdxThreads / 32 * E * sizeof(int32_t), s>>>(
       experts, n, E, topk, scratch, scatter_index, gather_index, topk_index);
   FLUXB_CUDA_OK(cudaGetLastError());
   g_launches.fetch_add(3, std::memory_order_relaxed);
@@ -481,7 +488,7 @@ extern "C" int fluxb_moe_index_build_static(const int32_t* experts, int64_t n, i
                                             int32_t* topk_index, void* stream) {
   FLUXB_REQUIRE(experts && offsets && scatter_index, "moe index arguments");
   FLUXB_REQUIRE(E >= 1 && E <= kMaxExperts && topk >= 1 && n > 0, "moe index sizes");
-  const int64_t nblocks64 = (n + kIdxPerBlock - 1) / kIdxPerBlock;
+  const int64_t nblocks64 = (n + kIdxPerBlockStatic - 1) / kIdxPerBlockStatic;
   if (nblocks64 * E > FLUXB_MOE_INDEX_STATIC_ELEMS)
     return fail(kErrInvalid,
                 "fluxb_moe_index_build_static: ceil(n/4096)*E = " + std::to_string(nblocks64 * E) +
@@ -505,9 +512,9 @@ extern "C" int fluxb_moe_index_build_static(const int32_t* experts, int64_t n, i
   }
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const int nblocks = static_cast<int>(nblocks64);
-  moe_hist_kernel<<<nblocks, kIdxThreads, E * sizeof(int32_t), s>>>(experts, n, E, scratch);
+  moe_hist_kernel<kIdxPerBlockStatic><<<nblocks, kIdxThreads, E * sizeof(int32_t), s>>>(experts, n, E, scratch);
   moe_scan_kernel<<<1, kMaxExperts, 0, s>>>(scratch, nblocks, E, splits, offsets);
-  moe_place_kernel<<<nblocks, kIdxThreads, kIdxThreads / 32 * E * sizeof(int32_t), s>>>(
+  moe_place_kernel<kIdxPerBlockStatic><<<nblocks, kIdxThreads, kIdxThreads / 32 * E * sizeof(int32_t), s>>>(
       experts, n, E, topk, scratch, scatter_index, gather_index, topk_index);
   FLUXB_CUDA_OK(cudaGetLastError());
   g_launches.fetch_add(3, std::memory_order_relaxed);

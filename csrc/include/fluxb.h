@@ -195,7 +195,8 @@ typedef struct {
    * routing_idx [world * tokens_per_rank * topk] = sorted row of every (token, k); row_entry: int32
    * scratch of at least (rows of this rank) words; sc_flags[r]: world uint32 on rank r, zero at first
    * use; start_ctr and local_cnt (1 word) as above. d is not written. */
-  int32_t scatter, reserved2;
+  int32_t scatter;
+  int32_t reuse_schedule;    /* 1: `scratch` still holds the schedule of the launch before (same call, splits and N) */
   const int32_t* routing_idx;
   int32_t* row_entry;
   void* sc_stage[FLUXB_MAX_RANKS];

@@ -375,12 +375,12 @@ extern "C" int fluxb_moe_grouped_gemm(const fluxb_moe_gemm_args_t* a) {
     moe_schedule_kernel<<<entry_blocks, kSchedThreads, 0, stream>>>(
         a->splits, nullptr, a->E, a->e0, a->E_local, a->rank, a->world, n_tiles, bm, sp, tile_begin, hdr,
         a->scatter_index, a->n_entries, nullptr, a->gather_index, a->topk);
-  } else {
+  } else if (a->gathered || a->reuse_schedule == 0) {
     moe_schedule_kernel<<<1, kSchedThreads, 0, stream>>>(a->splits, by_src ? cnt : nullptr, a->E, a->e0, a->E_local,
                                                          a->rank, a->world, n_tiles, bm, sp, tile_begin, hdr, nullptr,
                                                          0, nullptr, nullptr, 1);
   }
-  g_launches.fetch_add(1, std::memory_order_relaxed);
+  if (a->gathered || a->scatter || a->reuse_schedule == 0) g_launches.fetch_add(1, std::memory_order_relaxed);
   FLUXB_CUDA_OK(cudaGetLastError());
 
   GroupedParams p;

@@ -57,7 +57,7 @@ class MoeGemmArgs(ctypes.Structure):
         ("timeout_ns", ctypes.c_uint64), ("status", _VP),
         ("ag_src", _VP), ("ag_land", _VP * _R), ("ag_flags", _VP * _R), ("start_ctr", _VP * _R),
         ("local_cnt", _VP), ("stream", _VP),
-        ("scatter", ctypes.c_int32), ("reserved2", ctypes.c_int32),
+        ("scatter", ctypes.c_int32), ("reuse_schedule", ctypes.c_int32),
         ("routing_idx", _VP), ("row_entry", _VP),
         ("sc_stage", _VP * _R), ("sc_flags", _VP * _R), ("sc_out", _VP),
     ]
@@ -243,6 +243,8 @@ class GemmGroupedV3AGScatter(FusedOpBase):
                 a.gathered = 0
                 a.a, a.a_rows = self._sorted.data_ptr(), self._sorted.shape[0]
                 a.scatter_index = a.gather_index = a.a_sorted = None
+                # (one rank: the sub-problems and their tiles are those of the launch before)
+                a.reuse_schedule = 1 if self.world == 1 and outs and N == weights[g - 1].shape[1] else 0
                 _native.check(_native.lib().fluxb_moe_grouped_gemm(ctypes.byref(a)), "fluxb_moe_grouped_gemm")
                 outs.append(out)
                 continue
