@@ -9,6 +9,7 @@ from typing import Optional, Sequence
 import torch
 
 from .. import _native
+from ..tuning import table as _table
 
 MAX_RANKS = 8
 PLAIN, ALLGATHER, REDUCE_SCATTER = 0, 1, 2
@@ -44,24 +45,26 @@ class DenseArgs(ctypes.Structure):
     ]
 
 
+_CODES = {torch.bfloat16: BF16, torch.float8_e4m3fn: FP8_E4M3, torch.float16: FP16, torch.float32: FP32,
+          torch.float8_e5m2: FP8_E5M2, torch.int8: INT8}
+
+
 def dtype_code(dt: torch.dtype) -> int:
-    if dt == torch.bfloat16:
-        return BF16
-    if dt == torch.float8_e4m3fn:
-        return FP8_E4M3
-    if dt == torch.float16:
-        return FP16
-    if dt == torch.float32:
-        return FP32
-    if dt == torch.float8_e5m2:
-        return FP8_E5M2
-    if dt == torch.int8:
-        return INT8
-    raise TypeError(f"unsupported dtype {dt}")
+    code = _CODES.get(dt)
+    if code is None:
+        raise TypeError(f"unsupported dtype {dt}")
+    return code
+
+
+# (the stream handle without a Stream object around it: 0.2 us instead of 4)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def current_stream_ptr(device=None) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    if _raw_stream is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    index = device.index if isinstance(device, torch.device) else device
+    return _raw_stream(torch.cuda.current_device() if index is None else index)
 
 
 def fill_ptrs(arr, ptrs: Optional[Sequence[int]]) -> None:
@@ -93,7 +96,7 @@ def _as_scale(t: Optional[torch.Tensor], dev) -> Optional[torch.Tensor]:
         return None
     if t.dtype != torch.float32 or t.device != dev:
         t = t.to(device=dev, dtype=torch.float32)
-    return t.reshape(-1).contiguous()
+    return t if t.is_contiguous() else t.reshape(-1).contiguous()
 
 
 _TIMELINE: Optional[torch.Tensor] = None
@@ -163,61 +166,65 @@ def base_args(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor], ou
     rows this GPU computes; when no tile knobs are given they come from the tuning table."""
     if not (a.is_cuda and b.is_cuda):
         raise RuntimeError("the sm_100a GEMM kernels need CUDA tensors")
-    if a.dim() != 2 or b.dim() != 2 or a.shape[1] != b.shape[1]:
-        raise ValueError(f"shape mismatch: A {tuple(a.shape)} B {tuple(b.shape)} (B is [N, K])")
+    sa_shape, sb_shape = a.shape, b.shape
+    if len(sa_shape) != 2 or len(sb_shape) != 2 or sa_shape[1] != sb_shape[1]:
+        raise ValueError(f"shape mismatch: A {tuple(sa_shape)} B {tuple(sb_shape)} (B is [N, K])")
+    N, K = sb_shape
+    dtype, dev = a.dtype, a.device
+    a_str, b_str = a.stride(), b.stride()
     # B is [N, K]; a transposed view of [K, N] memory (N contiguous) is read in place by the 16-bit kernels
-    b_kn = b.stride(1) != 1 and kn_in_place(b)
-    if b.stride(1) != 1 and not b_kn:
+    b_kn = b_str[1] != 1 and kn_in_place(b)
+    if b_str[1] != 1 and not b_kn:
         b = b.contiguous()
+        b_str = b.stride()
         if keep is not None:
             keep.append(b)
-    if a.stride(1) != 1:
+    if a_str[1] != 1:
         raise ValueError("A must have a contiguous K dimension")
-    if a.dtype != b.dtype:
+    if dtype != b.dtype:
         raise TypeError("A and B must share a dtype")
     args = DenseArgs()
     if _TIMELINE is not None:
         _TIMELINE.zero_()
         args.trace = _TIMELINE.data_ptr()
     args.a, args.b = a.data_ptr(), b.data_ptr()
-    args.lda, args.ldb = a.stride(0), (b.stride(1) if b_kn else b.stride(0))
+    args.lda, args.ldb = a_str[0], (b_str[1] if b_kn else b_str[0])
     args.b_kn = 1 if b_kn else 0
     args._b_ref = b   # (a re-laid-out copy must outlive the launch)
-    args.N, args.K = b.shape[0], a.shape[1]
-    args.in_dtype = dtype_code(a.dtype)
+    args.N, args.K = N, K
+    args.in_dtype = dtype_code(dtype)
     args.out_dtype = dtype_code(out_dtype)
     if bias is not None:
-        if bias.dtype != out_dtype or bias.shape[-1] != b.shape[0] or bias.stride(-1) != 1:
+        if bias.dtype != out_dtype or bias.shape[-1] != N or bias.stride(-1) != 1:
             raise ValueError("bias must be [1|M, N] in the output dtype")
         args.bias = bias.data_ptr()
         args.bias_row_stride = 0 if (bias.dim() == 1 or bias.shape[0] == 1) else bias.stride(0)
-    # per-row scales cover the rows of the whole problem (m), per-column scales the N outputs
-    sa_vec = check_scale(scale_a, m if m is not None else a.shape[0], "input_scale")
-    sb_vec = check_scale(scale_b, b.shape[0], "weight_scale")
-    sa, sb = _as_scale(scale_a, a.device), _as_scale(scale_b, a.device)
-    if sa is not None:
-        args.scale_a = sa.data_ptr()
-    if sb is not None:
-        args.scale_b = sb.data_ptr()
-    args.scale_flags = (1 if sa_vec else 0) | (2 if sb_vec else 0)
-    if keep is not None:
-        keep.extend([sa, sb])
+    if scale_a is not None or scale_b is not None:
+        # per-row scales cover the rows of the whole problem (m), per-column scales the N outputs
+        sa_vec = check_scale(scale_a, m if m is not None else sa_shape[0], "input_scale")
+        sb_vec = check_scale(scale_b, N, "weight_scale")
+        sa, sb = _as_scale(scale_a, dev), _as_scale(scale_b, dev)
+        if sa is not None:
+            args.scale_a = sa.data_ptr()
+        if sb is not None:
+            args.scale_b = sb.data_ptr()
+        args.scale_flags = (1 if sa_vec else 0) | (2 if sb_vec else 0)
+        if keep is not None:
+            keep.extend([sa, sb])
     if tile_n == 0 and cta_group == 0 and m is not None:
-        from ..tuning.table import lookup, pinned
-        knobs = lookup(m, b.shape[0], a.shape[1], a.element_size())
+        cta_group, tile_n, g, tm, pinned = _table.resolve(m, N, K, a.element_size())
         # (a measured or pinned entry is taken as it is; a default may give way to the split-K kernel)
-        args.auto_shape = 0 if pinned(m, b.shape[0], a.shape[1]) or group_m or tile_m else 1
-        tile_n, cta_group = knobs["tile_n"], knobs["cta_group"]
+        args.auto_shape = 0 if pinned or group_m or tile_m else 1
         if group_m == 0:
-            group_m = knobs["group_m"]
+            group_m = g
         if tile_m == 0:
-            tile_m = knobs.get("tile_m", 0)
+            tile_m = tm
     args.group_m, args.num_sms, args.tile_n = group_m, num_sms, tile_n
     args.tile_m = tile_m
     args.act = ACT[act]
     args.cta_group = cta_group
     args.status = status.data_ptr() if status is not None else None
-    args.stream = current_stream_ptr(a.device)
+    args.stream = current_stream_ptr(dev)
     return args
 
 

@@ -9,6 +9,7 @@ the entry to add; ``FLUXB_TUNE_FILE`` names a JSON file of extra entries.
 """
 from __future__ import annotations
 
+import functools
 import json
 import os
 from typing import Dict, Tuple
@@ -40,11 +41,19 @@ def _wave_eff(tiles: int, slots: int) -> float:
 
 
 def heuristic(m: int, n: int, k: int, elt: int = 2) -> Dict[str, int]:
-    """CTA pairs on 256 x 256 tiles wherever they need no more waves than single CTAs on 128 x 256 (1000 x 3000 x 5000
-    fp16: 41 against 53 us; 1500 x 4000 x 4096 bf16: 52 either way); tile_m stays 0, the launcher picks 512-row tiles
-    where K is long. Raster groups of 2048 rows (with wave-synchronous tile starts the grid walks K together, so the
-    group does not have to fit L2 over the whole K extent), of 4096 rows for the 256-row tiles of a short K (4096 x
-    16384 x 4096 bf16 434 -> 416 us, 8192 x 8192 x 8192 fp8 427 -> 416, never slower by more than the noise)."""
+    """The default of a shape without a measured entry, see ``_heuristic``."""
+    cg, bn, group = _heuristic(m, n, k, elt)
+    return {"cta_group": cg, "tile_n": bn, "group_m": group}
+
+
+@functools.lru_cache(maxsize=4096)
+def _heuristic(m: int, n: int, k: int, elt: int) -> Tuple[int, int, int]:
+    """(cta_group, tile_n, group_m): CTA pairs on 256 x 256 tiles wherever they need no more waves than single CTAs on
+    128 x 256 (1000 x 3000 x 5000 fp16: 41 against 53 us; 1500 x 4000 x 4096 bf16: 52 either way); tile_m stays 0, the
+    launcher picks 512-row tiles where K is long. Raster groups of 2048 rows (with wave-synchronous tile starts the
+    grid walks K together, so the group does not have to fit L2 over the whole K extent), of 4096 rows for the 256-row
+    tiles of a short K (4096 x 16384 x 4096 bf16 434 -> 416 us, 8192 x 8192 x 8192 fp8 427 -> 416, never slower by more
+    than the noise)."""
     up = lambda a, b: -(-a // b)  # noqa: E731
     t1, t2 = up(m, 128) * up(n, 256), up(m, 256) * up(n, 256)
     pairs = m >= 256 and n >= 256
@@ -56,7 +65,7 @@ def heuristic(m: int, n: int, k: int, elt: int = 2) -> Dict[str, int]:
     else:
         cg, bn = 1, 128
     group = 16 if cg == 1 or k * elt < 80 * 128 else 8
-    return {"cta_group": cg, "tile_n": bn, "group_m": group}
+    return cg, bn, group
 
 
 def candidates(m: int, n: int, k: int, elt: int = 2, segmented_rows: int = 0):
@@ -108,21 +117,29 @@ class override:
         return False
 
 
-def lookup(m: int, n: int, k: int, elt: int = 2) -> Dict[str, int]:
+def _entry(key: Key):
     global _EXTRA
     if _EXTRA is None:
         _EXTRA = _load_extra()
-    key = (m, n, k)
-    if key in _OVERRIDE:
-        return dict(_OVERRIDE[key])
-    if key in _EXTRA:
-        return dict(_EXTRA[key])
-    if key in DENSE_TABLE:
-        return dict(DENSE_TABLE[key])
-    return heuristic(m, n, k, elt)
+    for table in (_OVERRIDE, _EXTRA, DENSE_TABLE):
+        if key in table:
+            return table[key]
+    return None
+
+
+def lookup(m: int, n: int, k: int, elt: int = 2) -> Dict[str, int]:
+    e = _entry((m, n, k))
+    return dict(e) if e is not None else heuristic(m, n, k, elt)
 
 
 def pinned(m: int, n: int, k: int) -> bool:
     """True when ``lookup`` answers from a measured or pinned entry rather than from the heuristic."""
-    key = (m, n, k)
-    return key in _OVERRIDE or key in DENSE_TABLE or (_EXTRA is not None and key in _EXTRA)
+    return _entry((m, n, k)) is not None
+
+
+def resolve(m: int, n: int, k: int, elt: int = 2) -> Tuple[int, int, int, int, bool]:
+    """``lookup`` and ``pinned`` for a launch: (cta_group, tile_n, group_m, tile_m, pinned)."""
+    e = _entry((m, n, k))
+    if e is not None:
+        return e["cta_group"], e["tile_n"], e["group_m"], e.get("tile_m", 0), True
+    return (*_heuristic(m, n, k, elt), 0, False)
