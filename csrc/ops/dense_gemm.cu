@@ -550,8 +550,12 @@ static int dense_impl(const fluxb_dense_args_t* a, const fluxb_a2a_args_t* x) {
       const char* e = getenv("FLUXB_TAIL_SPLIT");
       return e ? atoi(e) : 1;
     }();
-    if (bn == 256 && !a->blockscale && !a->b_kn)
-      if ((rc = fluxb_tail_split(tiles, grid / cg, split_env, &p.split_from, &p.split_shift))) return rc;
+    // (block-scaled: halves, in the plain GEMM with one weight scale per block. 8192 x 3584 has 896 tiles, eight more
+    // than six waves: with 8192 x 8192 x 3584, which has no such rest, 504 -> 436 us for the two)
+    const bool bs_plain = a->blockscale == 1 && cg == 1 && p.mode == kModePlain;
+    if (bn == 256 && (!a->blockscale || bs_plain) && !a->b_kn)
+      if ((rc = fluxb_tail_split(tiles, grid / cg, bs_plain && split_env > 0 ? 2 : split_env, &p.split_from, &p.split_shift)))
+        return rc;
   }
   p.total_vtiles = p.split_from + static_cast<int32_t>((tiles - p.split_from) << p.split_shift);
   if (!multi && !a2a && static_cast<int64_t>(p.total_vtiles) * cg < grid) grid = p.total_vtiles * cg;

@@ -217,7 +217,7 @@ struct DenseCfg {
   static constexpr int TMEM_COLS = 512;
   static_assert(ACC_BUFS * BN <= TMEM_COLS, "accumulators must fit TMEM");
   // column pieces of a split tile are BN >> shift wide; the epilogue moves 64 columns at a time
-  static constexpr int MAX_SPLIT_SHIFT = (BN_ == 256 && !BS) ? 2 : 0;
+  static constexpr int MAX_SPLIT_SHIFT = BN_ != 256 ? 0 : (!BS ? 2 : (BS_ == kBsSquare ? 1 : 0));
 };
 
 struct TileCoord {
@@ -1320,14 +1320,15 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
       // scales and added to fp32 registers. Warp (quadrant q, half) owns rows q*32.. and the 128 columns of one
       // scale block of the weight for the whole tile. 128 accumulators and 32 staging registers leave about 40
       // for everything else, so nothing that can be computed again is kept across the loop.
-      // Measured at 8192 x 3584 x 8192: square 252 us (303 while one lane walked the issue loops, 320 with the
-      // general loop below: two polls of the full barrier and spills); per column 360 us (379; 1340 before,
-      // when every warp read the column scales from global memory where it multiplied by them). Sixteen warps
-      // of 64 columns, with the one-lane loops: 358 and 667 us. Register splits 24 / 240 and 56 / 224: within 2 % of 40 / 232.
+      // Measured at 8192 x 3584 x 8192: square 218 us (252 with the last wave's tiles whole, 303 while one lane walked
+      // the issue loops, 320 with the general loop below: two polls of the full barrier and spills); per column 360 us
+      // (379 with the one-lane loops; 1340 when every warp read the column scales from global memory where it
+      // multiplied by them). Sixteen warps of 64 columns, with the one-lane loops: 358 and 667 us. Register splits
+      // 24 / 240 and 56 / 224: within 2 % of 40 / 232.
       constexpr bool kColumn = Cfg::BS_FORM == kBsColumn;
       const int half = ew >> 2;
       const int kbs = k_blocks;
-      const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + half * 128;
+      const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
       uint32_t n = 0;                                  // k-blocks promoted so far: TMEM buffer n & 1
 #ifdef FLUXB_DEBUG_CHECKS
       uint64_t probe_wait = 0, probe_ld = 0;           // phase clocks of the self-checking build, as below
@@ -1341,10 +1342,16 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
           const int row = c.m_in_seg + q * 32 + lane;
           const int row_s = row < ((p.seg_rows + 127) & ~127) ? row : 0;
           so = static_cast<uint32_t>(row_s >> 7) * static_cast<uint32_t>(kbs) * 128u + (row_s & 127);
-          int nblk = (c.n0 >> 7) + half;
+          int nblk = (c.n0 >> 7) + (kColumn || c.shift == 0 ? half : 0);
           if (nblk >= (p.N >> 7)) nblk = (p.N >> 7) - 1;   // (the clipped half of the last tile)
           bo = static_cast<uint32_t>(nblk) * static_cast<uint32_t>(kbs) * (kColumn ? 128u : 1u) + (kColumn ? 4u * lane : 0u);
         }
+        // a warp owns 128 columns of a whole tile, 64 of one cut in two (both warps of a quadrant then share the scale
+        // block of the 128 columns)
+        // (the per-column form is left whole: it has no register for the choice, 363 -> 398 us)
+        const bool whole = kColumn || t < p.split_from || p.split_shift == 0;
+        const uint32_t tbase = lane_base + static_cast<uint32_t>(half) * (whole ? 128u : 64u);
+        const uint32_t col_off = whole ? 0u : static_cast<uint32_t>(half) * 256u;
         uint64_t acc[64];
 #pragma unroll
         for (int j = 0; j < 64; ++j) acc[j] = 0ull;
@@ -1393,9 +1400,10 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
           uint32_t r[32];
 #pragma unroll
           for (int c4 = 0; c4 < 4; ++c4) {
-            ptx::tmem_ld_32x32b_x32(lane_base + buf * 256u + 32 * c4, r);
+            if (c4 >= 2 && !whole) break;
+            ptx::tmem_ld_32x32b_x32(tbase + buf * 256u + 32 * c4, r);
             ptx::tmem_ld_wait();
-            if (c4 == 3) {
+            if (c4 == 3 || (c4 == 1 && !whole)) {
 #ifdef FLUXB_DEBUG_CHECKS
               probe_ld += static_cast<uint64_t>(clock64() - pc1);
 #endif
@@ -1407,7 +1415,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
             if constexpr (kColumn) {
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
-                const ulonglong2 sv = ptx::ld_shared_v2_b64(slot + 128u * c4 + 16u * j);
+                const ulonglong2 sv = ptx::ld_shared_v2_b64(slot + col_off + 128u * c4 + 16u * j);
                 uint64_t& a0 = acc[16 * c4 + 2 * j];
                 uint64_t& a1 = acc[16 * c4 + 2 * j + 1];
                 a0 = ptx::ffma2(ptx::pack_b32x2(r[4 * j], r[4 * j + 1]), ptx::fmul2(sc2, sv.x), a0);
@@ -1426,6 +1434,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
         const int row = c.m_in_seg + q * 32 + lane;
 #pragma unroll
         for (int ch = 0; ch < 2; ++ch) {
+          if (!kColumn && ch == 1 && c.shift != 0) break;
           uint32_t r0[32], r1[32];
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
@@ -1434,7 +1443,8 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
             r1[2 * j] = static_cast<uint32_t>(acc[ch * 32 + 16 + j]);
             r1[2 * j + 1] = static_cast<uint32_t>(acc[ch * 32 + 16 + j] >> 32);
           }
-          emit_chunk(r0, r1, c.n0 + half * 128 + ch * 64, row, row, c.m_in_seg + q * 32, &p.tm_d[0], 0, false);
+          const int col0 = c.n0 + half * (kColumn || c.shift == 0 ? 128 : 64) + ch * 64;
+          emit_chunk(r0, r1, col0, row, row, c.m_in_seg + q * 32, &p.tm_d[0], 0, false);
         }
       }
       if (lane == 0) ptx::bulk_wait<0>();

@@ -139,3 +139,30 @@ def test_split_k_block_scaled(dev, M, N, K):
     _dense.run(args)
     e_new, e_old = ((t.double() - ref).norm().item() for t in (new, old))
     assert not new.isnan().any() and e_new <= 1.02 * e_old and e_new <= 2e-3 * ref.norm().item()
+
+
+@pytest.mark.parametrize("M,N,K", [(200, 2176, 384), (128, 256, 128), (2432, 2304, 640), (1184, 4224, 256), (2500, 1920, 512)])
+@pytest.mark.parametrize("groupwise", [False, True])
+def test_cut_tiles_of_the_last_wave(dev, M, N, K, groupwise):
+    """128 x 256 tiles whose last wave is cut into 128-column halves (all tiles, some, none; a half past the last column),
+    with one weight scale per block and per column: against 64 bits, and bit for bit against whole 128 x 128 tiles,
+    which multiply and add in the same order."""
+    from tempname_new_b200.ops import _dense
+    from tempname_new_b200.ops.blockscale_gemm import blockscale_args
+    g = torch.Generator(device=dev).manual_seed(M + N + K)
+    a, b = (torch.randn(s, device=dev, generator=g).to(torch.float8_e4m3fn) for s in ((M, K), (N, K)))
+    sa = torch.rand((M + 127) // 128, K // 128, 128, device=dev, generator=g) + 0.5
+    sb = torch.rand(*((N // 128, K // 128) + ((128,) if groupwise else ())), device=dev, generator=g) + 0.5
+    ad = a.double().view(M, K // 128, 128) * sa.double().permute(0, 2, 1).reshape(-1, K // 128)[:M, :, None]
+    sbd = sb.double().permute(0, 2, 1).reshape(N, K // 128) if groupwise else sb.double().repeat_interleave(128, 0)
+    ref = ad.reshape(M, K) @ (b.double().view(N, K // 128, 128) * sbd[:, :, None]).reshape(N, K).t()
+    outs = []
+    for tile_n in (256, 128):
+        out = torch.full((M, N), float("nan"), device=dev, dtype=torch.bfloat16)
+        args = blockscale_args(a, b, sa, sb, None, torch.bfloat16, M)
+        args.auto_shape, args.tile_n, args.M, args.d, args.ldd = 0, tile_n, M, out.data_ptr(), N
+        args.mode, args.rank, args.world, args.epoch = _dense.PLAIN, 0, 1, 1
+        _dense.run(args)
+        assert (out.double() - ref).norm().item() <= 2e-3 * ref.norm().item()
+        outs.append(out)
+    assert torch.equal(*outs)
