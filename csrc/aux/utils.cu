@@ -361,6 +361,84 @@ __global__ void __launch_bounds__(kIdxThreads) moe_place_kernel(
   }
 }
 
+// The whole build in one block for up to kIdxSmall entries (a generation batch): counts per warp, prefix sums over
+// warps and experts, placement as above. For 512 entries 3.7 us, where the three launches took 6.8 and the gaps between
+// them (whole layer of 64 tokens 508 -> 499).
+constexpr int kIdxSmall = 4096;
+constexpr int kIdxSmallThreads = 512;
+static_assert(kMaxExperts <= kIdxSmallThreads, "one thread per expert");
+
+__global__ void __launch_bounds__(kIdxSmallThreads) moe_index_small_kernel(
+    const int32_t* experts, int n, int E, int topk, int32_t* splits, int32_t* offsets, int32_t* scatter_index,
+    int32_t* gather_index, int32_t* topk_index) {
+  constexpr int kWarps = kIdxSmallThreads / 32, kSteps = kIdxSmall / kIdxSmallThreads;
+  extern __shared__ int32_t running[];            // [kWarps][E]
+  __shared__ int32_t warp_sum[kWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int steps = (n + kIdxSmallThreads - 1) / kIdxSmallThreads;
+  const int base = warp * steps * 32;
+  int32_t* mine = running + warp * E;
+  int ex[kSteps];
+#pragma unroll
+  for (int i = 0; i < kSteps; ++i) {
+    const int idx = base + i * 32 + lane;
+    const int e = i < steps && idx < n ? experts[idx] : -1;
+    ex[i] = e >= 0 && e < E ? e : -1;
+  }
+  for (int e = lane; e < E; e += 32) mine[e] = 0;
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < kSteps; ++i)
+    if (ex[i] >= 0) atomicAdd(&mine[ex[i]], 1);
+  __syncthreads();
+  const int e = threadIdx.x;
+  int32_t total = 0;
+  if (e < E) {
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) total += running[w * E + e];
+  }
+  int32_t incl = total;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) warp_sum[warp] = incl;
+  __syncthreads();
+  if (e < E) {
+    int32_t run = incl - total;
+    for (int w = 0; w < warp; ++w) run += warp_sum[w];
+    offsets[e] = run;
+    if (e == E - 1) offsets[E] = run + total;
+    if (splits) splits[e] = total;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const int32_t c = running[w * E + e];
+      running[w * E + e] = run;
+      run += c;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kSteps; ++i) {
+    if (i >= steps) break;
+    const int idx = base + i * 32 + lane;
+    const int ee = ex[i];
+    const unsigned peers = __match_any_sync(0xffffffffu, ee);
+    const int before = __popc(peers & ((1u << lane) - 1u));
+    int32_t first = 0;
+    if (ee >= 0) first = mine[ee];
+    __syncwarp();
+    if (ee >= 0 && before == 0) mine[ee] = first + __popc(peers);
+    __syncwarp();
+    if (ee >= 0) {
+      const int32_t row = first + before;
+      scatter_index[idx] = row;
+      if (gather_index) gather_index[row] = idx / topk;
+      if (topk_index) topk_index[row] = idx % topk;
+    }
+  }
+}
+
 }  // namespace
 }  // namespace fluxb
 
@@ -463,6 +541,13 @@ extern "C" int fluxb_moe_index_build(const int32_t* experts, int64_t n, int E, i
   FLUXB_REQUIRE(experts && offsets && scatter_index && scratch, "moe index arguments");
   FLUXB_REQUIRE(E >= 1 && E <= kMaxExperts && topk >= 1 && n > 0, "moe index sizes");
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (n <= kIdxSmall) {
+    moe_index_small_kernel<<<1, kIdxSmallThreads, kIdxSmallThreads / 32 * E * sizeof(int32_t), s>>>(
+        experts, static_cast<int>(n), E, topk, splits, offsets, scatter_index, gather_index, topk_index);
+    FLUXB_CUDA_OK(cudaGetLastError());
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    return kOk;
+  }
   const int nblocks = static_cast<int>((n + kIdxPerBlock - 1) / kIdxPerBlock);
   moe_hist_kernel<kIdxPerBlock><<<nblocks, kIdxThreads, E * sizeof(int32_t), s>>>(experts, n, E, scratch);
   moe_scan_kernel<<<1, kMaxExperts, 0, s>>>(scratch, nblocks, E, splits, offsets);

@@ -150,7 +150,8 @@ def test_moe_layer0_gather_chunks(dev, tokens, E, topk, kind):
     op.check_status()
 
 
-@pytest.mark.parametrize("n,E", [(1, 1), (31, 512), (4096, 3), (4097, 64), (20000, 512), (70001, 7)])
+@pytest.mark.parametrize("n,E", [(1, 1), (31, 512), (511, 64), (513, 8), (4095, 512), (4096, 3), (4097, 64), (20000, 512),
+                                 (70001, 7)])
 def test_moe_index_build_stable(dev, n, E):
     """The counting sort is stable across lanes, warps and blocks."""
     import tempname_new_b200 as flux
