@@ -1320,8 +1320,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
       // scales and added to fp32 registers. Warp (quadrant q, half) owns rows q*32.. and the 128 columns of one
       // scale block of the weight for the whole tile. 128 accumulators and 32 staging registers leave about 40
       // for everything else, so nothing that can be computed again is kept across the loop.
-      // Measured at 8192 x 3584 x 8192: square 218 us (252 with the last wave's tiles whole, 303 while one lane walked
-      // the issue loops, 320 with the general loop below: two polls of the full barrier and spills); per column 360 us
+      // Measured, mean of 8192 x 3584 x 8192 and 8192 x 8192 x 3584: square 218 us (252 with the last wave's tiles
+      // whole, 300 while one lane walked the issue loops; 320 at the first shape with the general loop below: two polls
+      // of the full barrier and spills); per column, 3584 x 8192 x 8192, 360 us
       // (379 with the one-lane loops; 1340 when every warp read the column scales from global memory where it
       // multiplied by them). Sixteen warps of 64 columns, with the one-lane loops: 358 and 667 us. Register splits
       // 24 / 240 and 56 / 224: within 2 % of 40 / 232.
