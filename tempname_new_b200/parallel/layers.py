@@ -153,9 +153,10 @@ class RowParallelLinear(nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         b = self.bias
         if (b is not None and x.is_cuda and self._cache.world == 1 and b.dtype == x.dtype
-                and b.device == x.device and b.is_contiguous()):
+                and b.device == x.device and b.is_contiguous()
+                and (x.requires_grad or self.weight.requires_grad or not b.requires_grad)):
             # one rank: the GEMM's epilogue adds the bias to the fp32 sum (a broadcast add over 8192 x 12288 bf16
-            # is 235 us next to a GEMM of 970)
+            # is 235 us next to a GEMM of 970); a bias that trains alone keeps its add, whose backward is one sum
             return _RowParallelFn.apply(x, self.weight, self._cache, b)
         y = _RowParallelFn.apply(x, self.weight, self._cache)
         return y + b if b is not None else y

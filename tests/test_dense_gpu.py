@@ -411,6 +411,10 @@ def test_row_parallel_bias_one_rank(dev):
         assert (got.float() - want).abs().max().item() <= _tol(want)
     lin.bias.requires_grad_(False)
     assert torch.equal(lin(x), y)
+    lin.bias.requires_grad_(True)
+    lin.weight.requires_grad_(False)
+    (only,) = torch.autograd.grad(lin(x.detach()), [lin.bias], gy)
+    assert torch.equal(only, gy.sum(0))
     with torch.no_grad():
         wide = RowParallelLinear(256, 520, device=dev)
         wide.bias = torch.nn.Parameter(torch.zeros(520, device=dev))     # an fp32 bias still promotes the sum
