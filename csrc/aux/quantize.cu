@@ -73,6 +73,23 @@ __device__ __forceinline__ uint32_t cvt_fp8x2(float lo, float hi, bool e5m2) {
       __nv_cvt_float2_to_fp8x2(make_float2(lo, hi), __NV_SATFINITE, e5m2 ? __NV_E5M2 : __NV_E4M3));
 }
 
+// Maxima of eight rows over the 16 lanes that share them: each step of the exchange halves the rows a lane still
+// holds, so that lane l ends with row (l >> 1) & 7 (eight shuffles instead of 32), and a row's scale is divided out by
+// two lanes instead of sixteen. 8192 x 8192 bf16, 1x128: 43.8 -> 33.6 us (6.0 TB/s), with the transpose 58.5 -> 48.1.
+template <class Max>
+__device__ __forceinline__ uint32_t max_rows8(uint32_t (&m)[8], int lane, Max&& vmax) {
+#pragma unroll
+  for (int half = 4; half > 0; half >>= 1) {
+    const bool up = (lane & (2 * half)) != 0;
+#pragma unroll
+    for (int j = 0; j < half; ++j) {
+      const uint32_t send = up ? m[j] : m[j + half], keep = up ? m[j + half] : m[j];
+      m[j] = vmax(keep, __shfl_xor_sync(0xffffffffu, send, 2 * half));
+    }
+  }
+  return vmax(m[0], __shfl_xor_sync(0xffffffffu, m[0], 1));
+}
+
 template <bool BF16, bool SQUARE>
 __global__ void __launch_bounds__(kThreads) quant_tile_kernel(
     const uint16_t* __restrict__ x, int64_t ldx, uint8_t* __restrict__ q, uint8_t* __restrict__ qt,
@@ -105,7 +122,7 @@ __global__ void __launch_bounds__(kThreads) quant_tile_kernel(
       v[it][r] = *reinterpret_cast<const uint4*>(x + static_cast<int64_t>(row0 + 4 * g + r) * ldx + col0 + chunk * 8);
   }
   // ---- maxima: per row (over the 16 lanes that share it) and per column pair (over this thread's rows)
-  float row_amax[2][4];
+  uint32_t rm[8];                               // row 4 * it + r of this thread
   uint32_t cm[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
   for (int it = 0; it < 2; ++it)
@@ -117,10 +134,7 @@ __global__ void __launch_bounds__(kThreads) quant_tile_kernel(
       cm[1] = hmax2_bits<BF16>(cm[1], a1);
       cm[2] = hmax2_bits<BF16>(cm[2], a2);
       cm[3] = hmax2_bits<BF16>(cm[3], a3);
-      uint32_t m = hmax2_bits<BF16>(hmax2_bits<BF16>(a0, a1), hmax2_bits<BF16>(a2, a3));
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) m = hmax2_bits<BF16>(m, __shfl_xor_sync(0xffffffffu, m, o));
-      row_amax[it][r] = fmaxf(h_lo<BF16>(m), h_hi<BF16>(m));
+      rm[4 * it + r] = hmax2_bits<BF16>(hmax2_bits<BF16>(a0, a1), hmax2_bits<BF16>(a2, a3));
     }
   if (qt != nullptr || SQUARE) {
 #pragma unroll
@@ -150,6 +164,15 @@ __global__ void __launch_bounds__(kThreads) quant_tile_kernel(
       if (sinv_t) sinv_t[kb * MB + mb] = 1.f / tile_scale;
     }
   }
+  float row_scale = 1.f;                        // of row (lane >> 1) & 7
+  if constexpr (!SQUARE) {
+    const uint32_t m = max_rows8(rm, lane, [](uint32_t a, uint32_t b) { return hmax2_bits<BF16>(a, b); });
+    row_scale = compute_scale(fmaxf(h_lo<BF16>(m), h_hi<BF16>(m)), eps, fp8_max);
+    const int k = (lane >> 1) & 7;
+    if ((lane & 1) == 0)
+      sinv[(static_cast<int64_t>(mb) * KB + kb) * kTile + 4 * ((k >> 2) * 16 + warp * 2 + (lane >> 4)) + (k & 3)] =
+          1.f / row_scale;
+  }
   // ---- q: one scale per row (or the tile's), 8 bytes per thread and row
 #pragma unroll
   for (int it = 0; it < 2; ++it) {
@@ -157,10 +180,7 @@ __global__ void __launch_bounds__(kThreads) quant_tile_kernel(
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       float scale = tile_scale;
-      if constexpr (!SQUARE) {
-        scale = compute_scale(row_amax[it][r], eps, fp8_max);
-        if (chunk == 0) sinv[(static_cast<int64_t>(mb) * KB + kb) * kTile + 4 * g + r] = 1.f / scale;
-      }
+      if constexpr (!SQUARE) scale = __shfl_sync(0xffffffffu, row_scale, (lane & 16) | ((4 * it + r) << 1));
       const uint32_t w[4] = {v[it][r].x, v[it][r].y, v[it][r].z, v[it][r].w};
       uint2 o;
       o.x = cvt_fp8x2(h_lo<BF16>(w[0]) * scale, h_hi<BF16>(w[0]) * scale, e5) |
@@ -231,9 +251,10 @@ __global__ void __launch_bounds__(kThreads) quant_tile_kernel(
 // start may be on any byte (q with K % 8 != 0, q^T with M % 16 != 0) are written from the shared tile one warp
 // per row, in aligned 32-bit words put together from two neighbouring words of the tile: 128 contiguous bytes
 // per instruction whatever the alignment, and single bytes at the two ends only.
-// Bound by instruction issue, not by memory: 5000 x 8192 bf16, 1x128 with the transpose, takes 44 us (3.7 TB/s);
-// 70 us with one thread per column for the column maxima and byte stores of q^T, 73 us with fp32 maxima and
-// every row of q^T through the word writer (2.7 instructions per cycle and SM either way).
+// Bound by instruction issue, not by memory: 5000 x 8192 bf16, 1x128 with the transpose, takes 37 us (4.4 TB/s); 44 us
+// with a butterfly and sixteen divisions per row, 70 us with one thread per column for the column maxima and byte
+// stores of q^T, 73 us with fp32 maxima and every row of q^T through the word writer (2.7 instructions per cycle and SM
+// in all of these).
 // ---------------------------------------------------------------------------------------------
 template <typename T>
 struct Chunk8 {      // 8 consecutive elements of a row, as they are in memory
@@ -357,7 +378,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) quant_ragged
   // ---- maxima
   using C = Chunk8<T>;
   constexpr int NW = C::NW;
-  float row_amax[2][4];
+  uint32_t rm[8];                               // row 4 * it + r of this thread
   uint32_t cm[NW];
 #pragma unroll
   for (int j = 0; j < NW; ++j) cm[j] = 0u;
@@ -372,19 +393,13 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) quant_ragged
         m = C::vmax(m, w);
         cm[j] = C::vmax(cm[j], w);
       }
-      if constexpr (!SQUARE) {
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) m = C::vmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-      }
-      row_amax[it][r] = C::row(m);
+      rm[4 * it + r] = m;
     }
   float tile_scale = 1.f;
   if constexpr (SQUARE) {
     float m = 0.f;
 #pragma unroll
-    for (int it = 0; it < 2; ++it)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) m = fmaxf(m, row_amax[it][r]);
+    for (int k = 0; k < 8; ++k) m = fmaxf(m, C::row(rm[k]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     if (lane == 0) red[warp] = m;
@@ -406,6 +421,15 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) quant_ragged
         *reinterpret_cast<uint4*>(&colred[warp][chunk * NW + j]) = make_uint4(cm[j], cm[j + 1], cm[j + 2], cm[j + 3]);
     }
   }
+  float row_scale = 1.f;                        // of row (lane >> 1) & 7
+  if constexpr (!SQUARE) {
+    const uint32_t m = max_rows8(rm, lane, [](uint32_t a, uint32_t b) { return C::vmax(a, b); });
+    row_scale = compute_scale(C::row(m), eps, fp8_max);
+    const int k = (lane >> 1) & 7;
+    if ((lane & 1) == 0)
+      sinv[(static_cast<int64_t>(mb) * KB + kb) * kTile + 4 * ((k >> 2) * 16 + warp * 2 + (lane >> 4)) + (k & 3)] =
+          1.f / row_scale;
+  }
   // ---- q
 #pragma unroll
   for (int it = 0; it < 2; ++it) {
@@ -413,10 +437,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) quant_ragged
     for (int r = 0; r < 4; ++r) {
       const int row = 4 * (it * 16 + warp * 2 + (lane >> 4)) + r;
       float scale = tile_scale;
-      if constexpr (!SQUARE) {
-        scale = compute_scale(row_amax[it][r], eps, fp8_max);
-        if (chunk == 0) sinv[(static_cast<int64_t>(mb) * KB + kb) * kTile + row] = 1.f / scale;
-      }
+      if constexpr (!SQUARE) scale = __shfl_sync(0xffffffffu, row_scale, (lane & 16) | ((4 * it + r) << 1));
       const C& c = v[it][r];
       uint2 o;
       o.x = cvt_fp8x2(c.get(0) * scale, c.get(1) * scale, e5) | (cvt_fp8x2(c.get(2) * scale, c.get(3) * scale, e5) << 16);
