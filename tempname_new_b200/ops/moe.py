@@ -235,7 +235,8 @@ class GemmGroupedV3AGScatter(FusedOpBase):
             a.stream = _dense.current_stream_ptr(dev)
             # expert-sorted copy of this rank's rows, filled by the kernel's communication warps
             rows_cap = out.shape[0]
-            if self._sorted is None or self._sorted.shape[0] < rows_cap or self._sorted.shape[1] != H:
+            if (self._sorted is None or self._sorted.shape[0] < rows_cap or self._sorted.shape[1] != H
+                    or self._sorted.dtype != x.dtype or self._sorted.device != dev):
                 self._sorted = torch.empty((max(rows_cap, 128), H), dtype=x.dtype, device=dev)
             a.a_sorted, a.a_sorted_rows = self._sorted.data_ptr(), self._sorted.shape[0]
             a.local_cnt = self.ctrl.ptr(self.rank, OFF_LOCAL)

@@ -1,0 +1,75 @@
+"""What the MoE layer-0 op hands to its kernel, checked on the CPU: tensors that claim to live on a GPU take the op's
+CUDA branch, and a recorder stands in for the launch."""
+import ctypes
+
+import pytest
+import torch
+import torch.distributed as dist
+
+from conftest import free_port
+from moe_common import routed_problem
+
+
+class _AsCuda(torch.Tensor):
+    """A CPU tensor that takes the CUDA branch of the ops."""
+    is_cuda = True
+
+
+def _as_cuda(t):
+    return torch.Tensor._make_subclass(_AsCuda, t)
+
+
+class _Recorder:
+    """The native library, except that a grouped GEMM only leaves a copy of its arguments."""
+
+    def __init__(self, lib):
+        self._lib, self.calls = lib, []
+
+    def __getattr__(self, name):
+        return getattr(self._lib, name)
+
+    def fluxb_moe_grouped_gemm(self, ref):
+        kept = type(ref._obj)()
+        ctypes.memmove(ctypes.byref(kept), ref, ctypes.sizeof(kept))
+        self.calls.append(kept)
+        return 0
+
+
+@pytest.fixture
+def layer0(monkeypatch):
+    """(tokens, hidden, ffn, experts, topk, dtype) -> (op, recorder, routing of the tokens)."""
+    import tempname_new_b200 as flux
+    from tempname_new_b200 import _native
+    from tempname_new_b200.ops import _dense
+    monkeypatch.delenv("FLUXB_MOE_GATHER", raising=False)
+    created = not dist.is_initialized()
+    if created:
+        dist.init_process_group("gloo", init_method=f"tcp://127.0.0.1:{free_port()}", rank=0, world_size=1)
+    rec = _Recorder(_native.lib())
+    monkeypatch.setattr(_native, "lib", lambda: rec)
+    monkeypatch.setattr(_dense, "current_stream_ptr", lambda device=None: 0)
+
+    def make(tokens, H, ffn, E, topk, dtype):
+        env = flux.DistEnvTPWithEP(dist.group.WORLD, 1, None, ep_size=1)
+        op = flux.GemmGroupedV3AGScatter(env, flux.MoeArguments(tokens, H, ffn, E, topk, dtype, torch.bfloat16))
+        op.status = torch.zeros(4, dtype=torch.int32)
+        _, _, scatter, splits, _ = routed_problem(tokens, topk, E)
+        return op, rec, splits, scatter
+
+    yield make
+    if created:
+        dist.destroy_process_group()
+
+
+def test_sorted_rows_buffer_follows_the_element_type(layer0):
+    """The gather writes rows of the call's element type into the sorted buffer: one kept from a call with 1-byte rows
+    is half the size that a call with 2-byte rows of the same count writes."""
+    tokens, H, ffn, E, topk = 256, 64, 128, 4, 2
+    op, rec, splits, scatter = layer0(tokens, H, ffn, E, topk, torch.bfloat16)
+    for dtype in (torch.float8_e4m3fn, torch.bfloat16, torch.float8_e4m3fn):
+        x = _as_cuda(torch.zeros(tokens, H).to(dtype))
+        op.forward(x, torch.zeros(E, ffn, H).to(dtype), splits, scatter)
+        a = rec.calls[-1]
+        assert a.a_sorted == op._sorted.data_ptr() and a.a_sorted_rows >= tokens * topk
+        assert op._sorted.numel() * op._sorted.element_size() >= a.a_sorted_rows * H * dtype.itemsize
+        assert op._sorted.dtype == dtype
