@@ -203,7 +203,14 @@ class GemmGroupedV3AGScatter(FusedOpBase):
         if outputs_buf is None:
             # sizing the result needs this rank's row count on the host: one small D2H sync that
             # callers avoid by passing outputs_buf
-            rows_ep = int(splits[self.e0:self.e0 + self.E_local].sum().item())
+            rows_cap = rows_ep = int(splits[self.e0:self.e0 + self.E_local].sum().item())
+        else:
+            rows_cap = max((o.shape[0] for o in outputs_buf[:len(weights)]), default=0)
+        # expert-sorted copy of this rank's rows, filled by the communication warps of the first group's kernel and read
+        # by the groups after it: one buffer for the whole call, with room for the rows of the longest output
+        if (self._sorted is None or self._sorted.shape[0] < rows_cap or self._sorted.shape[1] != H
+                or self._sorted.dtype != x.dtype or self._sorted.device != dev):
+            self._sorted = torch.empty((max(rows_cap, 128), H), dtype=x.dtype, device=dev)
         outs = []
         keep = []
         for g, w in enumerate(weights):
@@ -233,11 +240,6 @@ class GemmGroupedV3AGScatter(FusedOpBase):
             a.rank, a.world = self.rank, self.world
             a.timeout_ns, a.status = int(self.timeout_s * 1e9), self.status.data_ptr()
             a.stream = _dense.current_stream_ptr(dev)
-            # expert-sorted copy of this rank's rows, filled by the kernel's communication warps
-            rows_cap = out.shape[0]
-            if (self._sorted is None or self._sorted.shape[0] < rows_cap or self._sorted.shape[1] != H
-                    or self._sorted.dtype != x.dtype or self._sorted.device != dev):
-                self._sorted = torch.empty((max(rows_cap, 128), H), dtype=x.dtype, device=dev)
             a.a_sorted, a.a_sorted_rows = self._sorted.data_ptr(), self._sorted.shape[0]
             a.local_cnt = self.ctrl.ptr(self.rank, OFF_LOCAL)
             if reuse_sorted:

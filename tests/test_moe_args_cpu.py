@@ -73,3 +73,16 @@ def test_sorted_rows_buffer_follows_the_element_type(layer0):
         assert a.a_sorted == op._sorted.data_ptr() and a.a_sorted_rows >= tokens * topk
         assert op._sorted.numel() * op._sorted.element_size() >= a.a_sorted_rows * H * dtype.itemsize
         assert op._sorted.dtype == dtype
+
+
+def test_weight_groups_share_one_sorted_rows_buffer(layer0):
+    """Groups after the first read the rows that the first one gathered, also when their output buffer is longer."""
+    tokens, H, ffn, E, topk = 256, 64, 128, 4, 2
+    op, rec, splits, scatter = layer0(tokens, H, ffn, E, topk, torch.bfloat16)
+    x = _as_cuda(torch.zeros(tokens, H).bfloat16())
+    w = torch.zeros(E, ffn, H).bfloat16()
+    bufs = [torch.empty(n, ffn).bfloat16() for n in (tokens * topk, tokens * topk + 300, tokens * topk)]
+    op.forward_multiple_weights(x, [w, w, w], splits, scatter, outputs_buf=bufs)
+    first, *rest = rec.calls
+    assert first.gathered == 1 and first.a_sorted_rows >= tokens * topk + 300
+    assert [(a.gathered, a.a, a.reuse_schedule) for a in rest] == [(0, first.a_sorted, 1)] * 2

@@ -202,3 +202,26 @@ def test_grouped_pairs(dev, dtype, splits, N, K):
         y = rs.forward_gather_rs(x, w, sp, scatter, output_vec_scale=gate)
         assert (y[perm].float() - ref * gate[:, None]).abs().max().item() <= tol
     rs.check_status()
+
+
+def test_moe_layer0_one_op_unequal_buffers_and_types(dev):
+    """One op called with 1-byte rows, then 2-byte rows, the second group's output buffer longer than the first's."""
+    from moe_common import routed_problem
+    import tempname_new_b200 as flux
+    tokens, H, ffn, E, topk = 300, 256, 264, 8, 2
+    _, _, scatter, splits, order = routed_problem(tokens, topk, E, seed=5, device=dev)
+    env = flux.DistEnvTPWithEP(dist.group.WORLD, 1, None, ep_size=1)
+    op = flux.GemmGroupedV3AGScatter(env, flux.MoeArguments(tokens, H, ffn, E, topk, torch.bfloat16, torch.bfloat16))
+    expert = torch.repeat_interleave(torch.arange(E, device=dev), splits.long())
+    for dtype in (torch.float8_e4m3fn, torch.bfloat16, torch.float8_e4m3fn):
+        x = (torch.randn(tokens, H, device=dev) * 0.5).to(dtype)
+        ws = [(torch.randn(E, ffn, H, device=dev) * 0.2).to(dtype) for _ in range(2)]
+        bufs = [torch.full((tokens * topk + extra, ffn), float("nan"), device=dev, dtype=torch.bfloat16)
+                for extra in (0, 500)]
+        outs = op.forward_multiple_weights(x, ws, splits, scatter, outputs_buf=bufs)
+        rows = x[order // topk].float()
+        for out, w in zip(outs, ws):
+            ref = torch.cat([rows[expert == e] @ w[e].float().t() for e in range(E)])
+            assert (out[:tokens * topk].float() - ref).abs().max().item() <= 1e-2 * ref.abs().max().item()
+            assert out[tokens * topk:].isnan().all()
+    op.check_status()
