@@ -192,6 +192,9 @@ class GemmGroupedV3AGScatter(FusedOpBase):
         if not inputs_shard.is_cuda:
             return self._forward_cpu(inputs_shard, weights, splits_gpu, scatter_index.reshape(tokens, topk),
                                      output_scale, outputs_buf, allgather_output)
+        if self.land is not None and tokens * H * inputs_shard.element_size() > self.land.nbytes:
+            raise ValueError(f"op was built for {self.args.hidden} {self.args.input_dtype} values per token; "
+                             f"{tokens} tokens of {H} {inputs_shard.dtype} do not fit its landing buffer")
         dev = inputs_shard.device
         x = inputs_shard if inputs_shard.is_contiguous() else inputs_shard.contiguous()
         splits = splits_gpu.to(device=dev, dtype=torch.int32).contiguous()

@@ -6,7 +6,7 @@ import pytest
 import torch
 import torch.distributed as dist
 
-from conftest import free_port
+from conftest import free_port, run_gloo
 from moe_common import routed_problem
 
 
@@ -86,3 +86,32 @@ def test_weight_groups_share_one_sorted_rows_buffer(layer0):
     first, *rest = rec.calls
     assert first.gathered == 1 and first.a_sorted_rows >= tokens * topk + 300
     assert [(a.gathered, a.a, a.reuse_schedule) for a in rest] == [(0, first.a_sorted, 1)] * 2
+
+
+def _landing_buffer(rank, world):
+    import tempname_new_b200 as flux
+    from tempname_new_b200 import _native
+    from tempname_new_b200.ops import _dense
+    tokens, H, ffn, E, topk = 128, 64, 128, 4, 2          # (of all ranks)
+    env = flux.DistEnvTPWithEP(dist.group.WORLD, 1, None, ep_size=world)
+    op = flux.GemmGroupedV3AGScatter(env, flux.MoeArguments(tokens, H, ffn, E, topk, torch.float8_e4m3fn))
+    op.status = torch.zeros(4, dtype=torch.int32)
+    rec = _Recorder(_native.lib())
+    _native.lib, _dense.current_stream_ptr = lambda: rec, lambda device=None: 0
+    _, _, scatter, splits, _ = routed_problem(tokens, topk, E)
+    for dtype, hidden, fits in ((torch.float8_e4m3fn, H, True), (torch.bfloat16, H, False),
+                                (torch.bfloat16, H // 2, True), (torch.float8_e4m3fn, 2 * H, False)):
+        x = _as_cuda(torch.zeros(tokens // world, hidden).to(dtype))
+        w = torch.zeros(E // world, ffn, hidden).to(dtype)
+        before = len(rec.calls)
+        if fits:
+            op.forward(x, w, splits, scatter)
+        else:
+            with pytest.raises(ValueError, match="landing buffer"):
+                op.forward(x, w, splits, scatter)
+        assert len(rec.calls) == before + fits
+
+
+def test_token_push_stays_inside_the_landing_buffers():
+    """Several ranks: tokens wider than the landing buffers were made for are refused, not written past their end."""
+    run_gloo(_landing_buffer, 2)
