@@ -268,8 +268,10 @@ class GemmGroupedV3AGScatter(FusedOpBase):
             else:
                 a.a_tokens = x.data_ptr()
             _native.check(_native.lib().fluxb_moe_grouped_gemm(ctypes.byref(a)), "fluxb_moe_grouped_gemm")
-            # (the in-loader gather variants selected by FLUXB_MOE_GATHER do not fill the sorted buffer)
-            self._sorted_complete = os.environ.get("FLUXB_MOE_GATHER", "") in ("", "pregather")
+            # (the in-loader gather variants do not fill the sorted buffer: those selected by FLUXB_MOE_GATHER, and
+            # what the launcher falls back to when there are more (expert, source rank) pairs than publishing flags)
+            pairs = self.E_local * (self.world if a.do_allgather else 1)
+            self._sorted_complete = pairs <= 512 and os.environ.get("FLUXB_MOE_GATHER", "") in ("", "pregather")
             outs.append(out)
         if allgather_output is not None:
             if self.world > 1:

@@ -115,3 +115,27 @@ def _landing_buffer(rank, world):
 def test_token_push_stays_inside_the_landing_buffers():
     """Several ranks: tokens wider than the landing buffers were made for are refused, not written past their end."""
     run_gloo(_landing_buffer, 2)
+
+
+def _many_experts(rank, world):
+    import tempname_new_b200 as flux
+    from tempname_new_b200 import _native
+    from tempname_new_b200.ops import _dense
+    tokens, H, ffn, topk = 128, 64, 128, 2
+    rec = _Recorder(_native.lib())
+    _native.lib, _dense.current_stream_ptr = lambda: rec, lambda device=None: 0
+    for E, first_gathers in ((256, True), (512, False)):
+        env = flux.DistEnvTPWithEP(dist.group.WORLD, 1, None, ep_size=1)
+        op = flux.GemmGroupedV3AGScatter(env, flux.MoeArguments(tokens, H, ffn * world, E, topk, torch.bfloat16))
+        op.status = torch.zeros(4, dtype=torch.int32)
+        _, _, scatter, splits, _ = routed_problem(tokens, topk, E)
+        w = torch.zeros(E, ffn, H).bfloat16()
+        del rec.calls[:]
+        op.forward_multiple_weights(_as_cuda(torch.zeros(tokens // world, H).bfloat16()), [w, w, w], splits, scatter)
+        # 512 experts from two sources: the first launch gathers in the loader, the second fills the buffer
+        assert [a.gathered for a in rec.calls] == ([1, 0, 0] if first_gathers else [1, 1, 0])
+        assert [a.do_allgather for a in rec.calls] == [1, 0, 0]
+
+
+def test_sorted_rows_are_reused_only_where_a_launch_filled_them():
+    run_gloo(_many_experts, 2)
