@@ -161,9 +161,10 @@ def base_args(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor], ou
               scale_a: Optional[torch.Tensor] = None, scale_b: Optional[torch.Tensor] = None, *,
               tile_n: int = 0, group_m: int = 0, num_sms: int = 0, act: Optional[str] = None,
               cta_group: int = 0, m: Optional[int] = None, tile_m: int = 0,
-              status: Optional[torch.Tensor] = None, keep: Optional[list] = None) -> DenseArgs:
+              status: Optional[torch.Tensor] = None, keep: Optional[list] = None, ranks: int = 1) -> DenseArgs:
     """Fill the operand part of a DenseArgs for A[rows,K], B[N,K]. ``m`` is the number of output
-    rows this GPU computes; when no tile knobs are given they come from the tuning table."""
+    rows this GPU computes; when no tile knobs are given they come from the tuning table, which answers for
+    a launch that ``ranks`` ranks take part in."""
     if not (a.is_cuda and b.is_cuda):
         raise RuntimeError("the sm_100a GEMM kernels need CUDA tensors")
     sa_shape, sb_shape = a.shape, b.shape
@@ -212,7 +213,7 @@ def base_args(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor], ou
         if keep is not None:
             keep.extend([sa, sb])
     if tile_n == 0 and cta_group == 0 and m is not None:
-        cta_group, tile_n, g, tm, pinned = _table.resolve(m, N, K, a.element_size())
+        cta_group, tile_n, g, tm, pinned = _table.resolve(m, N, K, a.element_size(), ranks)
         # (a measured or pinned entry is taken as it is; a default may give way to the split-K kernel)
         args.auto_shape = 0 if pinned or group_m or tile_m else 1
         if group_m == 0:

@@ -80,7 +80,7 @@ class AGKernel(FusedOpBase):
                 # the scales of all M rows, so they are gathered too (a small launch of the row-exchange kernel)
                 input_scale = self._gather_row_scales(input_scale, seg)
             args = _dense.base_args(a, w, bias, self.output_dtype, input_scale, weight_scale,
-                                    act=act, m=M, status=self.status, keep=keep)
+                                    act=act, m=M, status=self.status, keep=keep, ranks=self.world)
         args.M = M
         args.d, args.ldd = out.data_ptr(), out.stride(0)
         args.mode, args.rank, args.world = _dense.ALLGATHER, self.rank, self.world

@@ -76,7 +76,7 @@ class GemmRS(FusedOpBase):
                                    status=self.status, keep=keep)
         else:
             args = _dense.base_args(a, w, bias, self.output_dtype, input_scale, weight_scale,
-                                    m=M, status=self.status, keep=keep)
+                                    m=M, status=self.status, keep=keep, ranks=self.world)
         args.M = M
         args.num_sms = self._num_sms()
         args.mode, args.rank, args.world = _dense.REDUCE_SCATTER, self.rank, self.world

@@ -274,7 +274,8 @@ class GemmAllToAllTranspose(FusedOpBase):
             x2 = x2 if x2.is_contiguous() else x2.contiguous()
             keep: list = []
             args = A2AArgs()
-            base = _dense.base_args(x2, w, bias, self.output_dtype, m=x2.shape[0], status=self.status, keep=keep)
+            base = _dense.base_args(x2, w, bias, self.output_dtype, m=x2.shape[0], status=self.status, keep=keep,
+                                    ranks=self.world)
             base.M = x2.shape[0]
             # the all-to-all runs in the epilogue of the GEMM's own CTAs: nothing to carve out for
             # num_comm_sm; sm_margin shrinks the grid
@@ -475,7 +476,8 @@ class AllToAllTransposeGemm(FusedOpBase):
             keep: list = []
             land_local = self.land.view(self.rank, self.input_dtype, (M, self.hidden))
             args = A2AArgs()
-            base = _dense.base_args(land_local, w, bias, self.output_dtype, m=M, status=self.status, keep=keep)
+            base = _dense.base_args(land_local, w, bias, self.output_dtype, m=M, status=self.status, keep=keep,
+                                    ranks=self.world)
             base.M = M
             base.d, base.ldd = res.data_ptr(), N
             base.num_sms = self._num_sms(sm_margin)   # (the push runs in the GEMM's own CTAs)

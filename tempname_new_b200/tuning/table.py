@@ -32,6 +32,14 @@ DENSE_TABLE: Dict[Key, Dict[str, int]] = {
     (16384, 3584, 8192): {"cta_group": 2, "tile_n": 256, "tile_m": 512, "group_m": 2},    # 1255 | 1272
 }
 
+# The same for the fused ops of several ranks (rows of all ranks for all-gather and reduce-scatter): measured before
+# the single-GPU rules changed to what is faster there, and kept as they were measured.
+MULTI_RANK_TABLE: Dict[Key, Dict[str, int]] = {
+    (4096, 4096, 4096): {"cta_group": 2, "tile_n": 256, "tile_m": 512, "group_m": 8},
+    (4096, 12288, 4096): {"cta_group": 2, "tile_n": 256, "tile_m": 512, "group_m": 8},
+    (16384, 8192, 3584): {"cta_group": 2, "tile_n": 256, "tile_m": 512, "group_m": 8},
+}
+
 _NUM_SMS = 148
 
 
@@ -40,31 +48,37 @@ def _wave_eff(tiles: int, slots: int) -> float:
     return tiles / (waves * slots)
 
 
-def heuristic(m: int, n: int, k: int, elt: int = 2) -> Dict[str, int]:
-    """The default of a shape without a measured entry, see ``_heuristic``."""
-    cg, bn, group = _heuristic(m, n, k, elt)
+def heuristic(m: int, n: int, k: int, elt: int = 2, ranks: int = 1) -> Dict[str, int]:
+    """The default of a shape without a measured entry, see ``_heuristic``; ``ranks``: ranks of the fused op."""
+    cg, bn, group = _heuristic(m, n, k, elt, ranks)
     return {"cta_group": cg, "tile_n": bn, "group_m": group}
 
 
 @functools.lru_cache(maxsize=4096)
-def _heuristic(m: int, n: int, k: int, elt: int) -> Tuple[int, int, int]:
-    """(cta_group, tile_n, group_m): CTA pairs on 256 x 256 tiles wherever they need no more waves than single CTAs on
-    128 x 256 (1000 x 3000 x 5000 fp16: 41 against 53 us; 1500 x 4000 x 4096 bf16: 52 either way); tile_m stays 0, the
-    launcher picks 512-row tiles where K is long. Raster groups of 2048 rows (with wave-synchronous tile starts the
-    grid walks K together, so the group does not have to fit L2 over the whole K extent), of 4096 rows for the 256-row
-    tiles of a short K (4096 x 16384 x 4096 bf16 434 -> 416 us, 8192 x 8192 x 8192 fp8 427 -> 416, never slower by more
-    than the noise)."""
+def _heuristic(m: int, n: int, k: int, elt: int, ranks: int) -> Tuple[int, int, int]:
+    """(cta_group, tile_n, group_m); tile_m stays 0: the launcher picks 512-row tiles.
+
+    One rank: CTA pairs on 256 x 256 tiles wherever they need no more waves than single CTAs on 128 x 256 (1000 x
+    3000 x 5000 fp16: 41 against 53 us; 1500 x 4000 x 4096 bf16: 52 either way). Raster groups of 2048 rows (with
+    wave-synchronous tile starts the grid walks K together, so the group does not have to fit L2 over the whole K
+    extent), of 4096 rows for the 256-row tiles of a short K (4096 x 16384 x 4096 bf16 434 -> 416 us, 8192 x 8192 x
+    8192 fp8 427 -> 416, never slower by more than the noise).
+
+    Several ranks: pairs unless the problem is too small to fill 74 of them, eight tile rows per group. The tiles of
+    a short K have 512 rows there and a group that exceeds a segment's tile rows makes bands span two segments, so
+    the single-rank figures do not carry over; these are the choices that the fused ops were measured with."""
     up = lambda a, b: -(-a // b)  # noqa: E731
     t1, t2 = up(m, 128) * up(n, 256), up(m, 256) * up(n, 256)
-    pairs = m >= 256 and n >= 256
-    if pairs and ((m // 256) * up(n, 256) >= _NUM_SMS // 4 or
-                  (t2 >= _NUM_SMS // 8 and up(t2, _NUM_SMS // 2) <= up(t1, _NUM_SMS))):
+    fill = m >= 256 and n >= 256 and (m // 256) * up(n, 256) >= _NUM_SMS // 4
+    no_more_waves = (ranks == 1 and m >= 256 and n >= 256 and t2 >= _NUM_SMS // 8
+                     and up(t2, _NUM_SMS // 2) <= up(t1, _NUM_SMS))
+    if fill or no_more_waves:
         cg, bn = 2, 256
     elif n % 256 == 0 or n > 2048:
         cg, bn = 1, 256
     else:
         cg, bn = 1, 128
-    group = 16 if cg == 1 or k * elt < 80 * 128 else 8
+    group = 16 if cg == 1 or (ranks == 1 and k * elt < 80 * 128) else 8
     return cg, bn, group
 
 
@@ -117,19 +131,20 @@ class override:
         return False
 
 
-def _entry(key: Key):
+def _entry(key: Key, ranks: int = 1):
     global _EXTRA
     if _EXTRA is None:
         _EXTRA = _load_extra()
     for table in (_OVERRIDE, _EXTRA, DENSE_TABLE):
         if key in table:
             return table[key]
-    return None
+    return MULTI_RANK_TABLE.get(key) if ranks > 1 else None
 
 
-def lookup(m: int, n: int, k: int, elt: int = 2) -> Dict[str, int]:
-    e = _entry((m, n, k))
-    return dict(e) if e is not None else heuristic(m, n, k, elt)
+def lookup(m: int, n: int, k: int, elt: int = 2, ranks: int = 1) -> Dict[str, int]:
+    """Knobs of a dense launch of ``m`` rows, for an op whose ``ranks`` ranks take part in one fused launch."""
+    e = _entry((m, n, k), ranks)
+    return dict(e) if e is not None else heuristic(m, n, k, elt, ranks)
 
 
 def pinned(m: int, n: int, k: int) -> bool:
@@ -137,9 +152,9 @@ def pinned(m: int, n: int, k: int) -> bool:
     return _entry((m, n, k)) is not None
 
 
-def resolve(m: int, n: int, k: int, elt: int = 2) -> Tuple[int, int, int, int, bool]:
+def resolve(m: int, n: int, k: int, elt: int = 2, ranks: int = 1) -> Tuple[int, int, int, int, bool]:
     """``lookup`` and ``pinned`` for a launch: (cta_group, tile_n, group_m, tile_m, pinned)."""
-    e = _entry((m, n, k))
+    e = _entry((m, n, k), ranks)
     if e is not None:
         return e["cta_group"], e["tile_n"], e["group_m"], e.get("tile_m", 0), True
-    return (*_heuristic(m, n, k, elt), 0, False)
+    return (*_heuristic(m, n, k, elt, ranks), 0, False)

@@ -1,0 +1,57 @@
+"""The tile choices of the dense kernel and what the ops hand to its launcher, on the CPU."""
+import pytest
+import torch
+
+from conftest import run_gloo
+from fake_launch import as_cuda, record_launches
+from tempname_new_b200.tuning import table
+
+
+def _several_ranks(m, n, k):
+    """The choices that the fused ops of several ranks were measured with."""
+    if (m, n, k) in ((4096, 4096, 4096), (4096, 12288, 4096), (16384, 8192, 3584)):
+        return {"cta_group": 2, "tile_n": 256, "tile_m": 512, "group_m": 8}
+    if m >= 256 and n >= 256 and (m // 256) * -(-n // 256) >= 37:
+        return {"cta_group": 2, "tile_n": 256, "group_m": 8}
+    return {"cta_group": 1, "tile_n": 256 if n % 256 == 0 or n > 2048 else 128, "group_m": 16}
+
+
+@pytest.mark.parametrize("ranks", [2, 4, 8])
+def test_tile_choices_of_several_ranks(ranks):
+    for m in (64, 256, 300, 1000, 1024, 2048, 4096, 8192, 16384, 32768):
+        for n in (128, 264, 1024, 3000, 4096, 8192, 12288):
+            for k in (256, 3584, 4096, 5120, 12288):
+                if (m, n, k) not in table.DENSE_TABLE:
+                    for elt in (1, 2):
+                        assert table.lookup(m, n, k, elt, ranks) == _several_ranks(m, n, k)
+    assert table.lookup(8192, 12288, 49152, 2, ranks)["group_m"] == 4
+
+
+def _rank_counts(rank, world):
+    import tempname_new_b200 as flux
+    import torch.distributed as dist
+    rec = record_launches()
+    pg, status, bf = dist.group.WORLD, torch.zeros(4, dtype=torch.int32), torch.bfloat16
+    M, N, K = 2048, 4096, 1024              # a short K: one rank alone would take bands of 16 tile rows
+    seen = table.lookup(M, N, K), table.lookup(M, N, K, 2, world)
+    assert seen[0]["group_m"] == 16 and seen[1]["group_m"] == 8
+    x, w = as_cuda(torch.zeros(M, K, dtype=bf)), as_cuda(torch.zeros(N, K, dtype=bf))
+    rs = flux.GemmRS(pg, 1, M, N, bf)
+    ag = flux.AGKernel(pg, 1, M, N, K, bf)
+    pre = flux.GemmAllToAllTranspose(pg, 1, world, 1, M * world, K, 64, N, bf)
+    post = flux.AllToAllTransposeGemm(pg, 1, world, 1, K // 64, M * world, 64, bf)
+    for op in (rs, ag, pre, post):
+        op.status = status
+    post.land.view = lambda r, dtype, shape: as_cuda(torch.zeros(shape, dtype=dtype))
+    rs.forward(x, w)
+    ag.forward(x[:M // world], w)
+    pre.forward(x.view(1, M, K), w)
+    post.forward(as_cuda(torch.zeros(1, K // 64 // world, M * world, 64, dtype=bf)), w)
+    assert len(rec.calls) == 4
+    for a in rec.calls:
+        b = getattr(a, "base", a)
+        assert (b.cta_group, b.tile_n, b.group_m) == (2, 256, 8)
+
+
+def test_fused_ops_ask_for_their_rank_count():
+    run_gloo(_rank_counts, 2)

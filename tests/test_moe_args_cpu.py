@@ -1,38 +1,11 @@
-"""What the MoE layer-0 op hands to its kernel, checked on the CPU: tensors that claim to live on a GPU take the op's
-CUDA branch, and a recorder stands in for the launch."""
-import ctypes
-
+"""What the MoE layer-0 op hands to its kernel, on the CPU."""
 import pytest
 import torch
 import torch.distributed as dist
 
 from conftest import free_port, run_gloo
+from fake_launch import Recorder, as_cuda, record_launches
 from moe_common import routed_problem
-
-
-class _AsCuda(torch.Tensor):
-    """A CPU tensor that takes the CUDA branch of the ops."""
-    is_cuda = True
-
-
-def _as_cuda(t):
-    return torch.Tensor._make_subclass(_AsCuda, t)
-
-
-class _Recorder:
-    """The native library, except that a grouped GEMM only leaves a copy of its arguments."""
-
-    def __init__(self, lib):
-        self._lib, self.calls = lib, []
-
-    def __getattr__(self, name):
-        return getattr(self._lib, name)
-
-    def fluxb_moe_grouped_gemm(self, ref):
-        kept = type(ref._obj)()
-        ctypes.memmove(ctypes.byref(kept), ref, ctypes.sizeof(kept))
-        self.calls.append(kept)
-        return 0
 
 
 @pytest.fixture
@@ -45,7 +18,7 @@ def layer0(monkeypatch):
     created = not dist.is_initialized()
     if created:
         dist.init_process_group("gloo", init_method=f"tcp://127.0.0.1:{free_port()}", rank=0, world_size=1)
-    rec = _Recorder(_native.lib())
+    rec = Recorder(_native.lib())
     monkeypatch.setattr(_native, "lib", lambda: rec)
     monkeypatch.setattr(_dense, "current_stream_ptr", lambda device=None: 0)
 
@@ -67,7 +40,7 @@ def test_sorted_rows_buffer_follows_the_element_type(layer0):
     tokens, H, ffn, E, topk = 256, 64, 128, 4, 2
     op, rec, splits, scatter = layer0(tokens, H, ffn, E, topk, torch.bfloat16)
     for dtype in (torch.float8_e4m3fn, torch.bfloat16, torch.float8_e4m3fn):
-        x = _as_cuda(torch.zeros(tokens, H).to(dtype))
+        x = as_cuda(torch.zeros(tokens, H).to(dtype))
         op.forward(x, torch.zeros(E, ffn, H).to(dtype), splits, scatter)
         a = rec.calls[-1]
         assert a.a_sorted == op._sorted.data_ptr() and a.a_sorted_rows >= tokens * topk
@@ -79,7 +52,7 @@ def test_weight_groups_share_one_sorted_rows_buffer(layer0):
     """Groups after the first read the rows that the first one gathered, also when their output buffer is longer."""
     tokens, H, ffn, E, topk = 256, 64, 128, 4, 2
     op, rec, splits, scatter = layer0(tokens, H, ffn, E, topk, torch.bfloat16)
-    x = _as_cuda(torch.zeros(tokens, H).bfloat16())
+    x = as_cuda(torch.zeros(tokens, H).bfloat16())
     w = torch.zeros(E, ffn, H).bfloat16()
     bufs = [torch.empty(n, ffn).bfloat16() for n in (tokens * topk, tokens * topk + 300, tokens * topk)]
     op.forward_multiple_weights(x, [w, w, w], splits, scatter, outputs_buf=bufs)
@@ -90,18 +63,15 @@ def test_weight_groups_share_one_sorted_rows_buffer(layer0):
 
 def _landing_buffer(rank, world):
     import tempname_new_b200 as flux
-    from tempname_new_b200 import _native
-    from tempname_new_b200.ops import _dense
     tokens, H, ffn, E, topk = 128, 64, 128, 4, 2          # (of all ranks)
     env = flux.DistEnvTPWithEP(dist.group.WORLD, 1, None, ep_size=world)
     op = flux.GemmGroupedV3AGScatter(env, flux.MoeArguments(tokens, H, ffn, E, topk, torch.float8_e4m3fn))
     op.status = torch.zeros(4, dtype=torch.int32)
-    rec = _Recorder(_native.lib())
-    _native.lib, _dense.current_stream_ptr = lambda: rec, lambda device=None: 0
+    rec = record_launches()
     _, _, scatter, splits, _ = routed_problem(tokens, topk, E)
     for dtype, hidden, fits in ((torch.float8_e4m3fn, H, True), (torch.bfloat16, H, False),
                                 (torch.bfloat16, H // 2, True), (torch.float8_e4m3fn, 2 * H, False)):
-        x = _as_cuda(torch.zeros(tokens // world, hidden).to(dtype))
+        x = as_cuda(torch.zeros(tokens // world, hidden).to(dtype))
         w = torch.zeros(E // world, ffn, hidden).to(dtype)
         before = len(rec.calls)
         if fits:
@@ -119,11 +89,8 @@ def test_token_push_stays_inside_the_landing_buffers():
 
 def _many_experts(rank, world):
     import tempname_new_b200 as flux
-    from tempname_new_b200 import _native
-    from tempname_new_b200.ops import _dense
     tokens, H, ffn, topk = 128, 64, 128, 2
-    rec = _Recorder(_native.lib())
-    _native.lib, _dense.current_stream_ptr = lambda: rec, lambda device=None: 0
+    rec = record_launches()
     for E, first_gathers in ((256, True), (512, False)):
         env = flux.DistEnvTPWithEP(dist.group.WORLD, 1, None, ep_size=1)
         op = flux.GemmGroupedV3AGScatter(env, flux.MoeArguments(tokens, H, ffn * world, E, topk, torch.bfloat16))
@@ -131,7 +98,7 @@ def _many_experts(rank, world):
         _, _, scatter, splits, _ = routed_problem(tokens, topk, E)
         w = torch.zeros(E, ffn, H).bfloat16()
         del rec.calls[:]
-        op.forward_multiple_weights(_as_cuda(torch.zeros(tokens // world, H).bfloat16()), [w, w, w], splits, scatter)
+        op.forward_multiple_weights(as_cuda(torch.zeros(tokens // world, H).bfloat16()), [w, w, w], splits, scatter)
         # 512 experts from two sources: the first launch gathers in the loader, the second fills the buffer
         assert [a.gathered for a in rec.calls] == ([1, 0, 0] if first_gathers else [1, 1, 0])
         assert [a.do_allgather for a in rec.calls] == [1, 0, 0]
