@@ -20,6 +20,7 @@ from typing import Optional
 import torch
 import torch.distributed as dist
 from torch import nn
+from torch.autograd import forward_ad
 
 from ..ops.ag_gemm import AGKernel
 from ..ops.gemm_rs import GemmRS
@@ -154,9 +155,11 @@ class RowParallelLinear(nn.Module):
         b = self.bias
         if (b is not None and x.is_cuda and self._cache.world == 1 and b.dtype == x.dtype
                 and b.device == x.device and b.is_contiguous()
-                and (x.requires_grad or self.weight.requires_grad or not b.requires_grad)):
+                and (x.requires_grad or self.weight.requires_grad or not b.requires_grad)
+                and forward_ad.unpack_dual(b).tangent is None):
             # one rank: the GEMM's epilogue adds the bias to the fp32 sum (a broadcast add over 8192 x 12288 bf16
-            # is 235 us next to a GEMM of 970); a bias that trains alone keeps its add, whose backward is one sum
+            # is 235 us next to a GEMM of 970); a bias that trains alone keeps its add, whose backward is one sum, and so
+            # does one with a forward-mode tangent, which the fused op has no rule for
             return _RowParallelFn.apply(x, self.weight, self._cache, b)
         y = _RowParallelFn.apply(x, self.weight, self._cache)
         return y + b if b is not None else y

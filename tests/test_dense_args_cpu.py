@@ -1,9 +1,11 @@
 """The tile choices of the dense kernel and what the ops hand to its launcher, on the CPU."""
 import pytest
 import torch
+import torch.distributed as dist
+from torch.autograd import forward_ad
 
-from conftest import run_gloo
-from fake_launch import as_cuda, record_launches
+from conftest import free_port, run_gloo
+from fake_launch import Recorder, as_cuda, record_launches
 from tempname_new_b200.tuning import table
 
 
@@ -29,7 +31,6 @@ def test_tile_choices_of_several_ranks(ranks):
 
 def _rank_counts(rank, world):
     import tempname_new_b200 as flux
-    import torch.distributed as dist
     rec = record_launches()
     pg, status, bf = dist.group.WORLD, torch.zeros(4, dtype=torch.int32), torch.bfloat16
     M, N, K = 2048, 4096, 1024              # a short K: one rank alone would take bands of 16 tile rows
@@ -55,3 +56,39 @@ def _rank_counts(rank, world):
 
 def test_fused_ops_ask_for_their_rank_count():
     run_gloo(_rank_counts, 2)
+
+
+@pytest.fixture
+def row_parallel(monkeypatch):
+    """A row-parallel layer of one rank that takes the CUDA branch, its input, and the recorder."""
+    from tempname_new_b200 import _native
+    from tempname_new_b200.ops import _dense
+    from tempname_new_b200.parallel.layers import RowParallelLinear
+    created = not dist.is_initialized()
+    if created:
+        dist.init_process_group("gloo", init_method=f"tcp://127.0.0.1:{free_port()}", rank=0, world_size=1)
+    rec = Recorder(_native.lib())
+    monkeypatch.setattr(_native, "lib", lambda: rec)
+    monkeypatch.setattr(_dense, "current_stream_ptr", lambda device=None: 0)
+    lin = RowParallelLinear(64, 128)
+    lin.requires_grad_(False)
+    lin.weight = torch.nn.Parameter(as_cuda(lin.weight.data), requires_grad=False)
+    lin._cache.rs(32, 128, torch.bfloat16).status = torch.zeros(4, dtype=torch.int32)
+    yield lin, as_cuda(torch.zeros(32, 64, dtype=torch.bfloat16)), rec
+    lin._cache.ops.clear()
+    if created:
+        dist.destroy_process_group()
+
+
+def test_row_parallel_bias_with_a_forward_mode_tangent(row_parallel):
+    lin, x, rec = row_parallel
+    lin(x)
+    assert rec.calls[-1].bias == lin.bias.data_ptr()
+    bias = lin.bias.detach()
+    tangent = torch.randn(128).bfloat16()
+    del lin.bias
+    with forward_ad.dual_level():
+        lin.bias = forward_ad.make_dual(bias, tangent)
+        y = lin(x)
+        assert rec.calls[-1].bias is None
+        assert torch.equal(forward_ad.unpack_dual(y).tangent, tangent.expand(32, 128))
