@@ -154,7 +154,7 @@ class RowParallelLinear(nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         b = self.bias
         if (b is not None and x.is_cuda and self._cache.world == 1 and b.dtype == x.dtype
-                and b.device == x.device and b.is_contiguous()
+                and b.device == x.device and b.is_contiguous() and b.shape == self.weight.shape[:1]
                 and (x.requires_grad or self.weight.requires_grad or not b.requires_grad)
                 and forward_ad.unpack_dual(b).tangent is None):
             # one rank: the GEMM's epilogue adds the bias to the fp32 sum (a broadcast add over 8192 x 12288 bf16

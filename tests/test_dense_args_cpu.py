@@ -92,3 +92,15 @@ def test_row_parallel_bias_with_a_forward_mode_tangent(row_parallel):
         y = lin(x)
         assert rec.calls[-1].bias is None
         assert torch.equal(forward_ad.unpack_dual(y).tangent, tangent.expand(32, 128))
+
+
+@pytest.mark.parametrize("shape", [(1, 128), (1,), (), (32, 128)])
+def test_row_parallel_bias_that_broadcasts(row_parallel, shape):
+    """A bias of another shape than [out] is added as PyTorch broadcasts it, and gets a gradient of its shape."""
+    lin, x, rec = row_parallel
+    lin.bias = torch.nn.Parameter(torch.randn(shape).bfloat16())
+    x.requires_grad_(True)
+    y = lin(x)
+    assert rec.calls[-1].bias is None and y.shape == (32, 128)
+    (g,) = torch.autograd.grad(y, [lin.bias], torch.ones(32, 128).bfloat16())
+    assert g.shape == shape and torch.equal(g, torch.full(shape, 32 * 128 / max(1, lin.bias.numel())).bfloat16())
