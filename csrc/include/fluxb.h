@@ -111,6 +111,17 @@ int fluxb_decode_work_items(int32_t num_seg, int32_t seg_first, int32_t m_tiles_
                             int32_t split_from, int32_t split_shift, int32_t* out, int32_t n);
 /* number of kernels libfluxb launched from this process so far */
 uint64_t fluxb_launch_count(void);
+
+/* The last GEMM that the calling thread launched: which kernel the rules chose, and how (tests, profiles). */
+enum { FLUXB_KERNEL_NONE = 0, FLUXB_KERNEL_PERSISTENT = 1, FLUXB_KERNEL_SPLIT_K = 2, FLUXB_KERNEL_GROUPED = 3 };
+typedef struct {
+  int32_t kernel, tile_m, tile_n;   /* rows and columns of a tile */
+  int32_t cta_group;                /* CTAs that share a tile's MMAs: 1 or 2 */
+  int32_t splits;                   /* split-K: CTAs per tile, each with its share of K; persistent: column pieces
+                                       that each tile of the last wave is cut into; else 1 */
+  int32_t cooperative;              /* 1: launched with the cooperative attribute */
+} fluxb_gemm_launch_t;
+int fluxb_last_gemm(fluxb_gemm_launch_t* out);
 /* zero the launcher's per-stream wave counters of the current device (synchronises the device);
  * needed only after a launch was cut short by a timed-out wait */
 int fluxb_reset_wave_counters(void);

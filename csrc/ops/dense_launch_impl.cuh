@@ -46,6 +46,7 @@ int launch_dense(const DenseGemmParams& p, int grid, cudaStream_t stream, bool c
   }
   FLUXB_CUDA_OK(cudaGetLastError());
   g_launches.fetch_add(1, std::memory_order_relaxed);
+  note_gemm({FLUXB_KERNEL_PERSISTENT, Cfg::BM, Cfg::BN, Cfg::CG, 1 << p.split_shift, coop ? 1 : 0});
   return kOk;
 }
 

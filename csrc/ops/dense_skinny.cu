@@ -36,6 +36,7 @@ int launch_skinny(const SkinnyParams& p, int grid, cudaStream_t stream) {
   FLUXB_CUDA_OK(cudaLaunchKernelEx(&cfg, skinny_gemm_kernel<Cfg>, p));
   FLUXB_CUDA_OK(cudaGetLastError());
   g_launches.fetch_add(1, std::memory_order_relaxed);
+  note_gemm({FLUXB_KERNEL_SPLIT_K, 128, Cfg::BN, 1, p.splits, 0});
   return kOk;
 }
 

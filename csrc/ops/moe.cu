@@ -286,6 +286,7 @@ int launch_grouped(const GroupedParams& p, int grid, cudaStream_t stream) {
   }
   FLUXB_CUDA_OK(cudaGetLastError());
   g_launches.fetch_add(1, std::memory_order_relaxed);
+  note_gemm({FLUXB_KERNEL_GROUPED, Cfg::BM, Cfg::BN, Cfg::CG, 1, 0});
   return kOk;
 }
 

@@ -6,6 +6,9 @@
 namespace fluxb {
 
 static thread_local std::string g_last_error;
+static thread_local fluxb_gemm_launch_t g_last_gemm = {};
+
+void note_gemm(const fluxb_gemm_launch_t& launch) { g_last_gemm = launch; }
 
 void set_last_error(const std::string& msg) { g_last_error = msg; }
 
@@ -85,5 +88,11 @@ int device_sm_count(int* out) {
 }
 
 }  // namespace fluxb
+
+extern "C" int fluxb_last_gemm(fluxb_gemm_launch_t* out) {
+  FLUXB_REQUIRE(out != nullptr, "null record");
+  *out = fluxb::g_last_gemm;
+  return fluxb::kOk;
+}
 
 extern "C" const char* fluxb_last_error() { return fluxb::g_last_error.c_str(); }

@@ -9,6 +9,8 @@
 
 #include <string>
 
+#include "../include/fluxb.h"
+
 namespace fluxb {
 
 // Error codes returned by every extern "C" entry point.
@@ -46,6 +48,8 @@ int encode_tmap(CUtensorMap* out, CUtensorMapDataType dt, int nd, const void* ba
                 const uint64_t* dims, const uint64_t* strides_bytes, const uint32_t* box, Swz swz);
 
 int device_sm_count(int* out);
+// What fluxb_last_gemm answers on this thread from now on.
+void note_gemm(const fluxb_gemm_launch_t& launch);
 // A zeroed device word from a small per-device pool, for launches that keep their CTAs in step wave
 // by wave; the launch leaves it at zero again. One word per stream (csrc/ops/dense_gemm.cu); null
 // when the pool has no word left for a new stream.

@@ -145,3 +145,20 @@ def check(rc: int, what: str = "libfluxb call") -> None:
 
 def launch_count() -> int:
     return int(lib().fluxb_launch_count())
+
+
+class GemmLaunch(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_int32) for n in ("kernel", "tile_m", "tile_n", "cta_group", "splits", "cooperative")]
+
+
+_KERNELS = ("none", "persistent", "split_k", "grouped")
+
+
+def last_gemm() -> dict:
+    """Which kernel the calling thread's last GEMM launch took, and how: ``kernel`` ("persistent", "split_k" or
+    "grouped"), ``tile_m``, ``tile_n``, ``cta_group``, ``splits``, ``cooperative``."""
+    rec = GemmLaunch()
+    check(lib().fluxb_last_gemm(ctypes.byref(rec)), "fluxb_last_gemm")
+    out = {name: int(getattr(rec, name)) for name, _ in rec._fields_}
+    out["kernel"] = _KERNELS[out["kernel"]]
+    return out

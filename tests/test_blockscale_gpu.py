@@ -120,6 +120,7 @@ def test_blockscale_ragged_rows(dev):
                                    (1000, 2048, 2048), (64, 16384, 640)])
 def test_split_k_block_scaled(dev, M, N, K):
     """The split-K form against 64 bits and against the persistent kernel: partial row blocks, one to four splits."""
+    from tempname_new_b200 import _native
     from tempname_new_b200.ops import _dense
     from tempname_new_b200.ops.blockscale_gemm import blockscale_args
     import tempname_new_b200 as flux
@@ -132,21 +133,25 @@ def test_split_k_block_scaled(dev, M, N, K):
     bd = b.double().view(N, K // 128, 128) * sb.double().repeat_interleave(128, 0)[:, :, None]
     ref = ad.reshape(M, K) @ bd.reshape(N, K).t() + bias.double()
     new = flux.BlockScaleGemm().forward(a, b, bias=bias, input_scale=sa, weight_scale=sb)
+    assert _native.last_gemm()["kernel"] == "split_k"
     old = torch.empty(M, N, device=dev, dtype=torch.bfloat16)
     args = blockscale_args(a, b, sa, sb, bias, torch.bfloat16, M)
     args.auto_shape, args.tile_n, args.M, args.d, args.ldd = 0, 128, M, old.data_ptr(), N
     args.mode, args.rank, args.world, args.epoch = _dense.PLAIN, 0, 1, 1
     _dense.run(args)
+    assert _native.last_gemm()["kernel"] == "persistent"
     e_new, e_old = ((t.double() - ref).norm().item() for t in (new, old))
     assert not new.isnan().any() and e_new <= 1.02 * e_old and e_new <= 2e-3 * ref.norm().item()
 
 
-@pytest.mark.parametrize("M,N,K", [(200, 2176, 384), (128, 256, 128), (2432, 2304, 640), (1184, 4224, 256), (2500, 1920, 512)])
+@pytest.mark.parametrize("M,N,K", [(200, 2176, 384), (128, 256, 128), (2432, 2304, 640), (1184, 4224, 256),
+                                   (2500, 1792, 512), (2500, 1920, 512)])
 @pytest.mark.parametrize("groupwise", [False, True])
 def test_cut_tiles_of_the_last_wave(dev, M, N, K, groupwise):
     """128 x 256 tiles whose last wave is cut into 128-column halves (all tiles, some, none; a half past the last column),
-    with one weight scale per block and per column: against 64 bits, and bit for bit against whole 128 x 128 tiles,
-    which multiply and add in the same order."""
+    with one weight scale per block, and the same problems with one per column, whose tiles stay whole: against 64 bits,
+    and bit for bit against whole 128 x 128 tiles, which multiply and add in the same order."""
+    from tempname_new_b200 import _native
     from tempname_new_b200.ops import _dense
     from tempname_new_b200.ops.blockscale_gemm import blockscale_args
     g = torch.Generator(device=dev).manual_seed(M + N + K)
@@ -163,6 +168,10 @@ def test_cut_tiles_of_the_last_wave(dev, M, N, K, groupwise):
         args.auto_shape, args.tile_n, args.M, args.d, args.ldd = 0, tile_n, M, out.data_ptr(), N
         args.mode, args.rank, args.world, args.epoch = _dense.PLAIN, 0, 1, 1
         _dense.run(args)
+        ran = _native.last_gemm()
+        wide = tile_n == 256 and N != 1920         # (an odd number of 128-column blocks below 2048: narrow tiles)
+        cut = 2 if wide and not groupwise and M != 2500 else 1
+        assert (ran["kernel"], ran["tile_n"], ran["splits"]) == ("persistent", 256 if wide else 128, cut)
         assert (out.double() - ref).norm().item() <= 2e-3 * ref.norm().item()
         outs.append(out)
     assert torch.equal(*outs)

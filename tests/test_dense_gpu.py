@@ -309,6 +309,7 @@ def test_split_k(dev, M, N, K, dtype):
     fp32 sums in another order, so the outputs differ by an ulp of the 16-bit result here and there, and for int8,
     whose sums are exact, not at all."""
     import tempname_new_b200 as flux
+    from tempname_new_b200 import _native
     from tempname_new_b200.ops import _dense
     g = torch.Generator(device=dev).manual_seed(M + N + K)
     odt = torch.float16 if dtype == torch.float16 else torch.bfloat16
@@ -319,7 +320,8 @@ def test_split_k(dev, M, N, K, dtype):
         a, b = (torch.randn(s, device=dev, generator=g).to(dtype) for s in ((M, K), (N, K)))
         sa = sb = None if dtype.itemsize == 2 else torch.full((1,), 0.5, device=dev)
     eb = 128 // dtype.itemsize
-    assert _shape_rule(M, N, -(-K // eb))[0] != 0
+    rule = _shape_rule(M, N, -(-K // eb))
+    assert rule[0] != 0
     bias = torch.randn(1, N, device=dev, generator=g).to(odt)
     big = torch.full((M, N + 8), float("nan"), device=dev, dtype=odt)      # (an output with a row pitch)
     ref = a.double() @ b.double().t()
@@ -328,8 +330,11 @@ def test_split_k(dev, M, N, K, dtype):
     ref = ref + bias.double()
     out = flux.GemmOnly(dtype, output_dtype=odt, use_fp8_gemm=dtype.itemsize == 1).forward(
         a, b, bias=bias, output_buf=big[:, :N], input_scale=sa, weight_scale=sb)
+    ran = _native.last_gemm()
+    assert (ran["kernel"], ran["tile_n"], ran["splits"]) == ("split_k", rule[0], rule[2])
     old = torch.empty(M, N, device=dev, dtype=odt)
     _dense.plain_gemm(a, b, old, bias, sa, sb, tile_n=128, cta_group=1)
+    assert _native.last_gemm()["kernel"] == "persistent"
     assert big[:, N:].isnan().all() and not out.isnan().any()
     # half a unit in the last place: at most 2^-8 of the value with bf16's 8 significant bits, 2^-11 with fp16's 11;
     # the fp32 sums of K products err by far less
@@ -343,6 +348,7 @@ def test_split_k(dev, M, N, K, dtype):
         for act in ("gelu", "relu", "silu"):
             new = torch.empty(M, N, device=dev, dtype=odt)
             _dense.plain_gemm(a, b.t().contiguous().t(), new, bias[0], act=act)
+            assert _native.last_gemm()["kernel"] == "split_k"
             _dense.plain_gemm(a, b, old, bias[0], act=act, tile_n=128, cta_group=1)
             assert (new.double() - old.double()).abs().max() <= 2 * ulp * max(1.0, old.abs().max().item())
     again = torch.empty(M, N, device=dev, dtype=odt)
@@ -352,6 +358,7 @@ def test_split_k(dev, M, N, K, dtype):
 
 def test_split_k_rule_and_knobs(dev):
     """Pinned knobs, a margin of SMs and a timeline stay with the persistent kernel; a status word stays clear."""
+    from tempname_new_b200 import _native
     from tempname_new_b200.ops import _dense
     from tempname_new_b200.tuning import table
     assert _shape_rule(16, 4096, 256) == (128, 32, 4)
@@ -361,17 +368,20 @@ def test_split_k_rule_and_knobs(dev):
     a, b = _ab(16, 512, 1024, dev)
     out, ref = torch.empty(16, 512, device=dev, dtype=torch.bfloat16), a.float() @ b.float().t()
     status = torch.zeros(4, dtype=torch.int32, device=dev)
-    for kw in (dict(), dict(num_sms=20), dict(group_m=2)):
+    for kernel, kw in (("split_k", dict()), ("persistent", dict(num_sms=20)), ("persistent", dict(group_m=2))):
         out.fill_(float("nan"))
         _dense.plain_gemm(a, b, out, status=status, **kw)
+        assert _native.last_gemm()["kernel"] == kernel
         assert (out.float() - ref).abs().max().item() <= _tol(ref) and status.tolist()[0] == 0
     with table.override((16, 512, 1024), {"cta_group": 1, "tile_n": 128, "group_m": 8}):
-        assert table.pinned(16, 512, 1024)
+        assert table.resolve(16, 512, 1024)[-1]
+        out.fill_(float("nan"))
         _dense.plain_gemm(a, b, out)
-    assert not table.pinned(16, 512, 1024) and (out.float() - ref).abs().max().item() <= _tol(ref)
+        assert _native.last_gemm()["kernel"] == "persistent"
+    assert not table.resolve(16, 512, 1024)[-1] and (out.float() - ref).abs().max().item() <= _tol(ref)
     with _dense.KernelTimeline(dev) as tl:
         _dense.plain_gemm(a, b, out)
-        assert "entry_us" in tl.summary()
+        assert _native.last_gemm()["kernel"] == "persistent" and "entry_us" in tl.summary()
 
 
 @pytest.mark.parametrize("N,shift,rows", [(512, 0, 1), (520, 0, 1), (512, 1, 1), (512, 8, 1), (776, 0, 700), (776, 4, 700)])

@@ -114,16 +114,13 @@ def test_moe_layer1_fused_fp8(dev):
     op.check_status()
 
 
-@pytest.mark.parametrize("tokens,E,topk,kind", [(3, 8, 2, "random"), (64, 64, 8, "random"), (64, 64, 1, "one"),
-                                                (300, 128, 2, "few"), (4801, 32, 4, "random"), (4801, 8, 4, "one")])
-def test_moe_layer0_gather_chunks(dev, tokens, E, topk, kind):
-    """Rows are gathered in chunks that may touch several experts (one to four rows each), and an expert is published
-    when its last row is written: empty experts, one-row experts, all rows on one expert, twice on the same op."""
+def _gather_case(dev, tokens, E, topk, kind, H, ffn):
+    """Layer 0 with two weight groups, twice on one op, against fp32; returns (rows per chunk, the first GEMM's launch)."""
     import tempname_new_b200 as flux
-    H, ffn = 136, 128
+    from tempname_new_b200 import _native
     g = torch.Generator(device=dev).manual_seed(tokens + E)
     if kind == "random":
-        chosen = torch.stack([torch.randperm(E, device=dev, generator=g)[:topk] for _ in range(tokens)])
+        chosen = torch.rand(tokens, E, device=dev, generator=g).topk(topk, dim=1).indices
     elif kind == "one":
         chosen = torch.arange(topk, device=dev).add(E - topk).repeat(tokens, 1)
     else:
@@ -137,17 +134,49 @@ def test_moe_layer0_gather_chunks(dev, tokens, E, topk, kind):
     w = [(torch.randn(E, ffn, H, device=dev, generator=g) * 0.2).bfloat16() for _ in range(2)]
     env = flux.DistEnvTPWithEP(dist.group.WORLD, 1, None, ep_size=1)
     op = flux.GemmGroupedV3AGScatter(env, flux.MoeArguments(tokens, H, ffn, E, topk, torch.bfloat16, torch.bfloat16))
-    rows = x[order // topk].float()
+    rows = x[order // topk].double()
     expert = chosen.reshape(-1)[order].long()
-    ref = [torch.empty(tokens * topk, ffn, device=dev) for _ in range(2)]
+    ref = [torch.empty(tokens * topk, ffn, device=dev, dtype=torch.float64) for _ in range(2)]
     for e in range(E):
         sel = expert == e
         for i in range(2):
-            ref[i][sel] = rows[sel] @ w[i][e].float().t()
+            ref[i][sel] = rows[sel] @ w[i][e].double().t()
     for _ in range(2):
-        for got, want in zip(op.forward_multiple_weights(x, w, splits, scatter), ref):
-            assert (got.float() - want).abs().max().item() <= 1e-2 * max(1.0, want.abs().max().item())
+        x_now = x.clone()                      # (rows are gathered anew: nothing of the first call may be left over)
+        op._sorted = None if op._sorted is None else op._sorted.fill_(float("nan"))
+        for got, want in zip(op.forward_multiple_weights(x_now, w, splits, scatter), ref):
+            # half a unit in the last place of bf16 is at most 2^-8 of the value; the fp32 sums err by far less
+            assert ((got.double() - want).abs() <= 1.01 * 2.0 ** -8 * want.abs() + 2e-6 * H ** 0.5 * want.abs().max()).all()
     op.check_status()
+    warps = 2 * torch.cuda.get_device_properties(dev).multi_processor_count
+    return min(max(tokens * topk // (16 * warps), 1), 8), _native.last_gemm()
+
+
+@pytest.mark.parametrize("tokens,E,topk,kind", [(3, 8, 2, "random"), (64, 64, 8, "random"), (64, 64, 1, "one"),
+                                                (300, 128, 2, "few"), (4801, 32, 4, "random"), (4801, 8, 4, "one")])
+def test_moe_layer0_gather_chunks(dev, tokens, E, topk, kind):
+    """Rows are gathered in chunks that may touch several experts (here one to four rows each), and an expert is
+    published when its last row is written: empty experts, one-row experts, all rows on one expert, twice on the same op."""
+    chunk, _ = _gather_case(dev, tokens, E, topk, kind, H=136, ffn=128)
+    assert chunk == (4 if tokens == 4801 else 1)
+
+
+@pytest.mark.parametrize("tokens,E,topk,kind,H,ffn,chunk,pair", [
+    (4801, 64, 8, "random", 136, 128, 8, 0),       # eight rows per chunk, runs of experts that start anywhere
+    (3601, 128, 8, "random", 136, 128, 6, 0),
+    (300, 64, 4, "random", 2056, 128, 1, 0),       # rows of 4112 bytes: a whole piece and 16 bytes
+    (1201, 512, 8, "random", 2056, 128, 2, 0),     # the same, chunks over several experts
+    (400, 8, 2, "random", 4104, 264, 1, 0),        # two pieces and 16 bytes
+    (200, 8, 2, "random", 5000, 128, 1, 0),        # 10000 bytes: two pieces and 1808 bytes
+    (8209, 8, 2, "random", 2056, 2048, 3, 1),      # CTA pairs: long rows, chunks over expert boundaries
+    (13001, 16, 4, "random", 264, 1536, 8, 1),
+    (6500, 4, 2, "one", 264, 2048, 2, 1)])
+def test_moe_layer0_gather_pieces(dev, tokens, E, topk, kind, H, ffn, chunk, pair):
+    """Rows longer than one 4096-byte piece, chunks of up to eight rows that end inside an expert, on single CTAs and
+    on CTA pairs."""
+    got, ran = _gather_case(dev, tokens, E, topk, kind, H, ffn)
+    assert got == chunk
+    assert (ran["kernel"], ran["cta_group"], ran["tile_m"]) == (("grouped", 2, 256) if pair else ("grouped", 1, 128))
 
 
 @pytest.mark.parametrize("n,E", [(1, 1), (31, 512), (511, 64), (513, 8), (4095, 512), (4096, 3), (4097, 64), (20000, 512),
