@@ -583,15 +583,8 @@ static int dense_impl(const fluxb_dense_args_t* a, const fluxb_a2a_args_t* x) {
 
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(a->stream);
   // CTAs that wait for one another (wave-synchronous starts) or for peers (every multi-rank mode) must
-  // all be resident: those launches are cooperative unless FLUXB_COOPERATIVE=0
-  // (a kernel profiler that replays launches could not replay a cooperative cluster launch here:
-  // under an injected profiler the attribute is left off unless FLUXB_COOPERATIVE=1 asks for it)
-  static const int coop_env = [] {
-    const char* e = getenv("FLUXB_COOPERATIVE");
-    if (e) return atoi(e);
-    return (getenv("CUDA_INJECTION64_PATH") || getenv("NV_COMPUTE_PROFILER_PERFWORKS_DIR")) ? 0 : 1;
-  }();
-  bool coop = coop_env != 0 && (multi || a2a);
+  // all be resident
+  bool coop = cooperative_launches() && (multi || a2a);
   {
     // wave-synchronous tile starts pay off when a wave's operands do not fit L2 together
     static const int wave_env = [] {
@@ -602,7 +595,7 @@ static int dense_impl(const fluxb_dense_args_t* a, const fluxb_a2a_args_t* x) {
     const int kblocks = (a->K + bk - 1) / bk;
     const bool want = wave_env >= 0 ? wave_env != 0 : kblocks >= 48;
     if (want && p.total_vtiles > 2 * (grid / cg)) p.wave_ctr = a->wave_ctr ? a->wave_ctr : wave_counter_for(stream);
-    if (p.wave_ctr != nullptr && coop_env != 0) coop = true;
+    if (p.wave_ctr != nullptr && cooperative_launches()) coop = true;
   }
   if (a->blockscale) {
     if (cg == 2) {

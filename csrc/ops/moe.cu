@@ -267,26 +267,34 @@ int launch_grouped(const GroupedParams& p, int grid, cudaStream_t stream) {
                                        Cfg::SMEM_BYTES));
     if (dev < 64) configured[dev] = true;
   }
-  if constexpr (Cfg::CG == 1) {
-    grouped_gemm_kernel<Cfg><<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(p);
-  } else {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid & ~1, 1, 1);
-    cfg.blockDim = dim3(Cfg::THREADS, 1, 1);
-    cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    FLUXB_CUDA_OK(cudaLaunchKernelEx(&cfg, grouped_gemm_kernel<Cfg>, p));
+  // CTAs that wait for rows other CTAs gather, for the whole grid (the fused combine), for one another wave by wave
+  // or for peers must all be resident
+  const bool coop = cooperative_launches() && (Cfg::PREGATHER || Cfg::SCATTER || p.wave_ctr != nullptr || p.do_allgather);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid / Cfg::CG * Cfg::CG, 1, 1);
+  cfg.blockDim = dim3(Cfg::THREADS, 1, 1);
+  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int na = 0;
+  if constexpr (Cfg::CG == 2) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = 2;
+    attr[na].val.clusterDim.y = 1;
+    attr[na].val.clusterDim.z = 1;
+    ++na;
   }
+  if (coop) {
+    attr[na].id = cudaLaunchAttributeCooperative;
+    attr[na].val.cooperative = 1;
+    ++na;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = na;
+  FLUXB_CUDA_OK(cudaLaunchKernelEx(&cfg, grouped_gemm_kernel<Cfg>, p));
   FLUXB_CUDA_OK(cudaGetLastError());
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  note_gemm({FLUXB_KERNEL_GROUPED, Cfg::BM, Cfg::BN, Cfg::CG, 1, 0});
+  note_gemm({FLUXB_KERNEL_GROUPED, Cfg::BM, Cfg::BN, Cfg::CG, 1, coop ? 1 : 0});
   return kOk;
 }
 
@@ -566,7 +574,16 @@ extern "C" int fluxb_moe_combine(const fluxb_moe_combine_args_t* a) {
     const int v = e ? atoi(e) : 4;
     return v >= 1 && v <= 4 ? v : 4;
   }();
-  moe_combine_kernel<<<sms * per_sm, 256, 0, reinterpret_cast<cudaStream_t>(a->stream)>>>(p);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(sms * per_sm, 1, 1);
+  cfg.blockDim = dim3(256, 1, 1);
+  cfg.stream = reinterpret_cast<cudaStream_t>(a->stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cooperative_launches() ? 1 : 0;
+  FLUXB_CUDA_OK(cudaLaunchKernelEx(&cfg, moe_combine_kernel, p));
   FLUXB_CUDA_OK(cudaGetLastError());
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return kOk;

@@ -87,6 +87,15 @@ int device_sm_count(int* out) {
   return kOk;
 }
 
+bool cooperative_launches() {
+  static const bool on = [] {
+    const char* e = getenv("FLUXB_COOPERATIVE");
+    if (e) return atoi(e) != 0;
+    return getenv("CUDA_INJECTION64_PATH") == nullptr && getenv("NV_COMPUTE_PROFILER_PERFWORKS_DIR") == nullptr;
+  }();
+  return on;
+}
+
 }  // namespace fluxb
 
 extern "C" int fluxb_last_gemm(fluxb_gemm_launch_t* out) {

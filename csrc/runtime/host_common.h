@@ -48,6 +48,11 @@ int encode_tmap(CUtensorMap* out, CUtensorMapDataType dt, int nd, const void* ba
                 const uint64_t* dims, const uint64_t* strides_bytes, const uint32_t* box, Swz swz);
 
 int device_sm_count(int* out);
+// Whether launches whose CTAs wait for one another, or for peers, carry the cooperative attribute: the grid then only
+// starts when all of its CTAs can be resident together, and fails at launch, instead of waiting inside the kernel, when
+// they never can. FLUXB_COOPERATIVE=0 turns it off. A kernel profiler that replays launches could not replay a
+// cooperative cluster launch here: under an injected profiler it is off unless FLUXB_COOPERATIVE=1 asks for it.
+bool cooperative_launches();
 // What fluxb_last_gemm answers on this thread from now on.
 void note_gemm(const fluxb_gemm_launch_t& launch);
 // A zeroed device word from a small per-device pool, for launches that keep their CTAs in step wave

@@ -254,3 +254,26 @@ def test_moe_layer0_one_op_unequal_buffers_and_types(dev):
             assert (out[:tokens * topk].float() - ref).abs().max().item() <= 1e-2 * ref.abs().max().item()
             assert out[tokens * topk:].isnan().all()
     op.check_status()
+
+
+@pytest.mark.parametrize("rows", [64, 4096])        # single CTAs; CTA pairs where the rule takes them
+def test_grouped_launches_whose_blocks_wait_for_one_another_are_cooperative(dev, rows):
+    """The gather and the fused combine need the whole grid resident; a plain grouped GEMM does not."""
+    import tempname_new_b200 as flux
+    from tempname_new_b200 import _native
+    E, H, ffn = 2, 128, 256
+    chosen = torch.randint(0, E, (rows, 1), device=dev, dtype=torch.int32)
+    splits, _, scatter, _, _ = flux.moe_index_build(chosen, E)
+    x, w1, w2 = (torch.randn(*s, device=dev).bfloat16() for s in ((rows, H), (E, ffn, H), (E, H, ffn)))
+    env = flux.DistEnvTPWithEP(dist.group.WORLD, 1, None, ep_size=1)
+    l0 = flux.GemmGroupedV3AGScatter(env, flux.MoeArguments(rows, H, ffn, E, 1, torch.bfloat16))
+    h = l0.forward(x, w1, splits, scatter)
+    ran = [_native.last_gemm()]
+    flux.GemmGroupedV3GatherRS(E, rows, H, 1, 0, 1, 1, 1, tp_group=dist.group.WORLD).forward_gather_rs(
+        h, w2, splits, scatter.reshape(-1))
+    ran.append(_native.last_gemm())
+    flux.GemmGroupedV3(w1, E).forward(x, splits)
+    ran.append(_native.last_gemm())
+    assert [r["kernel"] for r in ran] == ["grouped"] * 3
+    on = 0 if os.environ.get("FLUXB_COOPERATIVE") == "0" else 1
+    assert [r["cooperative"] for r in ran] == [on, on, 0]
