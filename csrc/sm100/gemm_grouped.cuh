@@ -235,9 +235,10 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
         if (lane == 0) flag_wait_ge(wc, p.wave_ctr, need, kSiteStartBarrier);
       }
       __syncwarp();
-      // the whole warp walks the k-blocks, one elected lane issues
+      // the whole warp walks the k-blocks, one elected lane issues (a wait that gave up: nothing more is issued, so that
+      // what is in flight at the teardown is bounded by the depth of the pipeline)
       for (int kb = 0; kb < k_blocks; ++kb) {
-        mbar_wait_warp(wc, empty_bar(stage), phase ^ 1u, kSiteSmemEmpty);
+        if (!mbar_wait_warp(wc, empty_bar(stage), phase ^ 1u, kSiteSmemEmpty)) break;
         const uint32_t sa = smem_base + stage * Cfg::STAGE_BYTES;
         if (ptx::elect_one()) {
           if constexpr (Cfg::GATHER) {
@@ -281,11 +282,11 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
       for (int t = tile_first; t < total_tiles; t += tile_stride, ++it) {
         if (__any_sync(0xffffffffu, *abort_word)) break;   // a wait gave up: issue nothing more
         const int acc = it & 1;
-        mbar_wait_warp(wc, tempty_bar(acc), (((it >> 1) & 1) ^ 1u), kSiteTmemEmpty);
+        if (!mbar_wait_warp(wc, tempty_bar(acc), (((it >> 1) & 1) ^ 1u), kSiteTmemEmpty)) break;
         ptx::tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < k_blocks; ++kb) {
-          mbar_wait_warp(wc, full_bar(stage), phase, kSiteSmemFull);
+          if (!mbar_wait_warp(wc, full_bar(stage), phase, kSiteSmemFull)) break;
           // gathered A rows were written through the generic proxy (cp.async)
           if constexpr (Cfg::GATHER) ptx::fence_proxy_async_smem();
           ptx::tc_fence_after();
