@@ -326,7 +326,8 @@ class GemmGroupedV3GatherRS(FusedOpBase):
         # over ranks: partial sums per source, [W][tokens / W][H]
         self.fused = tp_world_size == 1
         slots = max(world_size, topk) if self.fused else world_size
-        self.stage = SymmBuffer(slots * self.max_tpr * n_dim * _ELEM[dtype], self.pg) \
+        # (8-bit inputs give 16-bit rows)
+        self.stage = SymmBuffer(slots * self.max_tpr * n_dim * max(2, _ELEM[dtype]), self.pg) \
             if (self.world > 1 or self.fused) else None
         self._scratch = None
         self._row_entry = None

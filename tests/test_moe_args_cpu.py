@@ -61,6 +61,16 @@ def test_weight_groups_share_one_sorted_rows_buffer(layer0):
     assert [(a.gathered, a.a, a.reuse_schedule) for a in rest] == [(0, first.a_sorted, 1)] * 2
 
 
+def test_combine_slots_hold_sixteen_bit_rows(layer0):
+    """An op built for 8-bit inputs receives 16-bit rows in its staging slots, like any other."""
+    import tempname_new_b200 as flux
+    tokens, H, E, topk = 64, 256, 4, 2
+    layer0(tokens, H, 128, E, topk, torch.bfloat16)
+    for dtype in (torch.bfloat16, torch.float8_e4m3fn, torch.float8_e5m2):
+        op = flux.GemmGroupedV3GatherRS(E, tokens * topk, H, topk, 0, 1, 1, 1, tp_group=dist.group.WORLD, dtype=dtype)
+        assert op.stage.nbytes >= tokens * topk * H * 2
+
+
 def _landing_buffer(rank, world):
     import tempname_new_b200 as flux
     tokens, H, ffn, E, topk = 128, 64, 128, 4, 2          # (of all ranks)
