@@ -57,6 +57,9 @@ class AGKernel(FusedOpBase):
             if input_scale is not None and input_scale.dim() == 3:
                 raise NotImplementedError("block-scaled AG+GEMM has no CPU path")
             return self._forward_cpu(input, w, bias, output, input_scale, weight_scale, gathered_input, act)
+        if self.land is not None and M * K * input.element_size() > self.land.nbytes:
+            raise ValueError(f"AGKernel was built for {self.input_dtype} inputs; {M} rows of {K} {input.dtype} values "
+                             "do not fit its landing buffer")
         a = input if input.is_contiguous() else input.contiguous()
         out = output if output is not None else torch.empty((M, N), dtype=self.output_dtype, device=input.device)
         keep: list = []

@@ -29,6 +29,27 @@ def test_tile_choices_of_several_ranks(ranks):
     assert table.lookup(8192, 12288, 49152, 2, ranks)["group_m"] == 4
 
 
+def _landing_buffer(rank, world):
+    import tempname_new_b200 as flux
+    rec = record_launches()
+    M, N, K = 512, 256, 256
+    op = flux.AGKernel(dist.group.WORLD, 1, M, N, K, torch.float8_e4m3fn)
+    op.status = torch.zeros(4, dtype=torch.int32)
+    for dtype, rows, fits in ((torch.float8_e4m3fn, M, True), (torch.bfloat16, M, False), (torch.bfloat16, M // 2, True)):
+        x, w = (as_cuda(torch.zeros(r, K).to(dtype)) for r in (rows // world, N))
+        before = len(rec.calls)
+        if fits:
+            op.forward(x, w)
+        else:
+            with pytest.raises(ValueError, match="landing buffer"):
+                op.forward(x, w)
+        assert len(rec.calls) == before + fits
+
+
+def test_all_gather_push_stays_inside_the_landing_buffers():
+    run_gloo(_landing_buffer, 2)
+
+
 def _rank_counts(rank, world):
     import tempname_new_b200 as flux
     rec = record_launches()
