@@ -432,12 +432,14 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) grouped_gemm_kernel(const __g
             if (!p.by_src) {
               // No source ranks: the rows of all experts are one run of the sorted order, dealt out in chunks of a
               // few rows. Each chunk adds its rows to its expert's counter once they are written, and the last one
-              // publishes the expert. At most eight rows: 65536 rows of 8 KB under a GEMM of 660 us then cost 110 us,
-              // with two 220, with four 115, with sixteen 115. Four slots of 4 KB, three loads in flight; a warp pays
-              // one drain and one atomic per chunk, whatever the number of experts (a drain, a fence and an atomic per warp
-              // and expert, with one load in flight, cost 260 us for 64 experts of 8 rows).
+              // publishes the expert. Four slots of 4 KB, three loads in flight; a warp pays one drain and one atomic per
+              // chunk, about 3 us, whatever the number of experts (a drain, a fence and an atomic per warp and expert, with
+              // one load in flight, cost 260 us for 64 experts of 8 rows). So two chunks per warp, and at most eight rows:
+              // 65536 rows of 8 KB under a GEMM of 660 us then cost 110 us, with two 220, with four 115, with sixteen 115.
+              // Whole layer 0, us, 16 / 4 / 2 / 1 chunks per warp: 6144 rows x 2048 bf16, 8 experts 105 / 65 / 59 / 60;
+              // 8192 x 4096 e4m3, 64 experts 207 / 113 / 112 / 112; 4096 x 4096 bf16, 128 experts 318 / 320 / 323 / 326.
               const int total = p.hdr[1];
-              const int cr = min(max(total / static_cast<int>(ncw * 16u), 1), 8);
+              const int cr = min(max(total / static_cast<int>(ncw * 2u), 1), 8);
               for (int r0 = static_cast<int>(cw) * cr; r0 < total; r0 += static_cast<int>(ncw) * cr) {
                 const int first = row_base + r0, last = row_base + min(r0 + cr, total);
                 int lo = 0, hi = p.E_local;                 // expert of the first row

@@ -115,7 +115,8 @@ def test_moe_layer1_fused_fp8(dev):
 
 
 def _gather_case(dev, tokens, E, topk, kind, H, ffn):
-    """Layer 0 with two weight groups, twice on one op, against fp32; returns (rows per chunk, the first GEMM's launch)."""
+    """Layer 0 with two weight groups, twice on one op, against 64 bits; returns the rows per chunk of the gather and what
+    the launch with the gather was."""
     import tempname_new_b200 as flux
     from tempname_new_b200 import _native
     g = torch.Generator(device=dev).manual_seed(tokens + E)
@@ -147,30 +148,35 @@ def _gather_case(dev, tokens, E, topk, kind, H, ffn):
         for got, want in zip(op.forward_multiple_weights(x_now, w, splits, scatter), ref):
             # half a unit in the last place of bf16 is at most 2^-8 of the value; the fp32 sums err by far less
             assert ((got.double() - want).abs() <= 1.01 * 2.0 ** -8 * want.abs() + 2e-6 * H ** 0.5 * want.abs().max()).all()
+    op.forward(x, w[0], splits, scatter)
+    ran = _native.last_gemm()
     op.check_status()
     warps = 2 * torch.cuda.get_device_properties(dev).multi_processor_count
-    return min(max(tokens * topk // (16 * warps), 1), 8), _native.last_gemm()
+    return min(max(tokens * topk // (2 * warps), 1), 8), ran
 
 
 @pytest.mark.parametrize("tokens,E,topk,kind", [(3, 8, 2, "random"), (64, 64, 8, "random"), (64, 64, 1, "one"),
                                                 (300, 128, 2, "few"), (4801, 32, 4, "random"), (4801, 8, 4, "one")])
 def test_moe_layer0_gather_chunks(dev, tokens, E, topk, kind):
-    """Rows are gathered in chunks that may touch several experts (here one to four rows each), and an expert is
+    """Rows are gathered in chunks that may touch several experts (here of one or eight rows), and an expert is
     published when its last row is written: empty experts, one-row experts, all rows on one expert, twice on the same op."""
     chunk, _ = _gather_case(dev, tokens, E, topk, kind, H=136, ffn=128)
-    assert chunk == (4 if tokens == 4801 else 1)
+    assert chunk == (8 if tokens == 4801 else 1)
 
 
 @pytest.mark.parametrize("tokens,E,topk,kind,H,ffn,chunk,pair", [
     (4801, 64, 8, "random", 136, 128, 8, 0),       # eight rows per chunk, runs of experts that start anywhere
-    (3601, 128, 8, "random", 136, 128, 6, 0),
-    (300, 64, 4, "random", 2056, 128, 1, 0),       # rows of 4112 bytes: a whole piece and 16 bytes
-    (1201, 512, 8, "random", 2056, 128, 2, 0),     # the same, chunks over several experts
+    (1801, 128, 2, "random", 136, 128, 6, 0),
+    (140, 64, 4, "random", 2056, 128, 1, 0),       # rows of 4112 bytes: a whole piece and 16 bytes
+    (300, 64, 4, "random", 2056, 128, 2, 0),       # the same, chunks over several experts
+    (1500, 512, 2, "random", 2056, 128, 5, 0),
+    (1201, 512, 8, "random", 2056, 128, 8, 0),
     (400, 8, 2, "random", 4104, 264, 1, 0),        # two pieces and 16 bytes
-    (200, 8, 2, "random", 5000, 128, 1, 0),        # 10000 bytes: two pieces and 1808 bytes
-    (8209, 8, 2, "random", 2056, 2048, 3, 1),      # CTA pairs: long rows, chunks over expert boundaries
+    (600, 8, 3, "random", 5000, 128, 3, 0),        # 10000 bytes: two pieces and 1808 bytes
+    (1700, 2, 1, "random", 2056, 2048, 2, 1),      # CTA pairs: long rows, chunks over expert boundaries
+    (8209, 8, 2, "random", 2056, 2048, 8, 1),
     (13001, 16, 4, "random", 264, 1536, 8, 1),
-    (6500, 4, 2, "one", 264, 2048, 2, 1)])
+    (6500, 4, 2, "one", 264, 2048, 8, 1)])
 def test_moe_layer0_gather_pieces(dev, tokens, E, topk, kind, H, ffn, chunk, pair):
     """Rows longer than one 4096-byte piece, chunks of up to eight rows that end inside an expert, on single CTAs and
     on CTA pairs."""
@@ -200,6 +206,12 @@ def test_grouped_pairs(dev, dtype, splits, N, K):
     """Tiles shared by two CTAs (768 rows per expert on average and more): one-row and empty experts, tiles whose second
     half has no rows, column and K remainders; contiguous rows, gathered rows and the fused combine."""
     import tempname_new_b200 as flux
+    from tempname_new_b200 import _native
+
+    def took_pairs():
+        ran = _native.last_gemm()
+        return (ran["kernel"], ran["cta_group"], ran["tile_m"], ran["tile_n"]) == ("grouped", 2, 256, 256)
+
     K = K if dtype.itemsize == 2 else K * 2
     E, rows = len(splits), sum(splits)
     assert rows >= 768 * E
@@ -210,6 +222,7 @@ def test_grouped_pairs(dev, dtype, splits, N, K):
     ref = torch.cat([x[expert == e].float() @ w[e].float().t() for e in range(E)])
     tol = 1e-2 * ref.abs().max().item()
     out = flux.GemmGroupedV3(w, E).forward(x, torch.tensor(splits))
+    assert took_pairs()
     assert (out.float() - ref).abs().max().item() <= tol
     # the same rows gathered from shuffled tokens (top-1), and back through the combine
     perm = torch.randperm(rows, device=dev, generator=g)          # token of every sorted row
@@ -223,14 +236,20 @@ def test_grouped_pairs(dev, dtype, splits, N, K):
     op = flux.GemmGroupedV3AGScatter(env, flux.MoeArguments(rows, K, N, E, 1, dtype, o16))
     for _ in range(2):
         got = op.forward(tokens, w, sp, scatter.view(rows, 1))
+        assert took_pairs()
         assert (got.float() - ref).abs().max().item() <= tol
     op.check_status()
     gate = torch.rand(rows, device=dev, generator=g)
     rs = flux.GemmGroupedV3GatherRS(E, rows, N, 1, 0, 1, 1, 1, tp_group=dist.group.WORLD, dtype=o16)
     for _ in range(2):
         y = rs.forward_gather_rs(x, w, sp, scatter, output_vec_scale=gate)
+        assert took_pairs()
         assert (y[perm].float() - ref * gate[:, None]).abs().max().item() <= tol
     rs.check_status()
+    # one row less than 768 per expert: single CTAs
+    short = torch.tensor([767 * E + E - 1] + [0] * (E - 1))
+    flux.GemmGroupedV3(w, E).forward(x.new_zeros(768 * E - 1, K), short)
+    assert not took_pairs()
 
 
 def test_moe_layer0_one_op_unequal_buffers_and_types(dev):
