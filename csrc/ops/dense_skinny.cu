@@ -109,7 +109,9 @@ using namespace fluxb;
 //  * more rows, as long as the 64-column tiles fit the chip twice: 128 x 4096 x 4096 32 -> 16, 1024 x 2048 x 8192
 //    63 -> 38, 300 x 1024 x 8192 58 -> 20. (1000 x 3000 x 5000, 376 tiles: 54 on the persistent kernel, 66 here.)
 //    64 columns balance better, but once they fill the chip without a split, two K halves of 128 columns read
-//    less: 2048 x 1024 x 4096 27 -> 23, from 32 k-blocks on (256 x 8192 x 1024: 12.0 on 64, 13.9 on 128).
+//    less: 2048 x 1024 x 4096 27 -> 23, from 49 k-blocks on. 64 / 128 columns, geometric means over 65 - 2048 rows in
+//    all types: 32 k-blocks 0.91, 40 0.95, 48 0.98, 64 1.04, 96 1.08 (128 x 16384 x 4096 int8 17.8 / 20.8, where the
+//    persistent kernel takes 17.8).
 //  * block scales: 64 columns (the fp32 row of a thread stays in registers): 48 x 3584 x 8192 46 -> 15,
 //    1024 x 2048 x 8192 46 -> 37; 64 x 24576 x 4096, 384 tiles: 31 on the persistent kernel, 37 here.
 // Splits: to one CTA per SM wherever four k-blocks are left each, on to two per SM only with 16 left each (8192
@@ -123,7 +125,7 @@ extern "C" int fluxb_skinny_shape(int32_t M, int32_t N, int32_t k_blocks, int32_
   const int64_t t64 = mt * ((N + 63) / 64), t128 = mt * ((N + 127) / 128);
   if ((blockscale != 0 || M > 64) && t64 > 2 * sms) return kOk;
   int w = (blockscale != 0 || M > 64) ? 64 : 128;
-  if (w == 64 && blockscale == 0 && t64 > sms && k_blocks >= 32) w = 128;
+  if (w == 64 && blockscale == 0 && t64 > sms && k_blocks > 48) w = 128;
   const int64_t t = w == 64 ? t64 : t128;
   int s = 1;
   while (s < 4 && 2 * s * t <= 2 * sms && k_blocks >= (2 * s * t <= sms ? 8 : 32) * s) s *= 2;

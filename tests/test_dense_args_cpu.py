@@ -125,3 +125,16 @@ def test_row_parallel_bias_that_broadcasts(row_parallel, shape):
     assert rec.calls[-1].bias is None and y.shape == (32, 128)
     (g,) = torch.autograd.grad(y, [lin.bias], torch.ones(32, 128).bfloat16())
     assert g.shape == shape and torch.equal(g, torch.full(shape, 32 * 128 / max(1, lin.bias.numel())).bfloat16())
+
+
+@pytest.mark.parametrize("M,N,k_blocks,rule", [
+    (128, 16384, 32, (64, 256, 1)), (2048, 1024, 48, (64, 256, 1)),       # 64 columns fill the chip without a split
+    (128, 16384, 49, (128, 128, 2)), (2048, 1024, 64, (128, 128, 2)),     # a long K: two halves of 128 columns
+    (128, 4096, 48, (64, 64, 2)), (128, 4096, 64, (64, 64, 4)), (64, 16384, 32, (128, 128, 2)), (128, 32768, 32, (0, 0, 0))])
+def test_split_k_tiles(M, N, k_blocks, rule):
+    """(columns, tiles, CTAs per tile) on both sides of the lines, for 148 SMs."""
+    import ctypes
+    from tempname_new_b200 import _native
+    v = [ctypes.c_int32() for _ in range(3)]
+    _native.check(_native.lib().fluxb_skinny_shape(M, N, k_blocks, 0, 148, *map(ctypes.byref, v)), "rule")
+    assert tuple(x.value for x in v) == rule
