@@ -265,12 +265,15 @@ static int dense_impl(const fluxb_dense_args_t* a, const fluxb_a2a_args_t* x) {
                     "tile_m must be 128 * cta_group, or 512 for CTA pairs on 256-column tiles");
       mt = (want == 512 && can) ? 2 : 1;
     } else if (can && (seg_rows % 512 == 0 || seg_rows >= 4096) &&
-               (multi || static_cast<int64_t>(a->K) * elt >= 80 * 128)) {
+               (multi || static_cast<int64_t>(a->K) * elt >= 80 * 128 ||
+                (static_cast<int64_t>(a->K) * elt <= 4 * 128 && static_cast<int64_t>(a->M) * a->N >= int64_t{1} << 26))) {
       // Two MMAs per B tile move a quarter less into shared memory, but the epilogue overlaps only the first stages of
       // the next tile: 512 rows from 80 k-blocks (of 128 bytes) on. 512 / 256 rows, us under the power cap:
       // 16384 x 3584 x 8192 bf16 746 / 781, 8192 x 12288 x 6144 935 / 964, 4096 x 16384 x 4096 424 / 416, 2048 x 2048 x
-      // 2048 22.5 / 20.5, 2048 x 12288 x 4096 fp8 97 / 90, 8192 x 8192 x 8192 fp8 432 / 416. (Several ranks: as
-      // measured there, wherever the rows allow it.)
+      // 2048 22.5 / 20.5, 2048 x 12288 x 4096 fp8 97 / 90, 8192 x 8192 x 8192 fp8 432 / 416. The other way round where
+      // there is next to no main loop and the output is all the traffic: up to four k-blocks under 2^26 outputs and more
+      // (16384 x 8192 x 64 bf16 108 / 117, 4096 x 16384 x 256 fp8 59 / 62; half the outputs 32 / 32, eight k-blocks
+      // 84 / 74). (Several ranks: as measured there, wherever the rows allow it.)
       mt = 2;
     }
   }

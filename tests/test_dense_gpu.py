@@ -429,3 +429,20 @@ def test_row_parallel_bias_one_rank(dev):
         wide = RowParallelLinear(256, 520, device=dev)
         wide.bias = torch.nn.Parameter(torch.zeros(520, device=dev))     # an fp32 bias still promotes the sum
         assert wide(x).dtype == torch.float32
+
+
+@pytest.mark.parametrize("M,N,K,dtype,tile_m", [
+    (4096, 16384, 64, torch.bfloat16, 512), (4096, 16384, 512, torch.float8_e4m3fn, 512),    # all output: 512 rows
+    (4096, 8192, 64, torch.bfloat16, 256), (4096, 16384, 320, torch.bfloat16, 256),          # half of it; five k-blocks
+    (2048, 2048, 5120, torch.bfloat16, 512), (2048, 2048, 5056, torch.bfloat16, 256)])       # 80 and 79 k-blocks
+def test_tile_rows_by_default(dev, M, N, K, dtype, tile_m):
+    from tempname_new_b200 import _native
+    from tempname_new_b200.ops import _dense
+    a, b = (torch.randn(*s, device=dev).to(dtype) for s in ((M, K), (N, K)))
+    out = torch.full((M, N), float("nan"), device=dev, dtype=torch.bfloat16)
+    _dense.plain_gemm(a, b, out)
+    ran = _native.last_gemm()
+    assert (ran["kernel"], ran["tile_m"], ran["tile_n"], ran["cta_group"]) == ("persistent", tile_m, 256, 2)
+    for rows in range(0, M, 1024):
+        ref = a[rows:rows + 1024].float() @ b.float().t()
+        assert (out[rows:rows + 1024].float() - ref).abs().max().item() <= _tol(ref)
