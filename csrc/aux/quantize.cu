@@ -44,8 +44,8 @@ __device__ __forceinline__ float compute_scale(float amax, float eps, float fp8_
 // so that a half-warp reads one 256-byte row segment per instruction; row maxima are reduced by
 // shuffles, column maxima through a small shared array; q leaves as 8-byte stores (128 contiguous
 // bytes per row), q^T is transposed through a swizzled shared tile (a thread's 4 rows of one column
-// are one 32-bit word) and leaves as 16-byte stores. About five instructions per element instead
-// of forty: the kernel is memory bound.
+// are one 32-bit word) and leaves as 16-byte stores. 16384 x 8192 bf16, 1x128: 90 us with the transpose, 68 without, both
+// 0.92 of the copy rate, so memory bounds it; 108 and 82 with the row maxima as a butterfly, bound by instruction issue.
 // ---------------------------------------------------------------------------------------------
 template <bool BF16>
 __device__ __forceinline__ uint32_t habs2_bits(uint32_t v) {
@@ -247,14 +247,15 @@ __global__ void __launch_bounds__(kThreads) quant_tile_kernel(
 // Any other shape, pitch or alignment, and fp32 inputs: the same register tile with guards. What is outside
 // the matrix reads as zero, so the scales of the rows and columns that pad the last blocks are those of
 // zeros. Maxima ignore NaN. An 8-column chunk is read with 16-byte loads where the row pitch and the base
-// allow them and element by element elsewhere; q leaves as 8-byte stores where K allows them. Rows whose
-// start may be on any byte (q with K % 8 != 0, q^T with M % 16 != 0) are written from the shared tile one warp
-// per row, in aligned 32-bit words put together from two neighbouring words of the tile: 128 contiguous bytes
-// per instruction whatever the alignment, and single bytes at the two ends only.
+// allow them, elsewhere with the widest loads its row allows; q leaves as 8-byte stores where K allows them. Rows whose
+// start may be on any byte (q with K % 8 != 0, q^T with M % 8 != 0) are written from the shared tile, half a warp per
+// row, in aligned 8-byte stores and one byte per lane for the two ends.
 // Bound by instruction issue, not by memory: 5000 x 8192 bf16, 1x128 with the transpose, takes 37 us (4.4 TB/s); 44 us
 // with a butterfly and sixteen divisions per row, 70 us with one thread per column for the column maxima and byte
 // stores of q^T, 73 us with fp32 maxima and every row of q^T through the word writer (2.7 instructions per cycle and SM
-// in all of these).
+// in all of these). Rows that start on any element, 5001 x 8191 bf16: 63 us with the transpose, 45 without (126 and 87 with
+// element loads and a warp per row of 4-byte stores; 87 and 66 with a shared tile read and written element by element);
+// few rows, 33 x 4096, 128 x 128 with the transpose: 4.2 us (7.2; 4.6).
 // ---------------------------------------------------------------------------------------------
 template <typename T>
 struct Chunk8 {      // 8 consecutive elements of a row, as they are in memory
@@ -274,6 +275,24 @@ struct Chunk8 {      // 8 consecutive elements of a row, as they are in memory
   __device__ __forceinline__ void load_vec(const T* p) {
     const uint4 v = *reinterpret_cast<const uint4*>(p);
     w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
+  }
+  __device__ __forceinline__ void load_any(const T* p) {      // 8 elements on any element boundary
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    if ((a & 7) == 0) {
+      const uint2 lo = reinterpret_cast<const uint2*>(p)[0], hi = reinterpret_cast<const uint2*>(p)[1];
+      w[0] = lo.x, w[1] = lo.y, w[2] = hi.x, w[3] = hi.y;
+    } else if ((a & 3) == 0) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[j] = reinterpret_cast<const uint32_t*>(p)[j];
+    } else {
+      const uint16_t* h = reinterpret_cast<const uint16_t*>(p);
+      const uint32_t* m = reinterpret_cast<const uint32_t*>(h + 1);
+      const uint32_t m0 = m[0], m1 = m[1], m2 = m[2];
+      w[0] = h[0] | (m0 << 16);
+      w[1] = __funnelshift_r(m0, m1, 16);
+      w[2] = __funnelshift_r(m1, m2, 16);
+      w[3] = (m2 >> 16) | (static_cast<uint32_t>(h[7]) << 16);
+    }
   }
   __device__ __forceinline__ void load_some(const T* p, int n) {
     zero();
@@ -304,6 +323,18 @@ struct Chunk8<float> {
     w[0] = a.x, w[1] = a.y, w[2] = a.z, w[3] = a.w;
     w[4] = b.x, w[5] = b.y, w[6] = b.z, w[7] = b.w;
   }
+  __device__ __forceinline__ void load_any(const float* p) {
+    if ((reinterpret_cast<uintptr_t>(p) & 7) == 0) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 v = reinterpret_cast<const float2*>(p)[j];
+        w[2 * j] = v.x, w[2 * j + 1] = v.y;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) w[j] = p[j];
+    }
+  }
   __device__ __forceinline__ void load_some(const float* p, int n) {
     zero();
 #pragma unroll
@@ -313,25 +344,22 @@ struct Chunk8<float> {
   __device__ __forceinline__ float get(int j) const { return w[j]; }
 };
 
-// A row of a 128 x 128-byte shared tile (word i at i ^ swz) -> n bytes at dst, any alignment; one warp. Lane i
-// writes the aligned word that holds byte 4 * i - a of the row; the bytes before the first and after the last whole
-// word are single stores.
-__device__ __forceinline__ void store_tile_row(const uint32_t* tile_row, int swz, uint8_t* dst, int n, int lane) {
-  const int a = static_cast<int>(reinterpret_cast<uintptr_t>(dst) & 3);
-  const int b0 = 4 * lane - a;
-  const uint32_t hi = tile_row[lane ^ swz];
-  const uint32_t lo = __shfl_up_sync(0xffffffffu, hi, 1);      // (lane 0: its own word, only used below byte 0)
-  const uint32_t word = __funnelshift_l(lo, hi, 8 * a);
-  if (b0 >= 0 && b0 + 4 <= n) {
-    *reinterpret_cast<uint32_t*>(dst + b0) = word;
-  } else {
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (b0 + j >= 0 && b0 + j < n) dst[b0 + j] = static_cast<uint8_t>(word >> (8 * j));
+// A row of a 128 x 128-byte shared tile (word i at i ^ swz) -> n bytes at dst, any alignment; half a warp, l = 0 .. 15.
+// What lies between the first and the last 8-byte boundary leaves as aligned 8-byte stores, each put together from three
+// words of the tile; the at most 14 bytes around it as one byte per lane.
+__device__ __forceinline__ void store_tile_row(const uint32_t* tile_row, int swz, uint8_t* dst, int n, int l) {
+  const int head = min(n, static_cast<int>((0 - reinterpret_cast<uintptr_t>(dst)) & 7));
+  const int body = (n - head) >> 3, tail = (n - head) & 7;
+  if (l < body) {
+    const int o = head + 8 * l, k = o >> 2, s = 8 * (o & 3);
+    // (o + 7 <= 127: word k + 2 is beyond the row only where s is 0 and nothing of it is used)
+    const uint32_t w0 = tile_row[k ^ swz], w1 = tile_row[(k + 1) ^ swz], w2 = tile_row[((k + 2) & 31) ^ swz];
+    *reinterpret_cast<uint2*>(dst + o) = make_uint2(__funnelshift_r(w0, w1, s), __funnelshift_r(w1, w2, s));
   }
-  if (lane == 31)      // the last a bytes of a full row
-    for (int j = 4 - a; j < 4; ++j)
-      if (124 + j < n) dst[124 + j] = static_cast<uint8_t>(hi >> (8 * j));
+  if (l < head + tail) {
+    const int b = l < head ? l : n - head - tail + l;
+    dst[b] = static_cast<uint8_t>(tile_row[(b >> 2) ^ swz] >> (8 * (b & 3)));
+  }
 }
 
 template <typename T, bool SQUARE>
@@ -357,24 +385,27 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) quant_ragged
   const int chunk = lane & 15;
   const bool e5 = e5m2 != 0;
   const int ncol = min(8, cols - chunk * 8);              // columns of this thread's chunk inside the matrix
-  const bool vec_x = ncol == 8 && ldx % (16 / static_cast<int>(sizeof(T))) == 0 &&
-                     (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  const bool vec_x = ldx % (16 / static_cast<int>(sizeof(T))) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
   const bool vec_q = (K & 7) == 0 && (reinterpret_cast<uintptr_t>(q) & 7) == 0;
   const bool vec_qt = (M & 15) == 0 && (reinterpret_cast<uintptr_t>(qt) & 15) == 0 && rows == kTile;
   const bool vec8_qt = (M & 7) == 0 && (reinterpret_cast<uintptr_t>(qt) & 7) == 0;
 
   // ---- load: pass `it`, row group g = it * 16 + warp * 2 + lane / 16, rows 4g .. 4g + 3
   Chunk8<T> v[2][4];
+  auto load = [&](auto&& whole) {
 #pragma unroll
-  for (int it = 0; it < 2; ++it)
+    for (int it = 0; it < 2; ++it)
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int row = 4 * (it * 16 + warp * 2 + (lane >> 4)) + r;
-      const T* src = x + static_cast<int64_t>(row0 + row) * ldx + col0 + chunk * 8;
-      if (row < rows && vec_x) v[it][r].load_vec(src);
-      else if (row < rows) v[it][r].load_some(src, ncol);
-      else v[it][r].zero();
-    }
+      for (int r = 0; r < 4; ++r) {
+        const int row = 4 * (it * 16 + warp * 2 + (lane >> 4)) + r;
+        const T* src = x + static_cast<int64_t>(row0 + row) * ldx + col0 + chunk * 8;
+        if (row < rows && ncol == 8) whole(v[it][r], src);
+        else if (row < rows) v[it][r].load_some(src, ncol);
+        else v[it][r].zero();
+      }
+  };
+  if (vec_x) load([](Chunk8<T>& c, const T* p) { c.load_vec(p); });
+  else load([](Chunk8<T>& c, const T* p) { c.load_any(p); });
   // ---- maxima
   using C = Chunk8<T>;
   constexpr int NW = C::NW;
@@ -449,8 +480,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) quant_ragged
   }
   if (!vec_q) {
     __syncthreads();
-    for (int r = warp; r < rows; r += kThreads / 32)
-      store_tile_row(&tile[r * 32], 0, q + static_cast<int64_t>(row0 + r) * K + col0, cols, lane);
+    for (int r = tid >> 4; r < rows; r += kThreads / 16)
+      store_tile_row(&tile[r * 32], 0, q + static_cast<int64_t>(row0 + r) * K + col0, cols, lane & 15);
   }
   if (qt == nullptr) return;
   // ---- q^T (the barrier also ends the reading of a staged q)
@@ -500,8 +531,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) quant_ragged
             *reinterpret_cast<const uint2*>(&tile[c * 32 + ((part * 2) ^ (((c >> 3) * 4) & 31))]);
     }
   } else {
-    for (int c = warp; c < cols; c += kThreads / 32)
-      store_tile_row(&tile[c * 32], ((c >> 3) * 4) & 31, qt + static_cast<int64_t>(col0 + c) * M + row0, rows, lane);
+    for (int c = tid >> 4; c < cols; c += kThreads / 16)
+      store_tile_row(&tile[c * 32], ((c >> 3) * 4) & 31, qt + static_cast<int64_t>(col0 + c) * M + row0, rows, lane & 15);
   }
 }
 
