@@ -230,9 +230,9 @@ static int dense_impl(const fluxb_dense_args_t* a, const fluxb_a2a_args_t* x) {
     // (one rank: the last row block may be partial - its scales exist, its rows are clipped)
     FLUXB_REQUIRE(!multi || (a->M / a->world) % 128 == 0,
                   "block-scaled fused ops need rows per rank in multiples of 128");
-    // Single CTAs on 128 x 128 tiles. CTA pairs on 256 x 128 tiles (half of B per CTA) exist and are
-    // chosen by cta_group = 2, but measured slower (977 against 1128 TFLOP/s at 16384 x 3584 x 8192): the
-    // k-block hand-over then waits for the slowest of sixteen promotion warps on two SMs.
+    // Single CTAs. CTA pairs on 256 x 128 tiles (half of B per CTA) exist and are chosen by cta_group = 2, but
+    // measured slower than single CTAs on 128 x 128 (977 against 1128 TFLOP/s at 16384 x 3584 x 8192, with one-lane
+    // issue loops): the k-block hand-over then waits for the slowest of sixteen promotion warps on two SMs.
     cg = (a->cta_group == 2 && a->tile_n != 256 && a->M / (multi ? a->world : 1) >= 256) ? 2 : 1;
     // 128 x 256 tiles wherever N allows (tile_n = 128 pins the narrow ones): 1330 - 1350 against 1010 - 1060 TFLOP/s
     // when both were bound by their one-lane issue loops; 2200 since those run on whole warps.

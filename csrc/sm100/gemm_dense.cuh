@@ -177,8 +177,9 @@ struct DenseCfg {
   static constexpr int COMM_BYTES = COMM_;
   static constexpr bool BS = BS_ != kBsNone;
   static constexpr int BS_FORM = BS_;
-  // The multi-rank code is left out: the promotion loop is short of registers, and what else the kernel
-  // holds decides where the compiler puts its spills (28 - 32 bytes, none in the loop; 168 with it).
+  // The multi-rank code is left out: the promotion loop is short of registers, and the compiler spills for what
+  // else the kernel holds. Bytes per thread stored / loaded, as ptxas reports them for 128 x 256 tiles: none with one
+  // weight scale per block, 16 / 88 with one per column, 132 / 192 in the general form.
   static constexpr bool PLAIN_ONLY = BS_ == kBsSquare || BS_ == kBsColumn;
   static constexpr int REGS_LEAD = BN_ == 256 ? 40 : 88;       // after setmaxnreg
   static constexpr int REGS_PROMOTE = BN_ == 256 ? 232 : 208;
@@ -216,8 +217,6 @@ struct DenseCfg {
   static_assert(SMEM_BYTES <= 232448, "over the 227 KB shared memory limit");
   static constexpr int TMEM_COLS = 512;
   static_assert(ACC_BUFS * BN <= TMEM_COLS, "accumulators must fit TMEM");
-  // column pieces of a split tile are BN >> shift wide; the epilogue moves 64 columns at a time
-  static constexpr int MAX_SPLIT_SHIFT = BN_ != 256 ? 0 : (!BS ? 2 : (BS_ == kBsSquare ? 1 : 0));
 };
 
 struct TileCoord {
@@ -472,9 +471,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
   if (warp < 4) {
   // (block-scaled variant) producer, issuer and communication warps give registers to the
   // promotion warps; all four warps of the group execute the same instruction here. With 256-column
-  // tiles the promotion warps hold 128 accumulators and take all they can get: 40 / 232 measured
-  // 1560 TFLOP/s where 56 / 224 gave 1376 and 24 / 240 the same 1560 (the compiler's spill report:
-  // 168, 176 and 226 bytes per thread, the last mostly in the leading warps).
+  // tiles the promotion warps hold 128 accumulators and take all they can get. In the general form, with the
+  // one-lane issue loops: 40 / 232 1560 TFLOP/s, 56 / 224 1376, 24 / 240 1560; the lean loop of the plain forms is
+  // within 2 % on all three.
   if constexpr (Cfg::BS) ptx::setmaxnreg_dec<Cfg::REGS_LEAD>();
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -1324,8 +1323,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) dense_gemm_kernel(const __gri
       // whole, 300 while one lane walked the issue loops; 320 at the first shape with the general loop below: two polls
       // of the full barrier and spills); per column, 3584 x 8192 x 8192, 360 us
       // (379 with the one-lane loops; 1340 when every warp read the column scales from global memory where it
-      // multiplied by them). Sixteen warps of 64 columns, with the one-lane loops: 358 and 667 us. Register splits
-      // 24 / 240 and 56 / 224: within 2 % of 40 / 232.
+      // multiplied by them). Sixteen warps of 64 columns, with the one-lane loops: 358 and 667 us.
       constexpr bool kColumn = Cfg::BS_FORM == kBsColumn;
       const int half = ew >> 2;
       const int kbs = k_blocks;
