@@ -234,8 +234,8 @@ static int dense_impl(const fluxb_dense_args_t* a, const fluxb_a2a_args_t* x) {
     // measured slower than single CTAs on 128 x 128 (977 against 1128 TFLOP/s at 16384 x 3584 x 8192, with one-lane
     // issue loops): the k-block hand-over then waits for the slowest of sixteen promotion warps on two SMs.
     cg = (a->cta_group == 2 && a->tile_n != 256 && a->M / (multi ? a->world : 1) >= 256) ? 2 : 1;
-    // 128 x 256 tiles wherever N allows (tile_n = 128 pins the narrow ones): 1330 - 1350 against 1010 - 1060 TFLOP/s
-    // when both were bound by their one-lane issue loops; 2200 since those run on whole warps.
+    // 128 x 256 tiles wherever N allows (tile_n = 128 pins the narrow ones): 2275 against 1128 TFLOP/s at 16384 x 3584 x
+    // 8192, 2165 against 1095 with half the rows (1330 - 1350 against 1010 - 1060 with one-lane issue loops).
     bn = (cg == 1 && a->tile_n != 128 && (a->N % 256 == 0 || a->N >= 2048)) ? 256 : 128;
   } else if (a->mode == FLUXB_A2A_GEMM) {
     if (cg == 2 && a->M >= 256) bn = 256;
