@@ -26,6 +26,11 @@ from ..ops.ag_gemm import AGKernel
 from ..ops.gemm_rs import GemmRS
 
 
+def _dual_level() -> int:
+    """The innermost forward-mode level, -1 outside of any (where no tensor carries a tangent)."""
+    return getattr(forward_ad, "_current_level", 0)
+
+
 class _OpCache:
     """Fused-op objects keyed by shape: they own symmetric buffers (an all-gather landing buffer, the
     reduce-scatter staging slabs: hundreds of MB at transformer shapes), so one set per process group
@@ -154,9 +159,9 @@ class RowParallelLinear(nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         b = self.bias
         if (b is not None and x.is_cuda and self._cache.world == 1 and b.dtype == x.dtype
-                and b.device == x.device and b.is_contiguous() and b.shape == self.weight.shape[:1]
+                and b.device == x.device and b.is_contiguous() and b.dim() == 1 and b.numel() == self.out_features
                 and (x.requires_grad or self.weight.requires_grad or not b.requires_grad)
-                and forward_ad.unpack_dual(b).tangent is None):
+                and (_dual_level() < 0 or forward_ad.unpack_dual(b).tangent is None)):
             # one rank: the GEMM's epilogue adds the bias to the fp32 sum (a broadcast add over 8192 x 12288 bf16
             # is 235 us next to a GEMM of 970); a bias that trains alone keeps its add, whose backward is one sum, and so
             # does one with a forward-mode tangent, which the fused op has no rule for
